@@ -137,8 +137,11 @@ __global__ void __launch_bounds__(128, MINB) dock_kernel(DockParams p) {
                     float* yv = pv + pad4(n);
                     float* mhy = yv + pad4(n);
                     const GridInter gi{&p.G, p.ep.v_inter, p.ep.slope};
-                    ce = dense_bfgs<true>(L, s, H, gc, pv, yv, mhy, gi, p.smooth, p.ep.v_intra, p.ep.fix,
-                                          p.ep.inv_fix, cs[kCsSteps], lane, evals);
+                    const auto eval = [&](const SkipArmijo& skip) {
+                        return eval_pose_t<true, true>(L, s.m, gi, p.smooth, p.ep.v_intra, p.ep.fix, p.ep.inv_fix,
+                                                       lane, skip);
+                    };
+                    ce = dense_bfgs(L, s, H, gc, pv, yv, mhy, eval, cs[kCsSteps], lane, evals);
                 } else {
                     // visited history (visited.cuh:48-227, quasi_newton.cuh:1937-1943):
                     // interesting() holds until 10 x (6 + ntors) runs have been

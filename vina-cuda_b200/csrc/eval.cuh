@@ -323,6 +323,112 @@ struct SkipAbove {
     __device__ __forceinline__ bool operator()(float e) const { return e > thr; }
 };
 
+// Phases 6-7: the pose gradient into m.g from the atoms' grid-term forces
+// (m.fx/fy/fz), their fixed-point pair forces (m.ns) and coordinates (m.c).
+__device__ __forceinline__ void adjoint_phases(const LigView& L, const WarpMem& m, float inv_fix, int lane) {
+    // 6: prefix sums over the heavy atoms of force and moment about the root
+    // origin.  Atoms are grouped by body in pre-order, so a subtree's atoms
+    // are one contiguous range and its sums are a difference of two prefixes.
+    // Lane l owns atoms [l*A, l*A + A); prefix forces overwrite fx/fy/fz.
+    const float4 xo4 = *reinterpret_cast<const float4*>(m.x);
+    const float ox = xo4.x, oy = xo4.y, oz = xo4.z;
+    {
+        const int A = (L.na + 31) >> 5, a0 = lane * A, a1 = min(L.na, a0 + A);
+        const int a4 = pad4(L.na);
+        float* mx = m.ns;
+        float* my = m.ns + a4;
+        float* mz = m.ns + 2 * a4;
+        auto contrib = [&](int i, float v[6]) {
+            const float4 ci = m.c[i];
+            const int* q = reinterpret_cast<const int*>(m.ns);  // read before this lane overwrites it
+            const float fx = m.fx[i] + from_fixed(q[i], inv_fix), fy = m.fy[i] + from_fixed(q[a4 + i], inv_fix),
+                        fz = m.fz[i] + from_fixed(q[2 * a4 + i], inv_fix);
+            const float dx = ci.x - ox, dy = ci.y - oy, dz = ci.z - oz;
+            v[0] = fx; v[1] = fy; v[2] = fz;
+            v[3] = dy * fz - dz * fy;
+            v[4] = dz * fx - dx * fz;
+            v[5] = dx * fy - dy * fx;
+        };
+        auto scan = [&](float (&run)[6]) {  // inclusive scan of the lane totals
+#pragma unroll
+            for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+                for (int j = 0; j < 6; ++j) {
+                    const float o = __shfl_up_sync(0xffffffffu, run[j], off);
+                    if (lane >= off) run[j] += o;
+                }
+            }
+        };
+        if (A == 1) {  // up to 32 atoms: a lane's inclusive scan value is its atom's prefix
+            float run[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (a0 < a1) contrib(a0, run);
+            scan(run);
+            if (a0 < a1) {
+                m.fx[a0] = run[0]; m.fy[a0] = run[1]; m.fz[a0] = run[2];
+                mx[a0] = run[3]; my[a0] = run[4]; mz[a0] = run[5];
+            }
+        } else {  // lane totals, their exclusive scan, then each atom's prefix
+            float run[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for (int i = a0; i < a1; ++i) {
+                float v[6];
+                contrib(i, v);
+#pragma unroll
+                for (int j = 0; j < 6; ++j) run[j] += v[j];
+            }
+            scan(run);
+            float acc[6];
+#pragma unroll
+            for (int j = 0; j < 6; ++j) acc[j] = __shfl_up_sync(0xffffffffu, run[j], 1);
+            if (lane == 0)
+#pragma unroll
+                for (int j = 0; j < 6; ++j) acc[j] = 0.f;
+            for (int i = a0; i < a1; ++i) {
+                float v[6];
+                contrib(i, v);
+#pragma unroll
+                for (int j = 0; j < 6; ++j) acc[j] += v[j];
+                m.fx[i] = acc[0]; m.fy[i] = acc[1]; m.fz[i] = acc[2];
+                mx[i] = acc[3]; my[i] = acc[4]; mz[i] = acc[5];
+            }
+        }
+    }
+    __syncwarp();
+    // 7: subtree sums (prefix differences), torques and the pose gradient
+    for (int k = lane; k < L.nn; k += 32) {
+        const float4 w1 = node_word(L.nodes, k, 1);  // {axis, first atom}
+        const int e1 = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 2).w), 0, L.na, kChkSubtree);
+        const int b = VD_DCLAMP(__float_as_int(w1.w), 0, e1, kChkSubtree);
+        const int a4 = pad4(L.na);
+        float F0 = 0.f, F1 = 0.f, F2 = 0.f, M0 = 0.f, M1 = 0.f, M2 = 0.f;
+        if (e1 > b) {
+            const int hi = e1 - 1;
+            F0 = m.fx[hi]; F1 = m.fy[hi]; F2 = m.fz[hi];
+            M0 = m.ns[hi]; M1 = m.ns[a4 + hi]; M2 = m.ns[2 * a4 + hi];
+            if (b > 0) {
+                const int lo = b - 1;
+                F0 -= m.fx[lo]; F1 -= m.fy[lo]; F2 -= m.fz[lo];
+                M0 -= m.ns[lo]; M1 -= m.ns[a4 + lo]; M2 -= m.ns[2 * a4 + lo];
+            }
+        }
+        if (k == 0) {
+            m.g[0] = F0; m.g[1] = F1; m.g[2] = F2; m.g[3] = M0; m.g[4] = M1; m.g[5] = M2;
+        } else {
+            const float4* nd = reinterpret_cast<const float4*>(m.nd + kNodeF * k);
+            const float4 r0 = nd[0], r1 = nd[1], r2 = nd[2];
+            const float dx = r0.w - ox, dy = r1.w - oy, dz = r2.w - oz;
+            const float T0 = M0 - (dy * F2 - dz * F1);
+            const float T1 = M1 - (dz * F0 - dx * F2);
+            const float T2 = M2 - (dx * F1 - dy * F0);
+            const float u0 = w1.x, u1 = w1.y, u2 = w1.z;
+            const float a0 = r0.x * u0 + r0.y * u1 + r0.z * u2;
+            const float a1 = r1.x * u0 + r1.y * u1 + r1.z * u2;
+            const float a2 = r2.x * u0 + r2.y * u1 + r2.z * u2;
+            m.g[6 + k - 1] = T0 * a0 + T1 * a1 + T2 * a2;
+        }
+    }
+    __syncwarp();
+}
+
 // pair_atomics: pairs from the search schedule, both atoms' forces by
 // atomics (no per-lane flush when the second atom changes: shorter, less
 // divergent code, which the latency-bound search prefers); otherwise the
@@ -497,107 +603,7 @@ __device__ inline float eval_pose_t(const LigView& L, const WarpMem& m, const In
     e = warp_sum(e);
     if (!want_grad || skip(e)) return e;
     __syncwarp();
-    // 6: prefix sums over the heavy atoms of force and moment about the root
-    // origin.  Atoms are grouped by body in pre-order, so a subtree's atoms
-    // are one contiguous range and its sums are a difference of two prefixes.
-    // Lane l owns atoms [l*A, l*A + A); prefix forces overwrite fx/fy/fz.
-    const float4 xo4 = *reinterpret_cast<const float4*>(m.x);
-    const float ox = xo4.x, oy = xo4.y, oz = xo4.z;
-    {
-        const int A = (L.na + 31) >> 5, a0 = lane * A, a1 = min(L.na, a0 + A);
-        const int a4 = pad4(L.na);
-        float* mx = m.ns;
-        float* my = m.ns + a4;
-        float* mz = m.ns + 2 * a4;
-        auto contrib = [&](int i, float v[6]) {
-            const float4 ci = m.c[i];
-            const int* q = reinterpret_cast<const int*>(m.ns);  // read before this lane overwrites it
-            const float fx = m.fx[i] + from_fixed(q[i], inv_fix), fy = m.fy[i] + from_fixed(q[a4 + i], inv_fix),
-                        fz = m.fz[i] + from_fixed(q[2 * a4 + i], inv_fix);
-            const float dx = ci.x - ox, dy = ci.y - oy, dz = ci.z - oz;
-            v[0] = fx; v[1] = fy; v[2] = fz;
-            v[3] = dy * fz - dz * fy;
-            v[4] = dz * fx - dx * fz;
-            v[5] = dx * fy - dy * fx;
-        };
-        auto scan = [&](float (&run)[6]) {  // inclusive scan of the lane totals
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-                for (int j = 0; j < 6; ++j) {
-                    const float o = __shfl_up_sync(0xffffffffu, run[j], off);
-                    if (lane >= off) run[j] += o;
-                }
-            }
-        };
-        if (A == 1) {  // up to 32 atoms: a lane's inclusive scan value is its atom's prefix
-            float run[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            if (a0 < a1) contrib(a0, run);
-            scan(run);
-            if (a0 < a1) {
-                m.fx[a0] = run[0]; m.fy[a0] = run[1]; m.fz[a0] = run[2];
-                mx[a0] = run[3]; my[a0] = run[4]; mz[a0] = run[5];
-            }
-        } else {  // lane totals, their exclusive scan, then each atom's prefix
-            float run[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            for (int i = a0; i < a1; ++i) {
-                float v[6];
-                contrib(i, v);
-#pragma unroll
-                for (int j = 0; j < 6; ++j) run[j] += v[j];
-            }
-            scan(run);
-            float acc[6];
-#pragma unroll
-            for (int j = 0; j < 6; ++j) acc[j] = __shfl_up_sync(0xffffffffu, run[j], 1);
-            if (lane == 0)
-#pragma unroll
-                for (int j = 0; j < 6; ++j) acc[j] = 0.f;
-            for (int i = a0; i < a1; ++i) {
-                float v[6];
-                contrib(i, v);
-#pragma unroll
-                for (int j = 0; j < 6; ++j) acc[j] += v[j];
-                m.fx[i] = acc[0]; m.fy[i] = acc[1]; m.fz[i] = acc[2];
-                mx[i] = acc[3]; my[i] = acc[4]; mz[i] = acc[5];
-            }
-        }
-    }
-    __syncwarp();
-    // 7: subtree sums (prefix differences), torques and the pose gradient
-    for (int k = lane; k < L.nn; k += 32) {
-        const float4 w1 = node_word(L.nodes, k, 1);  // {axis, first atom}
-        const int e1 = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 2).w), 0, L.na, kChkSubtree);
-        const int b = VD_DCLAMP(__float_as_int(w1.w), 0, e1, kChkSubtree);
-        const int a4 = pad4(L.na);
-        float F0 = 0.f, F1 = 0.f, F2 = 0.f, M0 = 0.f, M1 = 0.f, M2 = 0.f;
-        if (e1 > b) {
-            const int hi = e1 - 1;
-            F0 = m.fx[hi]; F1 = m.fy[hi]; F2 = m.fz[hi];
-            M0 = m.ns[hi]; M1 = m.ns[a4 + hi]; M2 = m.ns[2 * a4 + hi];
-            if (b > 0) {
-                const int lo = b - 1;
-                F0 -= m.fx[lo]; F1 -= m.fy[lo]; F2 -= m.fz[lo];
-                M0 -= m.ns[lo]; M1 -= m.ns[a4 + lo]; M2 -= m.ns[2 * a4 + lo];
-            }
-        }
-        if (k == 0) {
-            m.g[0] = F0; m.g[1] = F1; m.g[2] = F2; m.g[3] = M0; m.g[4] = M1; m.g[5] = M2;
-        } else {
-            const float4* nd = reinterpret_cast<const float4*>(m.nd + kNodeF * k);
-            const float4 r0 = nd[0], r1 = nd[1], r2 = nd[2];
-            const float dx = r0.w - ox, dy = r1.w - oy, dz = r2.w - oz;
-            const float T0 = M0 - (dy * F2 - dz * F1);
-            const float T1 = M1 - (dz * F0 - dx * F2);
-            const float T2 = M2 - (dx * F1 - dy * F0);
-            const float u0 = w1.x, u1 = w1.y, u2 = w1.z;
-            const float a0 = r0.x * u0 + r0.y * u1 + r0.z * u2;
-            const float a1 = r1.x * u0 + r1.y * u1 + r1.z * u2;
-            const float a2 = r2.x * u0 + r2.y * u1 + r2.z * u2;
-            m.g[6 + k - 1] = T0 * a0 + T1 * a1 + T2 * a2;
-        }
-    }
-    __syncwarp();
+    adjoint_phases(L, m, inv_fix, lane);
     return e;
 }
 

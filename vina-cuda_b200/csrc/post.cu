@@ -33,68 +33,23 @@ struct RecView {
     const double4* recd;        // same in double
     const int32_t* cell_start;  // [cells+1]
     const int32_t* cell_list;   // atom indices per cell
-    double init[3], range[3];   // szv_grid cell geometry
+    float init[3], per[3];      // szv_grid cell geometry: origin, cells per A
     int32_t dim[3];
     double gb[3], ge[3];        // box (non_cache gd)
+    float gbf[3], gef[3];       // the same in FP32
 };
 
-__device__ __forceinline__ int cell_of(const RecView& R, double x, double y, double z) {
-    const double c[3] = {x, y, z};
+// szv_grid.cpp:92-107 (fl_to_sz) in FP32: a point within rounding of a cell
+// face may take the neighbour cell, whose list reaches a little further
+// than the cutoff (ensure_receptor_cells) and so holds the same atoms in
+// reach, in the same order.
+__device__ __forceinline__ int cell_of(const RecView& R, float x, float y, float z) {
+    const float c[3] = {x, y, z};
     int idx[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {  // szv_grid.cpp:92-107, fl_to_sz
-        const double t = (c[d] - R.init[d]) * R.dim[d] / R.range[d];
-        const int mx = R.dim[d] - 1;
-        idx[d] = (t <= 0) ? 0 : ((t >= mx) ? mx : min(int(t), mx));
-    }
+    for (int d = 0; d < 3; ++d) idx[d] = max(0, min(int((c[d] - R.init[d]) * R.per[d]), R.dim[d] - 1));
     return VD_DCLAMP(idx[0] + R.dim[0] * (idx[1] + R.dim[1] * idx[2]), 0, R.dim[0] * R.dim[1] * R.dim[2] - 1, kChkCell);
 }
-
-// non_cache::eval_deriv term of one atom (FP32), smooth table, curl v.
-struct DirectInter {
-    const RecView* R;
-    const float4* smooth;
-    float v, slope;
-    __device__ __forceinline__ float operator()(int t1, float px, float py, float pz, float& gx, float& gy,
-                                                float& gz) const {
-        float a[3] = {px, py, pz}, od[3] = {0.f, 0.f, 0.f};
-        float oob = 0.f;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float b = float(R->gb[d]), e = float(R->ge[d]);
-            if (a[d] < b) { oob += fabsf(a[d] - b); a[d] = b; od[d] = -1.f; }
-            else if (a[d] > e) { oob += fabsf(a[d] - e); a[d] = e; od[d] = 1.f; }
-        }
-        const int c = cell_of(*R, a[0], a[1], a[2]);
-        const int q0 = __ldg(&R->cell_start[c]), q1 = __ldg(&R->cell_start[c + 1]);
-        float this_e = 0.f, dx = 0.f, dy = 0.f, dz = 0.f;
-        for (int q = q0; q < q1; ++q) {
-            const float4 b = __ldg(&R->rec[__ldg(&R->cell_list[q])]);
-            const float rx = a[0] - b.x, ry = a[1] - b.y, rz = a[2] - b.z;
-            const float r2 = rx * rx + ry * ry + rz * rz;
-            if (r2 < 64.f) {
-                const int t2 = int(b.w);
-                const int tp = (t1 <= t2) ? t1 + t2 * (t2 + 1) / 2 : t2 + t1 * (t1 + 1) / 2;
-                const float rf = 32.f * r2;
-                const int i1 = int(rf);
-                const float rem = rf - float(i1);
-                const float4 tv = __ldg(smooth + size_t(tp) * kBins + i1);
-                this_e += tv.x + rem * (tv.z - tv.x);
-                const float dor = tv.y + rem * (tv.w - tv.y);
-                dx += dor * rx; dy += dor * ry; dz += dor * rz;
-            }
-        }
-        if (this_e > 0.f) {
-            const float tt = v / (v + this_e);
-            this_e *= tt;
-            dx *= tt * tt; dy *= tt * tt; dz *= tt * tt;
-        }
-        gx = dx + slope * od[0];
-        gy = dy + slope * od[1];
-        gz = dz + slope * od[2];
-        return this_e + slope * oob;
-    }
-};
 
 // ------------------------------------------------------------ cluster
 struct ClusterParams {
@@ -192,62 +147,392 @@ struct RefineParams {
     RecView R;
     const float4* smooth;
     float fix, inv_fix;         // fixed-point scale of the pair forces (EvalParams::fix) and 1/fix
-    int32_t warp_floats;
     unsigned long long* evals;
     int32_t skip_invalid;       // leave poses whose e_out is FLT_MAX untouched
 };
 
-constexpr int kRefineWarps = 4;
+// One block refines one pose.  A dense-BFGS run is a serial chain of
+// evaluations, and an evaluation on the direct-sum score is mostly receptor
+// neighbours (tens to hundreds per atom, three dependent loads each) and
+// intra pairs: with one warp a pose, one lane walked an atom's neighbours
+// one after the other and a 20-pose call kept 5 SMs busy.  Warp 0 runs the
+// optimiser; for each evaluation it places the atoms, then all warps compute
+// the neighbour and pair terms in parallel into shared memory, and their sums
+// are taken from there in the order a single lane would take them (a
+// receptor cell's list order per atom, 32 segments of the pair list), so the
+// refined poses do not depend on how the work was spread.
+// 20 poses of 45 atoms / 12 torsions in an 8,000-atom receptor, B200:
+// 12.79 ms with one warp a pose, 2.22 ms with sixteen (a single docked ligand's
+// 20 modes, 31 atoms / 8 torsions: 1.95 -> 0.57 ms).  What is left is latency:
+// ~1,900 cycles of body frames, ~5,000 of receptor terms (two thirds of them
+// gathers from L2), ~1,200 of pairs, ~2,300 of optimiser per evaluation.
+constexpr int kRefineWarps = 16;
+constexpr int kNb = 32;    // neighbours of an atom per tile (one per lane)
+constexpr int kSlots = 4;  // atoms a warp takes at a time
+
+// Per-warp tile of neighbour terms, one row of kNb neighbours per atom and
+// component: [kSlots * 4] {x, y, z, energy}, then [kSlots] derivatives; rows
+// of 36 floats keep the row-wise 128-bit reads free of bank conflicts.  Then
+// the atoms' clamped positions and cell ranges.
+constexpr int kRow = kNb + 4;
+constexpr int kTileFloats = kSlots * 5 * kRow + kSlots * 4 + kSlots * 2;
+static_assert(kTileFloats % 4 == 0, "tiles stay 16-byte aligned");
+
+struct TeamMem {
+    float* tile;        // this warp's
+    float* eatom;       // [na] receptor terms
+    float* pair;        // [4][np] force on the second atom, energy
+    uint16_t* run;      // [runs + 1] first pair of each run of one second atom
+    int* cmd;           // 0: leave, 1: evaluate
+    float* slope;
+    int* runs;
+};
+
+__host__ __device__ inline int team_floats(int na, int np) {
+    return kRefineWarps * kTileFloats + pad4(na) + 4 * np + pad4((np + 2) / 2) + 4;
+}
+
+// non_cache::eval_deriv terms (FP32, smooth table, curl v) of the atom
+// groups `wid`, `wid` + kRefineWarps, ..: gradients to m.fx/fy/fz, energies
+// to eatom.  Lanes are neighbours, a tile of kNb per atom at a time; then
+// lane 4 s + c adds up component c (x, y, z, energy) of atom s in list order.
+__device__ __forceinline__ void direct_terms(const LigView& L, const WarpMem& m, const RecView& R, const float4* smooth,
+                                             float v, float slope, const TeamMem& tm, int wid, int lane) {
+    float* const td = tm.tile + kSlots * 4 * kRow;
+    float4* const at = reinterpret_cast<float4*>(td + kSlots * kRow);
+    int2* const range = reinterpret_cast<int2*>(at + kSlots);
+    const int groups = (L.na + kSlots - 1) / kSlots;
+    for (int g = wid; g < groups; g += kRefineWarps) {
+        float a[3] = {0.f, 0.f, 0.f}, od[3] = {0.f, 0.f, 0.f}, oob = 0.f;
+        int n = 0;
+        if (lane < kSlots) {
+            const int i = g * kSlots + lane;
+            int2 q = make_int2(0, 0);
+            int t1 = 0;
+            if (i < L.na) {
+                const float4 c = m.c[i];
+                a[0] = c.x; a[1] = c.y; a[2] = c.z;
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const float b = R.gbf[d], e = R.gef[d];
+                    if (a[d] < b) { oob += fabsf(a[d] - b); a[d] = b; od[d] = -1.f; }
+                    else if (a[d] > e) { oob += fabsf(a[d] - e); a[d] = e; od[d] = 1.f; }
+                }
+                const int cell = cell_of(R, a[0], a[1], a[2]);
+                q = make_int2(__ldg(&R.cell_start[cell]), __ldg(&R.cell_start[cell + 1]));
+                t1 = __float_as_int(__ldg(&L.atoms[i].w)) & 0xff;
+            }
+            n = q.y - q.x;
+            at[lane] = make_float4(a[0], a[1], a[2], __int_as_float(t1));
+            range[lane] = q;
+        }
+        n = __reduce_max_sync(0xffffffffu, n);
+        __syncwarp();
+        const int s = (lane >> 2) < kSlots ? lane >> 2 : 0, c = lane & 3;
+        float acc = 0.f;
+        int idx[kSlots];  // the tile's neighbours, loaded one tile ahead; -1: none
+        auto load_idx = [&](int k0) {
+#pragma unroll
+            for (int j = 0; j < kSlots; ++j) {
+                const int2 q = range[j];
+                const int qi = q.x + k0 + lane;
+                idx[j] = qi < q.y ? __ldg(&R.cell_list[qi]) : -1;
+            }
+        };
+        load_idx(0);
+        for (int k0 = 0; k0 < n; k0 += kNb) {
+            // all slots' loads in flight per stage, no branches
+            float4 nb[kSlots], tv[kSlots];
+            float rem[kSlots];
+            bool in[kSlots];
+#pragma unroll
+            for (int j = 0; j < kSlots; ++j) {
+                in[j] = idx[j] >= 0;
+                nb[j] = __ldg(&R.rec[max(idx[j], 0)]);  // entry 0 always exists
+            }
+            if (k0 + kNb < n) load_idx(k0 + kNb);
+#pragma unroll
+            for (int j = 0; j < kSlots; ++j) {
+                const float4 p = at[j];
+                const float rx = p.x - nb[j].x, ry = p.y - nb[j].y, rz = p.z - nb[j].z;
+                const float r2 = rx * rx + ry * ry + rz * rz;
+                const int t1 = __float_as_int(p.w), t2 = int(nb[j].w);
+                const int tp = (t1 <= t2) ? t1 + t2 * (t2 + 1) / 2 : t2 + t1 * (t1 + 1) / 2;
+                in[j] = in[j] && r2 < 64.f;
+                const float rf = in[j] ? 32.f * r2 : 0.f;
+                const int i1 = int(rf);
+                rem[j] = rf - float(i1);
+                nb[j] = make_float4(rx, ry, rz, 0.f);
+                tv[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (in[j]) tv[j] = __ldg(smooth + size_t(tp) * kBins + i1);
+            }
+#pragma unroll
+            for (int j = 0; j < kSlots; ++j) {  // out of reach: all terms zero
+                const float e = tv[j].x + rem[j] * (tv[j].z - tv[j].x), dor = tv[j].y + rem[j] * (tv[j].w - tv[j].y);
+                float* const row = tm.tile + 4 * j * kRow + lane;
+                row[0] = in[j] ? nb[j].x : 0.f;
+                row[kRow] = in[j] ? nb[j].y : 0.f;
+                row[2 * kRow] = in[j] ? nb[j].z : 0.f;
+                row[3 * kRow] = in[j] ? e : 0.f;
+                td[j * kRow + lane] = in[j] ? dor : 0.f;
+            }
+            __syncwarp();
+            const int m_here = min(kNb, n - k0);  // rounded up to eights: the rest are zero terms
+            const float4* const xr = reinterpret_cast<const float4*>(tm.tile + (4 * s + c) * kRow);
+            const float4* const fr = reinterpret_cast<const float4*>(td + s * kRow);
+            auto add = [&](float f, float x) { acc = fmaf(c < 3 ? f : 1.f, x, acc); };  // energy: 1 * e; force: derivative * r
+            for (int k = 0; k < m_here; k += 8) {
+                const float4 x0 = xr[k / 4], x1 = xr[k / 4 + 1], f0 = fr[k / 4], f1 = fr[k / 4 + 1];
+                add(f0.x, x0.x); add(f0.y, x0.y); add(f0.z, x0.z); add(f0.w, x0.w);
+                add(f1.x, x1.x); add(f1.y, x1.y); add(f1.z, x1.z); add(f1.w, x1.w);
+            }
+            __syncwarp();
+        }
+        const float this_e = __shfl_sync(0xffffffffu, acc, lane | 3);
+        if (this_e > 0.f) {
+            const float tt = v / (v + this_e);
+            acc = (c < 3) ? acc * (tt * tt) : acc * tt;
+        }
+        const float o0 = __shfl_sync(0xffffffffu, od[0], s), o1 = __shfl_sync(0xffffffffu, od[1], s),
+                    o2 = __shfl_sync(0xffffffffu, od[2], s), o3 = __shfl_sync(0xffffffffu, oob, s);
+        const int i = g * kSlots + s;
+        if ((lane >> 2) < kSlots && i < L.na) {
+            float* const dst = c == 0 ? m.fx : c == 1 ? m.fy : c == 2 ? m.fz : tm.eatom;
+            dst[i] = acc + slope * (c == 0 ? o0 : c == 1 ? o1 : c == 2 ? o2 : o3);
+        }
+        __syncwarp();
+    }
+}
+
+// Intra-pair terms of one evaluation, one pair per thread: the pair's capped
+// energy and force to tm.pair, the force on the first atom into its
+// fixed-point accumulator (integer sums: exact in any order).  Two pairs'
+// loads are in flight per thread.
+__device__ __forceinline__ void pair_terms(const LigView& L, const WarpMem& m, const float4* smooth, float v, float fix,
+                                           const TeamMem& tm, int tid) {
+    constexpr int kStep = 32 * kRefineWarps;
+    int* const qx = reinterpret_cast<int*>(m.ns);
+    int* const qy = qx + pad4(L.na);
+    int* const qz = qy + pad4(L.na);
+    for (int p0 = tid; p0 < L.np; p0 += 2 * kStep) {
+        float4 r[2], t[2];
+        int a[2];
+        bool in[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int p = p0 + j * kStep;
+            in[j] = p < L.np;
+            const int2 q = in[j] ? __ldg(&L.pairs[p]) : make_int2(0, 0);
+            a[j] = VD_DCLAMP(q.x & 0xffff, 0, L.na - 1, kChkPairAtom);
+            const float4 ca = m.c[a[j]], cb = m.c[VD_DCLAMP(q.x >> 16, 0, L.na - 1, kChkPairAtom)];
+            const float rx = cb.x - ca.x, ry = cb.y - ca.y, rz = cb.z - ca.z;
+            const float d = rx * rx + ry * ry + rz * rz;
+            const float rf = fminf(32.f * d, 2047.5f);
+            const int i = VD_DCLAMP(int(rf), 0, kBins - 2, kChkTableBin);
+            r[j] = make_float4(rx, ry, rz, rf - float(i));
+            in[j] = in[j] && d < 64.f;
+            t[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (in[j]) t[j] = __ldg(smooth + size_t(VD_DCLAMP(q.y, 0, kPairTypes - 1, kChkPairType)) * kBins + i);
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            float4 out = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (in[j]) {
+                const float w = r[j].w;
+                const float e = t[j].x + w * (t[j].z - t[j].x), g = t[j].y + w * (t[j].w - t[j].y);
+                const float c = (e > 0.f) ? __fdividef(v, v + e) : 1.f;
+                const float gc = g * c * c;
+                out = make_float4(gc * r[j].x, gc * r[j].y, gc * r[j].z, e * c);
+                atomicAdd(&qx[a[j]], to_fixed(-out.x, fix)); atomicAdd(&qy[a[j]], to_fixed(-out.y, fix));
+                atomicAdd(&qz[a[j]], to_fixed(-out.z, fix));
+            }
+            const int p = p0 + j * kStep;
+            if (p < L.np) {
+                tm.pair[p] = out.x;
+                tm.pair[L.np + p] = out.y;
+                tm.pair[2 * L.np + p] = out.z;
+                tm.pair[3 * L.np + p] = out.w;
+            }
+        }
+    }
+}
+
+// The pair list (sorted by second atom) is 32 segments, one per lane of a
+// single-warp evaluation; a run is a stretch of one segment with one second
+// atom.  First pairs of the runs to tm.run (tm.run[runs] = pairs).
+__device__ __forceinline__ int find_runs(const LigView& L, const TeamMem& tm, int lane) {
+    int runs = 0;
+    for (int p0 = 0; p0 < L.np; p0 += 32) {
+        const int p = p0 + lane;
+        bool first = false;
+        if (p < L.np) {
+            // p starts a segment: some l has l * np / 32 (rounded down) = p
+            const int l = (p * 32 + L.np - 1) / L.np;
+            first = p == 0 || ((l * L.np) >> 5) == p || (L.pairs[p].x >> 16) != (L.pairs[p - 1].x >> 16);
+        }
+        const unsigned b = __ballot_sync(0xffffffffu, first);
+        if (first) tm.run[runs + __popc(b & ((1u << lane) - 1u))] = uint16_t(p);
+        runs += __popc(b);
+    }
+    if (lane == 0) {
+        tm.run[runs] = uint16_t(L.np);
+        *tm.runs = runs;
+    }
+    __syncwarp();
+    return runs;
+}
+
+// The second atoms' forces: one thread per run and component adds the run's
+// forces in list order, then the run to its atom's accumulator.
+__device__ __forceinline__ void run_terms(const LigView& L, const WarpMem& m, float fix, const TeamMem& tm, int tid,
+                                          int threads) {
+    const int n = 3 * *tm.runs;
+    for (int j = tid; j < n; j += threads) {
+        const int r = j / 3, c = j - 3 * r;
+        const int p0 = tm.run[r], p1 = tm.run[r + 1];
+        const float* f = tm.pair + c * L.np;
+        float b = 0.f;
+        for (int p = p0; p < p1; p += 8) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = p + k < p1 ? f[p + k] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k) b += v[k];
+        }
+        const int atom = VD_DCLAMP(L.pairs[p0].x >> 16, 0, L.na - 1, kChkPairAtom);
+        atomicAdd(reinterpret_cast<int*>(m.ns) + c * pad4(L.na) + atom, to_fixed(b, fix));
+    }
+}
+
+// The energy: lane l takes atoms l, l + 32, .. and segment l of the pair list,
+// two pairs at a time.
+__device__ __forceinline__ float sum_energy(const LigView& L, const TeamMem& tm, int lane) {
+    float e = 0.f;
+    for (int i = lane; i < L.na; i += 32) e += tm.eatom[i];
+    const float* pe = tm.pair + 3 * L.np;
+    const int p1 = ((lane + 1) * L.np) >> 5;
+    for (int p = (lane * L.np) >> 5; p < p1; p += 8) {
+        float f[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = p + j < p1 ? pe[p + j] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 8; j += 2) e += f[j] + f[j + 1];
+    }
+    return warp_sum(e);
+}
 
 __device__ __forceinline__ bool m_out(float v, double b, double e) {
     return v < float(b - 1e-4) || v > float(e + 1e-4);
 }
 
-__global__ void __launch_bounds__(32 * kRefineWarps) refine_kernel(RefineParams p) {
+// Barriers of a refinement block: 1, the atoms are placed (or the pose is
+// done); 3, all warps: the terms are in shared memory; 2, the second atoms'
+// forces are added.  Warp 0 arrives at 1 and waits at 2, the others the other
+// way round; every thread takes part in each once per evaluation, and in 1
+// once more at the end.
+__device__ __forceinline__ void team_sync(int id) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(32 * kRefineWarps) : "memory");
+}
+__device__ __forceinline__ void team_arrive(int id) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(32 * kRefineWarps) : "memory");
+}
+
+__global__ void __launch_bounds__(32 * kRefineWarps, 1) refine_kernel(RefineParams p) {
     extern __shared__ float4 smem4[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float* base = reinterpret_cast<float*>(smem4) + size_t(wid) * p.warp_floats;
-    int evals = 0;
-    for (int pose = blockIdx.x * kRefineWarps + wid; pose < p.n_poses; pose += gridDim.x * kRefineWarps) {
-        const int li = p.pose_lig ? p.pose_lig[pose] : 0;
-        if (p.skip_invalid && !(p.e_out[pose] < FLT_MAX)) continue;
-        const LigView L = lig_view(p.pool, p.lig_off[li]);
-        const int n = 6 + L.nt, nc = 7 + L.nt;
-        SearchMem s;
-        s.m = carve(base, L.na, L.nn, L.np, L.nt);
-        s.xp = base + warp_floats(L.na, L.nn, L.np, L.nt);
-        s.xo = s.xp + pad4(nc);
-        float* H = s.xo + pad4(nc);
-        float* gc = H + pad4(n * n);
-        float* pv = gc + pad4(n);
-        float* yv = pv + pad4(n);
-        float* mhy = yv + pad4(n);
-        float* x = p.poses + size_t(pose) * p.stride;
-        for (int i = lane; i < nc; i += 32) s.m.x[i] = x[i];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, pose = blockIdx.x;
+    const int li = p.pose_lig ? p.pose_lig[pose] : 0;
+    if (p.skip_invalid && !(p.e_out[pose] < FLT_MAX)) return;  // the whole block
+    const LigView L = lig_view(p.pool, p.lig_off[li]);
+    const int n = 6 + L.nt, nc = 7 + L.nt;
+    float* base = reinterpret_cast<float*>(smem4);
+    SearchMem s;
+    s.m = carve(base, L.na, L.nn, L.np, L.nt);
+    s.xp = base + warp_floats(L.na, L.nn, L.np, L.nt);
+    s.xo = s.xp + pad4(nc);
+    float* H = s.xo + pad4(nc);
+    float* gc = H + pad4(n * n);
+    float* pv = gc + pad4(n);
+    float* yv = pv + pad4(n);
+    float* mhy = yv + pad4(n);
+    TeamMem tm;
+    float* team = mhy + pad4(n);
+    tm.tile = team + wid * kTileFloats;
+    tm.eatom = team + kRefineWarps * kTileFloats;
+    tm.pair = tm.eatom + pad4(L.na);
+    tm.run = reinterpret_cast<uint16_t*>(tm.pair + 4 * L.np);
+    tm.cmd = reinterpret_cast<int*>(tm.eatom + pad4(L.na) + 4 * L.np + pad4((L.np + 2) / 2));
+    tm.slope = reinterpret_cast<float*>(tm.cmd + 1);
+    tm.runs = tm.cmd + 2;
+    auto terms = [&](float slope) {
+        direct_terms(L, s.m, p.R, p.smooth, 1000.f, slope, tm, wid, lane);
+        pair_terms(L, s.m, p.smooth, 1000.f, p.fix, tm, threadIdx.x);
         __syncwarp();
-        const int max_steps = p.max_steps ? p.max_steps[li] : p.max_steps_default;
-        float e = FLT_MAX;
-        bool inside = false;
-        for (int ramp = 0; ramp < 5; ++ramp) {
-            const float slope = 100.f * powf(10.f, 2.f * ramp);
-            const DirectInter di{&p.R, p.smooth, 1000.f, slope};
-            e = dense_bfgs(L, s, H, gc, pv, yv, mhy, di, p.smooth, 1000.f, p.fix, p.inv_fix, max_steps, lane, evals);
-            kinematics(L, s.m, lane);
-            bool ok = true;  // non_cache::within, margin 1e-4
-            for (int i = lane; i < L.na; i += 32) {
-                if (m_out(s.m.c[i].x, p.R.gb[0], p.R.ge[0]) || m_out(s.m.c[i].y, p.R.gb[1], p.R.ge[1]) ||
-                    m_out(s.m.c[i].z, p.R.gb[2], p.R.ge[2]))
-                    ok = false;
-            }
-            inside = __all_sync(0xffffffffu, ok);
-            if (inside) break;
+        team_sync(3);
+    };
+    if (wid == 0) find_runs(L, tm, lane);
+    __syncthreads();
+    if (wid > 0) {
+        for (;;) {
+            team_sync(1);
+            if (*tm.cmd == 0) break;
+            terms(*tm.slope);
+            run_terms(L, s.m, p.fix, tm, threadIdx.x - 32, 32 * (kRefineWarps - 1));
+            __syncwarp();
+            team_arrive(2);
         }
-        if (!inside) e = FLT_MAX;
-        for (int i = lane; i < nc; i += 32) x[i] = s.m.x[i];
-        if (lane == 0) p.e_out[pose] = e;
-        __syncwarp();
+        return;
     }
-    if (lane == 0 && evals) atomicAdd(p.evals, (unsigned long long)evals);
+    int evals = 0;
+    float* x = p.poses + size_t(pose) * p.stride;
+    for (int i = lane; i < nc; i += 32) s.m.x[i] = x[i];
+    __syncwarp();
+    const int max_steps = p.max_steps ? p.max_steps[li] : p.max_steps_default;
+    float e = FLT_MAX;
+    bool inside = false;
+    for (int ramp = 0; ramp < 5; ++ramp) {
+        const float slope = 100.f * powf(10.f, 2.f * ramp);
+        const auto eval = [&](const SkipArmijo& skip) {
+            frames(L, s.m, lane);
+            int* const q = reinterpret_cast<int*>(s.m.ns);  // pair-force accumulators start at zero
+            const int a4 = pad4(L.na);
+            for (int i = lane; i < L.na; i += 32) {
+                s.m.c[i] = atom_position(L, s.m, __ldg(&L.atoms[i]));
+                q[i] = 0; q[a4 + i] = 0; q[2 * a4 + i] = 0;
+            }
+            if (lane == 0) {
+                *tm.cmd = 1;
+                *tm.slope = slope;
+            }
+            __syncwarp();
+            team_arrive(1);
+            terms(slope);
+            const float sum = sum_energy(L, tm, lane);
+            __syncwarp();
+            team_sync(2);
+            if (skip(sum)) return sum;
+            adjoint_phases(L, s.m, p.inv_fix, lane);
+            return sum;
+        };
+        e = dense_bfgs(L, s, H, gc, pv, yv, mhy, eval, max_steps, lane, evals);
+        kinematics(L, s.m, lane);
+        bool ok = true;  // non_cache::within, margin 1e-4
+        for (int i = lane; i < L.na; i += 32) {
+            if (m_out(s.m.c[i].x, p.R.gb[0], p.R.ge[0]) || m_out(s.m.c[i].y, p.R.gb[1], p.R.ge[1]) ||
+                m_out(s.m.c[i].z, p.R.gb[2], p.R.ge[2]))
+                ok = false;
+        }
+        inside = __all_sync(0xffffffffu, ok);
+        if (inside) break;
+    }
+    if (!inside) e = FLT_MAX;
+    for (int i = lane; i < nc; i += 32) x[i] = s.m.x[i];
+    if (lane == 0) {
+        p.e_out[pose] = e;
+        if (evals) atomicAdd(p.evals, (unsigned long long)evals);
+        *tm.cmd = 0;
+    }
+    __syncwarp();
+    team_arrive(1);
 }
 
 // ------------------------------------------------------------ score (double)
@@ -371,7 +656,7 @@ __device__ double inter_fast(const LigView& L, const RecView& R, const double* c
             else if (a[d] > R.ge[d]) { oob += fabs(a[d] - R.ge[d]); a[d] = R.ge[d]; }
         }
         oob *= 1e6;
-        const int ce = cell_of(R, a[0], a[1], a[2]);
+        const int ce = cell_of(R, float(a[0]), float(a[1]), float(a[2]));
         double this_e = 0;
         for (int q = R.cell_start[ce]; q < R.cell_start[ce + 1]; ++q) {
             const double4 b = R.recd[R.cell_list[q]];
@@ -598,6 +883,12 @@ vd_status ensure_receptor_cells(Ctx* c) {
     const int n_rec = int(c->rec_xs.size());
     for (int i = 0; i < n_rec; ++i)
         if (c->rec_xs[i] >= 0 && brick(init, end, &c->rec_xyz[3 * size_t(i)]) < kCutoff2) rel.push_back(i);
+    // A cell's list reaches a little further than the cutoff, so that a point
+    // that FP32 rounding puts into the cell next to its own (cell_of) still
+    // finds every atom within 8 A there.
+    double far = 0;
+    for (int d = 0; d < 3; ++d) far = std::max({far, std::fabs(init[d]), std::fabs(end[d])});
+    const double margin = 1e-3 + 1e-6 * far, reach2 = (8.0 + margin) * (8.0 + margin);
     const int ncell = dim[0] * dim[1] * dim[2];
     std::vector<std::vector<int>> cells(ncell);
     auto coord = [&](int d, int i) { return init[d] + range[d] * i / dim[d]; };
@@ -605,15 +896,15 @@ vd_status ensure_receptor_cells(Ctx* c) {
         const double* a = &c->rec_xyz[3 * size_t(rel[r])];
         int lo[3], hi[3];
         for (int d = 0; d < 3; ++d) {  // candidate cells within the cutoff, then the exact test
-            lo[d] = std::max(0, int(std::floor((a[d] - 8.0 - init[d]) * dim[d] / range[d])) - 1);
-            hi[d] = std::min(dim[d] - 1, int(std::floor((a[d] + 8.0 - init[d]) * dim[d] / range[d])) + 1);
+            lo[d] = std::max(0, int(std::floor((a[d] - 8.0 - margin - init[d]) * dim[d] / range[d])) - 1);
+            hi[d] = std::min(dim[d] - 1, int(std::floor((a[d] + 8.0 + margin - init[d]) * dim[d] / range[d])) + 1);
         }
         for (int z = lo[2]; z <= hi[2]; ++z)
             for (int y = lo[1]; y <= hi[1]; ++y)
                 for (int x = lo[0]; x <= hi[0]; ++x) {
                     const double b[3] = {coord(0, x), coord(1, y), coord(2, z)};
                     const double e[3] = {coord(0, x + 1), coord(1, y + 1), coord(2, z + 1)};
-                    if (brick(b, e, a) < kCutoff2) cells[x + dim[0] * (y + dim[1] * z)].push_back(r);
+                    if (brick(b, e, a) < reach2) cells[x + dim[0] * (y + dim[1] * z)].push_back(r);
                 }
     }
     std::vector<int32_t> start(ncell + 1, 0), list;
@@ -668,18 +959,21 @@ RecView rec_view(const Ctx& c) {
     R.cell_start = c.d_cell_start;
     R.cell_list = c.d_cell_list;
     for (int d = 0; d < 3; ++d) {
-        R.init[d] = c.cell_init[d];
-        R.range[d] = c.cell_range[d];
+        R.init[d] = float(c.cell_init[d]);
+        R.per[d] = float(c.cell_dim[d] / c.cell_range[d]);
         R.dim[d] = c.cell_dim[d];
+        R.gbf[d] = float(c.geom.begin[d]);
+        R.gef[d] = float(c.geom.end[d]);
         R.gb[d] = c.geom.begin[d];
         R.ge[d] = c.geom.end[d];
     }
     return R;
 }
 
-int refine_warp_floats(const HostLigand& L) {
+// Shared-memory floats of one pose's refinement block.
+int refine_floats(const HostLigand& L) {
     const int n = 6 + L.h.ntors, nc = 7 + L.h.ntors;
-    return lig_warp_floats(L) + 2 * pad4(nc) + pad4(n * n) + 4 * pad4(n);
+    return lig_warp_floats(L) + 2 * pad4(nc) + pad4(n * n) + 4 * pad4(n) + team_floats(L.h.n_atoms, L.h.n_pairs);
 }
 
 inline size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -710,7 +1004,7 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
         search_defaults(L, sp, depth[i], steps[i]);
         max_chains = std::max(max_chains, db.prefix[i + 1] - db.prefix[i]);
         max_wf = std::max(max_wf, lig_warp_floats(L));
-        max_rwf = std::max(max_rwf, refine_warp_floats(L));
+        max_rwf = std::max(max_rwf, refine_floats(L));
         max_na = std::max(max_na, L.h.n_atoms);
         max_nn = std::max(max_nn, L.h.n_nodes);
     }
@@ -778,13 +1072,12 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
         rp.smooth = c.d_smooth;
         rp.fix = c.fix_scale;
         rp.inv_fix = 1.f / c.fix_scale;
-        rp.warp_floats = max_rwf;
         rp.evals = reinterpret_cast<unsigned long long*>(c.d_counter + 4);
         rp.skip_invalid = 1;
-        smem_r = size_t(max_rwf) * kRefineWarps * 4;
+        smem_r = size_t(max_rwf) * 4;
         VD_CHECK(smem_r <= 227 * 1024, VD_ERR_CAPACITY, "refine kernel shared memory exceeds 227 KB");
         VD_CUDA(cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_r)));
-        blocks_r = (n * VD_MAX_MODES + kRefineWarps - 1) / kRefineWarps;
+        blocks_r = n * VD_MAX_MODES;
     }
     // score
     ScoreParams sc{};
@@ -1017,13 +1310,12 @@ vd_status vd_refine(vd_ctx* h, int32_t lig, int32_t n, float* poses, int32_t max
     rp.smooth = c.d_smooth;
     rp.fix = c.fix_scale;
     rp.inv_fix = 1.f / c.fix_scale;
-    rp.warp_floats = refine_warp_floats(L);
     rp.evals = reinterpret_cast<unsigned long long*>(c.d_counter + 4);
     rp.skip_invalid = 0;
-    const size_t smem_r = size_t(rp.warp_floats) * kRefineWarps * 4;
+    const size_t smem_r = size_t(refine_floats(L)) * 4;
     VD_CHECK(smem_r <= 227 * 1024, VD_ERR_CAPACITY, "refine kernel shared memory exceeds 227 KB");
     VD_CUDA(cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_r)));
-    refine_kernel<<<(n + kRefineWarps - 1) / kRefineWarps, 32 * kRefineWarps, smem_r, c.stream>>>(rp);
+    refine_kernel<<<n, 32 * kRefineWarps, smem_r, c.stream>>>(rp);
     VD_CUDA(cudaGetLastError());
     VD_CUDA(cudaMemcpyAsync(poses, d_p, size_t(n) * nc * 4, cudaMemcpyDeviceToHost, c.stream));
     VD_CUDA(cudaMemcpyAsync(e_out, d_e, n * 4, cudaMemcpyDeviceToHost, c.stream));

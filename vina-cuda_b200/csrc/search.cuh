@@ -265,11 +265,11 @@ struct SkipArmijo {
 // parallel: the inverse Hessian H (n x n, full storage) and the vectors gc,
 // pv, yv, mhy (n floats each) in the warp's shared memory.  Used by the
 // refinement (direct-sum score) and by the Monte-Carlo search with
-// --rilc_bfgs 0 (grid maps).  pair_atomics as in eval_pose_t.
-template <bool pair_atomics = false, class Inter>
+// --rilc_bfgs 0 (grid maps).  eval(skip): energy of the pose in s.m.x and,
+// unless skip(energy), its gradient in s.m.g.
+template <class Eval>
 __device__ float dense_bfgs(const LigView& L, const SearchMem& s, float* H, float* gc, float* pv, float* yv,
-                           float* mhy, const Inter& inter, const float4* smooth, float v_intra, float fix,
-                           float inv_fix, int max_steps, int lane, int& evals) {
+                           float* mhy, const Eval& eval, int max_steps, int lane, int& evals) {
     const int n = 6 + L.nt, nc = 7 + L.nt;
     for (int i = lane; i < n * n; i += 32) H[i] = (i / n == i % n) ? 1.f : 0.f;
     // One evaluation site (the entry evaluation and every line-search trial),
@@ -286,8 +286,7 @@ __device__ float dense_bfgs(const LigView& L, const SearchMem& s, float* H, floa
         // a trial that fails the Armijo test before the tenth reads no
         // gradient: its adjoint is skipped
         const float armijo = 0.0001f * alpha * pg;
-        const float fe = eval_pose_t<true, pair_atomics>(L, s.m, inter, smooth, v_intra, fix, inv_fix, lane,
-                                                         SkipArmijo{f0, armijo, !first && trial + 1 < 10});
+        const float fe = eval(SkipArmijo{f0, armijo, !first && trial + 1 < 10});
         ++evals;
         if (first) {
             first = false;
