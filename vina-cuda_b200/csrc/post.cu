@@ -64,6 +64,7 @@ struct ClusterParams {
     int32_t* kept;              // [n_ligs][20] item indices, -1 padded
     int32_t sort_n;             // power of two >= chains per ligand
     int32_t warp_floats;
+    int32_t warps;              // candidates placed at a time
 };
 
 __device__ __forceinline__ uint32_t ordered(float f) {
@@ -71,8 +72,18 @@ __device__ __forceinline__ uint32_t ordered(float f) {
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 
-__global__ void __launch_bounds__(256) cluster_kernel(ClusterParams p) {
+// One block per ligand.  Its serial part is the greedy pass: with one warp,
+// each candidate cost a pose load, its kinematics and up to 20 RMSDs one
+// after the other.  p.warps warps take the next candidates together, each
+// tests its own against the poses kept so far, and then the first survivor
+// is kept and the ones behind it test it, until none is left: the same poses
+// as taking candidates one by one.  6,500 chains of a 31-atom ligand, B200:
+// 382 us with 256 threads and one greedy warp, 101 us (half of it the sort).
+constexpr int kClusterThreads = 1024;
+
+__global__ void __launch_bounds__(kClusterThreads) cluster_kernel(ClusterParams p) {
     extern __shared__ float4 smem4[];
+    __shared__ int s_open[2];  // first survivor (warp index), alternating
     unsigned long long* keys = reinterpret_cast<unsigned long long*>(smem4);
     const int li = blockIdx.x;
     const int b0 = p.prefix[li], n = p.prefix[li + 1] - b0;
@@ -87,50 +98,64 @@ __global__ void __launch_bounds__(256) cluster_kernel(ClusterParams p) {
     __syncthreads();
     for (int size = 2; size <= p.sort_n; size <<= 1)  // bitonic sort, ascending
         for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int i = threadIdx.x; i < p.sort_n; i += blockDim.x) {
-                const int j = i ^ stride;
-                if (j > i) {
-                    const bool up = (i & size) == 0;
-                    const unsigned long long a = keys[i], b = keys[j];
-                    if ((a > b) == up) { keys[i] = b; keys[j] = a; }
-                }
+            for (int j = threadIdx.x; j < p.sort_n / 2; j += blockDim.x) {
+                const int i = 2 * j - (j & (stride - 1));  // lower index of the j-th exchange
+                const bool up = (i & size) == 0;
+                const unsigned long long a = keys[i], b = keys[i + stride];
+                if ((a > b) == up) { keys[i] = b; keys[i + stride] = a; }
             }
             __syncthreads();
         }
-    if (threadIdx.x >= 32) return;
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const LigView L = lig_view(p.pool, p.lig_off[li]);
     float* wbase = reinterpret_cast<float*>(keys + p.sort_n);
-    WarpMem m = carve(wbase, L.na, L.nn, L.np, L.nt);
-    float* kc = wbase + p.warp_floats;  // kept coordinates [20][na][3]
-    int nk = 0;
+    const WarpMem m = carve(wbase + size_t(min(wid, p.warps - 1)) * p.warp_floats, L.na, L.nn, L.np, L.nt);
+    float* kc = wbase + size_t(p.warps) * p.warp_floats;  // kept coordinates [20][na][3]
     const int nc = 7 + L.nt;
-    for (int r = 0; r < n && nk < p.max_keep; ++r) {
-        const unsigned long long k = keys[r];
-        if (k == ~0ull) break;
-        const int item = b0 + VD_DCLAMP(int(uint32_t(k)), 0, n - 1, kChkClusterKept);
-        for (int i = lane; i < nc; i += 32) m.x[i] = p.conf[size_t(item) * p.stride + i];
-        __syncwarp();
-        kinematics(L, m, lane);
-        bool close = false;
-        for (int j = 0; j < nk && !close; ++j) {
-            const float* c = kc + size_t(j) * 3 * L.na;
-            float acc = 0.f;
-            for (int i = lane; i < L.na; i += 32) {
-                const float dx = m.c[i].x - c[3 * i], dy = m.c[i].y - c[3 * i + 1], dz = m.c[i].z - c[3 * i + 2];
-                acc += dx * dx + dy * dy + dz * dz;
-            }
-            acc = warp_sum(acc);
-            close = sqrtf(acc / float(L.na)) < p.min_rmsd;
+    auto close_to = [&](int j) {
+        const float* c = kc + size_t(j) * 3 * L.na;
+        float acc = 0.f;
+        for (int i = lane; i < L.na; i += 32) {
+            const float dx = m.c[i].x - c[3 * i], dy = m.c[i].y - c[3 * i + 1], dz = m.c[i].z - c[3 * i + 2];
+            acc += dx * dx + dy * dy + dz * dz;
         }
-        if (close) continue;
-        float* c = kc + size_t(nk) * 3 * L.na;
-        for (int i = lane; i < L.na; i += 32) { c[3 * i] = m.c[i].x; c[3 * i + 1] = m.c[i].y; c[3 * i + 2] = m.c[i].z; }
-        if (lane == 0) p.kept[li * VD_MAX_MODES + nk] = item;
-        ++nk;
-        __syncwarp();
+        acc = warp_sum(acc);
+        return sqrtf(acc / float(L.na)) < p.min_rmsd;
+    };
+    int nk = 0;
+    if (threadIdx.x < 2) s_open[threadIdx.x] = p.warps;
+    __syncthreads();
+    for (int r0 = 0, turn = 0; r0 < n && nk < p.max_keep; r0 += p.warps) {
+        const int r = r0 + wid;
+        const unsigned long long k = (wid < p.warps && r < n) ? keys[r] : ~0ull;
+        bool open = k != ~0ull;  // finite energies sort first
+        int item = 0;
+        if (open) {
+            item = b0 + VD_DCLAMP(int(uint32_t(k)), 0, n - 1, kChkClusterKept);
+            for (int i = lane; i < nc; i += 32) m.x[i] = p.conf[size_t(item) * p.stride + i];
+            __syncwarp();
+            kinematics(L, m, lane);
+            for (int j = 0; j < nk && open; ++j) open = !close_to(j);
+        }
+        while (nk < p.max_keep) {
+            if (open && lane == 0) atomicMin(&s_open[turn], wid);
+            __syncthreads();
+            const int first = s_open[turn];
+            turn ^= 1;
+            if (first < p.warps && wid == first) {
+                float* c = kc + size_t(nk) * 3 * L.na;
+                for (int i = lane; i < L.na; i += 32) { c[3 * i] = m.c[i].x; c[3 * i + 1] = m.c[i].y; c[3 * i + 2] = m.c[i].z; }
+                if (lane == 0) p.kept[li * VD_MAX_MODES + nk] = item;
+                open = false;
+            }
+            __syncthreads();
+            if (threadIdx.x == 0) s_open[turn ^ 1] = p.warps;  // read by all above, next used a turn later
+            if (first >= p.warps) break;  // no survivor: next candidates
+            ++nk;
+            if (open) open = !close_to(nk - 1);
+        }
     }
-    for (int j = nk + lane; j < VD_MAX_MODES; j += 32) p.kept[li * VD_MAX_MODES + j] = -1;
+    for (int j = nk + threadIdx.x; j < VD_MAX_MODES; j += blockDim.x) p.kept[li * VD_MAX_MODES + j] = -1;
 }
 
 // ------------------------------------------------------------ refine
@@ -628,50 +653,75 @@ __device__ __forceinline__ double warp_sum_d(double v) {
     return v;
 }
 
-// model.cpp:1206-1219 (eval_interacting_pairs, eval_fast, curl 1000)
-__device__ double intra_fast(const LigView& L, const double* c, const double* fastd, int lane) {
+// model.cpp:1206-1219 (eval_interacting_pairs, eval_fast, curl 1000): this
+// lane's share of the pairs tid, tid + step, ..
+__device__ __forceinline__ double intra_fast(const LigView& L, const double* c, const double* fastd, int tid, int step) {
     double e = 0;
-    for (int p = lane; p < L.np; p += 32) {
-        const int2 pr = L.pairs[p];
+#pragma unroll 4
+    for (int p = tid; p < L.np; p += step) {
+        const int2 pr = __ldg(&L.pairs[p]);
         const int a = pr.x & 0xffff, b = pr.x >> 16;
         const double dx = c[3 * a] - c[3 * b], dy = c[3 * a + 1] - c[3 * b + 1], dz = c[3 * a + 2] - c[3 * b + 2];
         const double r2 = (dx * dx + dy * dy) + dz * dz;
         if (r2 < 64.0) {
-            double t = fastd[size_t(pr.y) * kBins + int(32.0 * r2)];
+            double t = __ldg(&fastd[size_t(pr.y) * kBins + int(32.0 * r2)]);
             if (t > 0) t *= 1000.0 / (1000.0 + t);
             e += t;
         }
     }
-    return warp_sum_d(e);
+    return e;
 }
 
-// non_cache.cpp:20-55 (non_cache::eval, eval_fast, curl 1000, slope 1e6)
-__device__ double inter_fast(const LigView& L, const RecView& R, const double* c, const double* fastd, int lane) {
+// non_cache.cpp:20-55 (non_cache::eval, eval_fast, curl 1000, slope 1e6) of the
+// atom groups g, g + step, ..: four atoms at a time, lanes over a cell's
+// receptor atoms (a lane walking its own atom's list alone paid three dependent
+// loads per neighbour).  Same value in every lane.
+__device__ __forceinline__ double inter_fast(const LigView& L, const RecView& R, const double* c, const double* fastd,
+                                             int g, int step, int lane) {
     double e = 0;
-    for (int i = lane; i < L.na; i += 32) {
-        const int t1 = __float_as_int(L.atoms[i].w) & 0xff;
-        double a[3] = {c[3 * i], c[3 * i + 1], c[3 * i + 2]}, oob = 0;
-        for (int d = 0; d < 3; ++d) {
-            if (a[d] < R.gb[d]) { oob += fabs(a[d] - R.gb[d]); a[d] = R.gb[d]; }
-            else if (a[d] > R.ge[d]) { oob += fabs(a[d] - R.ge[d]); a[d] = R.ge[d]; }
+    for (int i0 = 4 * g; i0 < L.na; i0 += 4 * step) {
+        double a[4][3], oob[4], sum[4];
+        int t1[4], q0[4], q1[4], longest = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int i = min(i0 + j, L.na - 1);
+            t1[j] = __float_as_int(__ldg(&L.atoms[i].w)) & 0xff;
+            oob[j] = sum[j] = 0;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                a[j][d] = c[3 * i + d];
+                if (a[j][d] < R.gb[d]) { oob[j] += fabs(a[j][d] - R.gb[d]); a[j][d] = R.gb[d]; }
+                else if (a[j][d] > R.ge[d]) { oob[j] += fabs(a[j][d] - R.ge[d]); a[j][d] = R.ge[d]; }
+            }
+            const int ce = cell_of(R, float(a[j][0]), float(a[j][1]), float(a[j][2]));
+            q0[j] = __ldg(&R.cell_start[ce]);
+            q1[j] = __ldg(&R.cell_start[ce + 1]);
+            longest = max(longest, q1[j] - q0[j]);
         }
-        oob *= 1e6;
-        const int ce = cell_of(R, float(a[0]), float(a[1]), float(a[2]));
-        double this_e = 0;
-        for (int q = R.cell_start[ce]; q < R.cell_start[ce + 1]; ++q) {
-            const double4 b = R.recd[R.cell_list[q]];
-            const double rx = a[0] - b.x, ry = a[1] - b.y, rz = a[2] - b.z;
-            const double r2 = (rx * rx + ry * ry) + rz * rz;
-            if (r2 < 64.0) {
-                const int t2 = int(b.w);
-                const int tp = (t1 <= t2) ? t1 + t2 * (t2 + 1) / 2 : t2 + t1 * (t1 + 1) / 2;
-                this_e += fastd[size_t(tp) * kBins + int(32.0 * r2)];
+        for (int k = lane; k < longest; k += 32) {
+            int idx[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) idx[j] = q0[j] + k < q1[j] ? __ldg(&R.cell_list[q0[j] + k]) : -1;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const double4 b = R.recd[max(idx[j], 0)];  // entry 0 always exists
+                const double rx = a[j][0] - b.x, ry = a[j][1] - b.y, rz = a[j][2] - b.z;
+                const double r2 = (rx * rx + ry * ry) + rz * rz;
+                if (idx[j] >= 0 && r2 < 64.0) {
+                    const int t2 = int(b.w);
+                    const int tp = (t1[j] <= t2) ? t1[j] + t2 * (t2 + 1) / 2 : t2 + t1[j] * (t1[j] + 1) / 2;
+                    sum[j] += __ldg(&fastd[size_t(tp) * kBins + int(32.0 * r2)]);
+                }
             }
         }
-        if (this_e > 0) this_e *= 1000.0 / (1000.0 + this_e);
-        e += this_e + oob;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            double this_e = warp_sum_d(sum[j]);
+            if (this_e > 0) this_e *= 1000.0 / (1000.0 + this_e);
+            if (i0 + j < L.na) e += this_e + oob[j] * 1e6;
+        }
     }
-    return warp_sum_d(e);
+    return e;
 }
 
 // Kept chain results -> refinement buffer ([ligand][20] slots).
@@ -688,19 +738,22 @@ __global__ void gather_kernel(const int32_t* kept, const float* conf, const floa
 // model.cpp:1485-1523: RMSD upper bound (each heavy atom to the same atom)
 // and lower bound (each heavy atom to the nearest atom of the same element,
 // the larger of the two directions) between heavy-atom coordinate sets a and
-// b ([na][3] floats); sums in double.  Same value in every lane.
-__device__ void rmsd_bounds(const LigView& L, const float* a, const float* b, int lane, double& lb, double& ub) {
+// b ([na][3], taken as floats); sums in double.  Same value in every lane.
+template <class T>
+__device__ void rmsd_bounds(const LigView& L, const T* pa, const T* pb, int lane, double& lb, double& ub) {
+    const auto a = [pa](int k) { return float(pa[k]); };
+    const auto b = [pb](int k) { return float(pb[k]); };
     double su = 0, s1 = 0, s2 = 0;
     for (int i = lane; i < L.na; i += 32) {
         const int ei = (__float_as_int(L.atoms[i].w) >> 16) & 0xff;
         double d2 = 0, m1 = DBL_MAX, m2 = DBL_MAX;
-        for (int d = 0; d < 3; ++d) d2 += double(a[3 * i + d] - b[3 * i + d]) * double(a[3 * i + d] - b[3 * i + d]);
+        for (int d = 0; d < 3; ++d) d2 += double(a(3 * i + d) - b(3 * i + d)) * double(a(3 * i + d) - b(3 * i + d));
         for (int q = 0; q < L.na; ++q) {
             if (((__float_as_int(L.atoms[q].w) >> 16) & 0xff) != ei) continue;
             double t1 = 0, t2 = 0;
             for (int d = 0; d < 3; ++d) {
-                t1 += double(a[3 * i + d] - b[3 * q + d]) * double(a[3 * i + d] - b[3 * q + d]);
-                t2 += double(b[3 * i + d] - a[3 * q + d]) * double(b[3 * i + d] - a[3 * q + d]);
+                t1 += double(a(3 * i + d) - b(3 * q + d)) * double(a(3 * i + d) - b(3 * q + d));
+                t2 += double(b(3 * i + d) - a(3 * q + d)) * double(b(3 * i + d) - a(3 * q + d));
             }
             m1 = fmin(m1, t1);
             m2 = fmin(m2, t2);
@@ -712,142 +765,160 @@ __device__ void rmsd_bounds(const LigView& L, const float* a, const float* b, in
     lb = fmax(sqrt(s1 / L.na), sqrt(s2 / L.na));
 }
 
+// Doubles one warp needs for a pose: body frames, then its coordinates.
+__host__ __device__ inline int pose_doubles(int na, int nn) { return 16 * nn + 3 * na; }
+
 // RMSD bounds of poses to pose 0 (vd_rmsd_bounds): heavy-atom coordinates in
-// double, stored as floats as the output stage stores its kept modes.
-__global__ void __launch_bounds__(32) rmsd_poses_kernel(const float4* pool, const int64_t* off, const float* poses,
-                                                         int n, int stride, double* out) {
+// double, taken as floats as the output stage does.  A warp per pose, and one
+// more per block for pose 0.  20 poses of 45 atoms, B200: 278 us with one
+// warp for all poses, 20 us.
+constexpr int kRmsdWarps = 4;
+__global__ void __launch_bounds__(32 * (kRmsdWarps + 1)) rmsd_poses_kernel(const float4* pool, const int64_t* off,
+                                                                           const float* poses, int n, int stride,
+                                                                           double* out) {
     extern __shared__ double smemd[];
-    const int lane = threadIdx.x;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const LigView L = lig_view(pool, off[0]);
-    double* nd = smemd;
-    double* c = nd + 16 * L.nn;
-    float* k0 = reinterpret_cast<float*>(c + 3 * L.na);
-    float* ki = k0 + 3 * L.na;
-    coords_d(L, poses, nd, c, lane);
-    for (int a = lane; a < 3 * L.na; a += 32) k0[a] = float(c[a]);
-    __syncwarp();
-    for (int i = 0; i < n; ++i) {
-        coords_d(L, poses + size_t(i) * stride, nd, c, lane);
-        for (int a = lane; a < 3 * L.na; a += 32) ki[a] = float(c[a]);
-        __syncwarp();
-        double lb, ub;
-        rmsd_bounds(L, ki, k0, lane, lb, ub);
-        if (lane == 0) {
-            out[2 * i] = lb;
-            out[2 * i + 1] = ub;
-        }
-        __syncwarp();
+    const int per = pose_doubles(L.na, L.nn);
+    const int i = wid < kRmsdWarps ? int(blockIdx.x) * kRmsdWarps + wid : 0;
+    double* nd = smemd + wid * per;
+    if (i < n) coords_d(L, poses + size_t(i) * stride, nd, nd + 16 * L.nn, lane);
+    __syncthreads();
+    if (wid == kRmsdWarps || i >= n) return;
+    double lb, ub;
+    rmsd_bounds(L, nd + 16 * L.nn, smemd + kRmsdWarps * per + 16 * L.nn, lane, lb, ub);
+    if (lane == 0) {
+        out[2 * i] = lb;
+        out[2 * i + 1] = ub;
     }
 }
 
-// Adjusted score and intramolecular energy of up to 20 poses (vd_score).
-__global__ void __launch_bounds__(32) score_poses_kernel(const float4* pool, const int64_t* off, const float* poses,
-                                                          int n, int stride, RecView R, const double* fastd,
-                                                          double w_rot, double* out) {
+// Receptor-ligand and intramolecular energy of a pose (vd_score; the caller
+// relates them to pose 0's).  A block per pose: warp 0 places the atoms, all
+// warps share them and the pairs.  20 poses of 45 atoms, B200: 1,386 us with
+// one warp for all poses, 24 us (a launch, a pose placement in FP64, one round of
+// neighbours).
+constexpr int kScoreWarps = 8;
+__global__ void __launch_bounds__(32 * kScoreWarps) score_poses_kernel(const float4* pool, const int64_t* off,
+                                                                       const float* poses, int stride, RecView R,
+                                                                       const double* fastd, double* out) {
     extern __shared__ double smemd[];
-    const int lane = threadIdx.x;
+    __shared__ double part[2][kScoreWarps];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, i = blockIdx.x;
     const LigView L = lig_view(pool, off[0]);
-    double* nd = smemd;
-    double* c = nd + 16 * L.nn;
-    double intra0 = 0;
-    for (int i = 0; i < n; ++i) {
-        coords_d(L, poses + size_t(i) * stride, nd, c, lane);
-        const double intra = intra_fast(L, c, fastd, lane);
-        if (i == 0) intra0 = intra;
-        const double e = inter_fast(L, R, c, fastd, lane) + intra;
-        const double x = e - intra0, y = 1 + w_rot * double(L.num_tors) / 5.0;
-        if (lane == 0) {
-            out[2 * i] = (fabs(x) < DBL_EPSILON) ? 0.0 : x / y;
-            out[2 * i + 1] = intra;
-        }
-        __syncwarp();
+    double* c = smemd + 16 * L.nn;
+    if (wid == 0) coords_d(L, poses + size_t(i) * stride, smemd, c, lane);
+    __syncthreads();
+    const double inter = inter_fast(L, R, c, fastd, wid, kScoreWarps, lane);
+    const double intra = warp_sum_d(intra_fast(L, c, fastd, threadIdx.x, 32 * kScoreWarps));
+    if (lane == 0) {
+        part[0][wid] = inter;
+        part[1][wid] = intra;
+    }
+    __syncthreads();
+    if (threadIdx.x < 2) {
+        double e = 0;
+        for (int w = 0; w < kScoreWarps; ++w) e += part[threadIdx.x][w];
+        out[2 * i + threadIdx.x] = e;
     }
 }
 
-__global__ void __launch_bounds__(32) score_kernel(ScoreParams p) {
+// Final scores, order, redundancy and RMSD bounds of a ligand's refined poses:
+// a block per ligand, a warp per pose, every pose's coordinates kept in shared
+// memory.  One warp going through them took 938 us for a 31-atom ligand's 20
+// poses, latency all of it; 88 us.
+__global__ void __launch_bounds__(32 * VD_MAX_MODES) score_kernel(ScoreParams p) {
     extern __shared__ double smemd[];
-    const int li = blockIdx.x, lane = threadIdx.x;
+    __shared__ int order[VD_MAX_MODES], kept[VD_MAX_MODES], s_nk;
+    __shared__ double adj[VD_MAX_MODES], s_intra[VD_MAX_MODES];
+    __shared__ unsigned near[VD_MAX_MODES];  // bit q: within min_rmsd of the pose q places up the order
+    const int li = blockIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const LigView L = lig_view(p.pool, p.lig_off[li]);
-    double* nd = smemd;                        // [nn][8] + [nn][8]
-    double* c = nd + 16 * L.nn;                // [na][3]
-    float* kc = reinterpret_cast<float*>(c + 3 * L.na);  // [20][na][3]
-    __shared__ int order[VD_MAX_MODES], kept[VD_MAX_MODES];
-    __shared__ double adj[VD_MAX_MODES];
+    const int per = pose_doubles(L.na, L.nn);
+    const auto coords = [&](int i) { return smemd + size_t(i) * per + 16 * L.nn; };
     const int n = p.n_in[li];
     const float* poses = p.poses + size_t(li) * VD_MAX_MODES * p.stride;
     const float* er = p.e_ref + size_t(li) * VD_MAX_MODES;
     vd_dock_result* out = p.out + li;
-    if (lane == 0) {
-        for (int i = 0; i < n; ++i) order[i] = i;
-        for (int i = 1; i < n; ++i)  // stable insertion sort by refined energy
-            for (int j = i; j > 0 && er[order[j]] < er[order[j - 1]]; --j) {
-                const int t = order[j]; order[j] = order[j - 1]; order[j - 1] = t;
-            }
-    }
-    __syncwarp();
-    double intra_best = 0;
-    if (n > 0) {
-        coords_d(L, poses + size_t(order[0]) * p.stride, nd, c, lane);
-        intra_best = intra_fast(L, c, p.fastd, lane);
-    }
+    // the best refined pose: the first of a stable ascending sort, which no
+    // pose passes a NaN in
+    int best = 0;
     for (int i = 0; i < n; ++i) {
+        if (!(er[i] == er[i])) break;
+        if (er[i] < er[best]) best = i;
+    }
+    const bool valid = w < n && er[w] < FLT_MAX;
+    double e = 0;
+    if (valid || (w == best && n > 0)) {
+        coords_d(L, poses + size_t(w) * p.stride, smemd + size_t(w) * per, coords(w), lane);
+        const double intra = warp_sum_d(intra_fast(L, coords(w), p.fastd, lane, 32));
+        if (lane == 0) s_intra[w] = intra;
+        if (valid) e = inter_fast(L, p.R, coords(w), p.fastd, 0, 1, lane) + intra;
+    }
+    __syncthreads();
+    if (w < n && lane == 0) {
         double v = DBL_MAX;
-        if (er[i] < FLT_MAX) {
-            coords_d(L, poses + size_t(i) * p.stride, nd, c, lane);
-            const double e = inter_fast(L, p.R, c, p.fastd, lane) + intra_fast(L, c, p.fastd, lane);
-            const double x = e - intra_best, y = 1 + p.w_rot * double(L.num_tors) / 5.0;
+        if (valid) {
+            const double x = e - s_intra[best], y = 1 + p.w_rot * double(L.num_tors) / 5.0;
             v = (fabs(x) < DBL_EPSILON) ? 0.0 : x / y;  // smooth_div, everything.cpp:232-236
         }
-        if (lane == 0) adj[i] = v;
+        adj[w] = v;
     }
-    __syncwarp();
-    if (lane == 0) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
         for (int i = 0; i < n; ++i) order[i] = i;
-        for (int i = 1; i < n; ++i)
+        for (int i = 1; i < n; ++i)  // stable insertion sort
             for (int j = i; j > 0 && adj[order[j]] < adj[order[j - 1]]; --j) {
                 const int t = order[j]; order[j] = order[j - 1]; order[j - 1] = t;
             }
     }
-    __syncwarp();
-    int nk = 0;  // remove_redundant (main.cpp:172-178) then the mode cut
-    for (int r = 0; r < n; ++r) {
-        const int i = order[r];
-        if (!(adj[i] < 0.1 * DBL_MAX)) break;
-        if (nk >= p.num_modes) break;
-        if (nk > 0 && adj[i] > adj[kept[0]] + p.energy_range) break;
-        coords_d(L, poses + size_t(i) * p.stride, nd, c, lane);
-        bool close = false;
-        for (int j = 0; j < nk && !close; ++j) {
-            const float* k = kc + size_t(j) * 3 * L.na;
+    __syncthreads();
+    if (w < n && adj[order[w]] < 0.1 * DBL_MAX) {
+        const double* c = coords(order[w]);
+        unsigned bits = 0;
+        for (int j = 0; j < w; ++j) {
+            if (!(adj[order[j]] < 0.1 * DBL_MAX)) continue;
+            const double* k = coords(order[j]);
             double acc = 0;
             for (int a = lane; a < L.na; a += 32)
-                for (int d = 0; d < 3; ++d) acc += (c[3 * a + d] - k[3 * a + d]) * (c[3 * a + d] - k[3 * a + d]);
+                for (int d = 0; d < 3; ++d) {
+                    const double x = c[3 * a + d] - double(float(k[3 * a + d]));
+                    acc += x * x;
+                }
             acc = warp_sum_d(acc);
-            close = sqrt(acc / L.na) < p.min_rmsd;
+            if (sqrt(acc / L.na) < p.min_rmsd) bits |= 1u << j;
         }
-        if (close) continue;
-        float* k = kc + size_t(nk) * 3 * L.na;
-        for (int a = lane; a < 3 * L.na; a += 32) k[a] = float(c[a]);
-        if (lane == 0) kept[nk] = i;
-        ++nk;
-        __syncwarp();
+        if (lane == 0) near[w] = bits;
     }
-    __syncwarp();
-    // outputs with RMSD bounds to mode 1 (model.cpp:1485-1523)
-    for (int j = 0; j < nk; ++j) {
-        double lb, ub;
-        rmsd_bounds(L, kc + size_t(j) * 3 * L.na, kc, lane, lb, ub);
-        const int i = kept[j];
-        if (lane == 0) {
-            out->energy[j] = float(adj[i]);
-            out->rmsd_ub[j] = float(ub);
-            out->rmsd_lb[j] = float(lb);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int nk = 0;  // remove_redundant (main.cpp:172-178) then the mode cut
+        unsigned taken = 0;
+        for (int r = 0; r < n; ++r) {
+            const int i = order[r];
+            if (!(adj[i] < 0.1 * DBL_MAX)) break;
+            if (nk >= p.num_modes) break;
+            if (nk > 0 && adj[i] > adj[kept[0]] + p.energy_range) break;
+            if (near[r] & taken) continue;
+            taken |= 1u << r;
+            kept[nk++] = i;
         }
-        for (int q = lane; q < 7 + L.nt; q += 32) out->pose[j][q] = poses[size_t(i) * p.stride + q];
-    }
-    if (lane == 0) {
+        s_nk = nk;
         out->n_modes = nk;
         out->ntors = L.nt;
+    }
+    __syncthreads();
+    // outputs with RMSD bounds to mode 1 (model.cpp:1485-1523)
+    if (w < s_nk) {
+        double lb, ub;
+        rmsd_bounds(L, coords(kept[w]), coords(kept[0]), lane, lb, ub);
+        const int i = kept[w];
+        if (lane == 0) {
+            out->energy[w] = float(adj[i]);
+            out->rmsd_ub[w] = float(ub);
+            out->rmsd_lb[w] = float(lb);
+        }
+        for (int q = lane; q < 7 + L.nt; q += 32) out->pose[w][q] = poses[size_t(i) * p.stride + q];
     }
 }
 
@@ -1051,8 +1122,12 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     cp.kept = d_kept;
     cp.sort_n = sort_n;
     cp.warp_floats = max_wf;
-    const size_t smem_c = size_t(sort_n) * 8 + size_t(max_wf) * 4 + size_t(VD_MAX_MODES) * 3 * max_na * 4;
-    VD_CHECK(smem_c <= 227 * 1024, VD_ERR_CAPACITY, "cluster kernel shared memory exceeds 227 KB");
+    // as many candidates at a time as the shared memory left holds
+    const size_t smem_c1 = size_t(sort_n) * 8 + size_t(VD_MAX_MODES) * 3 * max_na * 4, b_wf = size_t(max_wf) * 4;
+    VD_CHECK(smem_c1 + b_wf <= 227 * 1024, VD_ERR_CAPACITY, "cluster kernel shared memory exceeds 227 KB");
+    cp.warps = int(std::min<size_t>(kClusterThreads / 32, (227 * 1024 - 64 - smem_c1) / b_wf));
+    cp.warps = std::max(1, cp.warps);
+    const size_t smem_c = smem_c1 + cp.warps * b_wf;
     VD_CUDA(cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_c)));
     // refine
     const bool refine = sp.refine != 0;
@@ -1094,17 +1169,18 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     sc.energy_range = sp.energy_range > 0 ? sp.energy_range : 3.0;
     sc.min_rmsd = 1.0;
     sc.out = d_out;
-    const size_t smem_s = size_t(16 * max_nn + 3 * max_na) * 8 + size_t(VD_MAX_MODES) * 3 * max_na * 4;
+    const size_t smem_s = size_t(VD_MAX_MODES) * pose_doubles(max_na, max_nn) * 8;
+    VD_CHECK(smem_s <= 226 * 1024, VD_ERR_CAPACITY, "score kernel shared memory exceeds 226 KB");
     VD_CUDA(cudaFuncSetAttribute(score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_s)));
     const int stride = db.stride;
     const float* conf = db.d_conf;
     const float* e = db.d_e;
     pp.launch = [=](cudaStream_t stream) {
-        cluster_kernel<<<n, 256, smem_c, stream>>>(cp);
+        cluster_kernel<<<n, kClusterThreads, smem_c, stream>>>(cp);
         // gather kept poses (missing slots get e = FLT_MAX)
         gather_kernel<<<n * VD_MAX_MODES, 64, 0, stream>>>(d_kept, conf, e, stride, n * VD_MAX_MODES, d_rp, d_re);
         if (refine) refine_kernel<<<blocks_r, 32 * kRefineWarps, smem_r, stream>>>(rp);
-        score_kernel<<<n, 32, smem_s, stream>>>(sc);
+        score_kernel<<<n, 32 * VD_MAX_MODES, smem_s, stream>>>(sc);
         return cudaGetLastError();
     };
     return VD_OK;
@@ -1345,15 +1421,19 @@ vd_status vd_score(vd_ctx* h, int32_t lig, int32_t n, const float* poses, float*
     VD_CUDA(cudaMemcpyAsync(d_p, poses, size_t(n) * nc * 4, cudaMemcpyHostToDevice, c.stream));
     const int64_t off = L.pool_offset;
     VD_CUDA(cudaMemcpyAsync(d_off, &off, 8, cudaMemcpyHostToDevice, c.stream));
-    score_poses_kernel<<<1, 32, size_t(16 * L.h.n_nodes + 3 * L.h.n_atoms) * 8, c.stream>>>(
-        c.d_pool, d_off, d_p, n, nc, rec_view(c), c.d_fastd, 0.1 * (c.weights[5] + 1), d_o);
+    VD_CUDA(cudaFuncSetAttribute(score_poses_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(pose_doubles(L.h.n_atoms, L.h.n_nodes)) * 8));
+    score_poses_kernel<<<n, 32 * kScoreWarps, size_t(pose_doubles(L.h.n_atoms, L.h.n_nodes)) * 8, c.stream>>>(
+        c.d_pool, d_off, d_p, nc, rec_view(c), c.d_fastd, d_o);
     VD_CUDA(cudaGetLastError());
     std::vector<double> o(size_t(n) * 2);
     VD_CUDA(cudaMemcpyAsync(o.data(), d_o, o.size() * 8, cudaMemcpyDeviceToHost, c.stream));
     VD_CUDA(cudaStreamSynchronize(c.stream));
     { const vd_status cs = take_device_checks("scoring kernel"); if (cs != VD_OK) return cs; }
+    const double y = 1 + 0.1 * (c.weights[5] + 1) * double(L.h.num_tors) / 5.0;
     for (int i = 0; i < n; ++i) {
-        if (adjusted) adjusted[i] = float(o[2 * i]);
+        const double x = o[2 * i] + o[2 * i + 1] - o[1];  // relative to pose 0's intramolecular energy
+        if (adjusted) adjusted[i] = float(std::fabs(x) < DBL_EPSILON ? 0.0 : x / y);
         if (intra) intra[i] = float(o[2 * i + 1]);
     }
     return VD_OK;
@@ -1378,8 +1458,10 @@ vd_status vd_rmsd_bounds(vd_ctx* h, int32_t lig, int32_t n, const float* poses, 
     VD_CUDA(cudaMemcpyAsync(d_p, poses, size_t(n) * nc * 4, cudaMemcpyHostToDevice, c.stream));
     const int64_t off = L.pool_offset;
     VD_CUDA(cudaMemcpyAsync(d_off, &off, 8, cudaMemcpyHostToDevice, c.stream));
-    const size_t smem = size_t(16 * L.h.n_nodes + 3 * L.h.n_atoms) * 8 + size_t(6 * L.h.n_atoms) * 4;
-    rmsd_poses_kernel<<<1, 32, smem, c.stream>>>(c.d_pool, d_off, d_p, n, nc, d_o);
+    const size_t smem = size_t(kRmsdWarps + 1) * pose_doubles(L.h.n_atoms, L.h.n_nodes) * 8;
+    VD_CUDA(cudaFuncSetAttribute(rmsd_poses_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    rmsd_poses_kernel<<<(n + kRmsdWarps - 1) / kRmsdWarps, 32 * (kRmsdWarps + 1), smem, c.stream>>>(c.d_pool, d_off, d_p,
+                                                                                                   n, nc, d_o);
     VD_CUDA(cudaGetLastError());
     std::vector<double> o(size_t(n) * 2);
     VD_CUDA(cudaMemcpyAsync(o.data(), d_o, o.size() * 8, cudaMemcpyDeviceToHost, c.stream));
