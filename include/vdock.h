@@ -92,7 +92,9 @@ typedef struct {
     int32_t  launch_shape;    /* docking kernel shape: 0 = autotuned per
                                  workload (among 1, 4, 5), 1/2/3/4/5 =
                                  64/48/40/80/128 registers per thread
-                                 (8/10/12/6/4 blocks of 4 chains per SM);
+                                 (8/10/12/6/4 blocks of 4 chains per SM; with
+                                 few chains shape 5 runs a team of 4 warps
+                                 per chain, and 0 takes it in the plain form);
                                  results do not depend on it                */
     int32_t  dense_bfgs;      /* local search of the Monte-Carlo steps:
                                  0 = RILC-BFGS (--rilc_bfgs 1, default,

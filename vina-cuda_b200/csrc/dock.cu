@@ -75,13 +75,24 @@ enum : int { kCsItem, kCsLig, kCsChain, kCsUid, kCsDepth, kCsSteps, kCsEvals0, k
 enum : int { kCfCurrent, kCfBest };
 static_assert(kCsFloats + kCfBest + 1 <= kChainWords, "chain scalars exceed their shared words");
 
-template <bool persistent, int MINB, bool dense = false>
-__global__ void __launch_bounds__(128, MINB) dock_kernel(DockParams p) {
+//
+// team > 1: a block is one chain, evaluated by a team of warps (eval.cuh).
+template <bool persistent, int MINB, bool dense = false, int team = 1>
+__global__ void __launch_bounds__(team > 1 ? 32 * team : 128, MINB) dock_kernel(DockParams p) {
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float* base = reinterpret_cast<float*>(smem4) + size_t(wid) * p.warp_floats;
+    float* base = reinterpret_cast<float*>(smem4) + (team > 1 ? size_t(0) : size_t(wid) * p.warp_floats);
+    const PairTeam tm = pair_team(base + p.warp_floats);
+    if (team > 1 && wid > 0) {
+        const auto view = [&](int li, LigView& L, WarpMem& m) {
+            L = lig_view(p.pool, __ldg(&p.lig_off[VD_DCLAMP(li, 0, p.n_ligs - 1, kChkItem)]));
+            m = carve(base, L.na, L.nn, L.np, L.nt);
+        };
+        pair_team_helper<team>(view, p.smooth, p.ep.v_intra, p.ep.fix, wid, lane, tm);
+        return;
+    }
     int evals = 0;
-    int item = persistent ? 0 : blockIdx.x * p.warps_per_block + wid;
+    int item = persistent ? 0 : team > 1 ? int(blockIdx.x) : blockIdx.x * p.warps_per_block + wid;
     for (;;) {
         if (persistent) {
             int v = 0;
@@ -115,8 +126,16 @@ __global__ void __launch_bounds__(128, MINB) dock_kernel(DockParams p) {
             cs[kCsRuns] = 0;
             cf[kCfCurrent] = FLT_MAX;
             cf[kCfBest] = INFINITY;
+            if (team > 1) *tm.work = 1 + li0;  // the helpers wait at barrier 1
         }
         __syncwarp();
+        const auto eval = [&](const auto& skip) {
+            const GridInter gi{&p.G, p.ep.v_inter, p.ep.slope};
+            if constexpr (team > 1)
+                return eval_pose_team<team>(L, s.m, gi, p.ep.inv_fix, lane, tm, skip);
+            else
+                return eval_pose_t<true, true>(L, s.m, gi, p.smooth, p.ep.v_intra, p.ep.fix, p.ep.inv_fix, lane, skip);
+        };
         init_pose(xt, L.nt, p.seed, uint32_t(cs[kCsUid]), uint32_t(cs[kCsChain]), p.lo, p.hi, lane);
         copy_conf(xt, xb, nc, lane);
         for (int step = 0; step < cs[kCsDepth]; ++step) {
@@ -136,11 +155,6 @@ __global__ void __launch_bounds__(128, MINB) dock_kernel(DockParams p) {
                     float* pv = gc + pad4(n);
                     float* yv = pv + pad4(n);
                     float* mhy = yv + pad4(n);
-                    const GridInter gi{&p.G, p.ep.v_inter, p.ep.slope};
-                    const auto eval = [&](const SkipArmijo& skip) {
-                        return eval_pose_t<true, true>(L, s.m, gi, p.smooth, p.ep.v_intra, p.ep.fix, p.ep.inv_fix,
-                                                       lane, skip);
-                    };
                     ce = dense_bfgs(L, s, H, gc, pv, yv, mhy, eval, cs[kCsSteps], lane, evals);
                 } else {
                     // visited history (visited.cuh:48-227, quasi_newton.cuh:1937-1943):
@@ -151,7 +165,7 @@ __global__ void __launch_bounds__(128, MINB) dock_kernel(DockParams p) {
                     const bool skip = p.visited && runs >= 10 * (6 + L.nt);
                     __syncwarp();
                     if (lane == 0 && !skip) cs[kCsRuns] = runs + 1;
-                    ce = rilc_bfgs(L, s, p.G, p.smooth, p.ep, cs[kCsSteps], lane, evals, skip);
+                    ce = rilc_bfgs(L, s, eval, cs[kCsSteps], lane, evals, skip);
                 }
                 const int stp = cs[kCsStep];
                 float tmp_e = cf[kCfCurrent], best_e = cf[kCfBest];
@@ -197,6 +211,11 @@ __global__ void __launch_bounds__(128, MINB) dock_kernel(DockParams p) {
         if (!persistent) break;
     }
     if (lane == 0 && evals) atomicAdd(p.evals, (unsigned long long)evals);
+    if (team > 1) {
+        if (lane == 0) *tm.work = 0;
+        __syncwarp();
+        team_arrive<team>(1);
+    }
 }
 
 // Resident 4-warp blocks per SM each launch shape's register budget targets.
@@ -222,6 +241,26 @@ DockFn dense_dock_fn(int& shape) {
         case 4: return dock_kernel<persistent, 4, true>;
         default: shape = 0; return dock_kernel<persistent, 8, true>;
     }
+}
+
+// Few chains leave most warp slots empty and a chain is one long dependency:
+// frames, atoms, grid lookup, pairs, adjoint, optimiser.  A team of four warps
+// per chain takes the pairs off it (three warps compute them while the first
+// looks up the grid).  Chains of one ligand, 60 steps, 22 A box, ms on B200,
+// one warp per chain at 128 registers -> team:
+//   24 atoms / 5 torsions:  64 chains 9.96 -> 7.55, 592 11.39 -> 9.41, 1,024 11.87 -> 10.07,
+//                           1,500 12.99 -> 16.13
+//   40 atoms / 10 torsions: 256 chains 28.3 -> 16.7, 1,024 29.7 -> 20.9, 2,048 33.6 -> 36.7
+// so it is used while all chains are resident at once: 7 blocks per SM, the most
+// whose 72 registers per thread hold the kernel without spills.  (Teams of 2, 3, 6
+// and 8 warps: 10.94, 10.52, 16.1 and 16.4 at 1,024 chains of the first ligand.)
+constexpr int kTeamWarps = 4;   // warps per chain
+constexpr int kTeamChains = 7;  // chains resident per SM
+constexpr int kWideShape = 4;   // the 128-register shape
+template <bool persistent>
+DockFn team_dock_fn(bool dense) {
+    return dense ? DockFn(dock_kernel<persistent, kTeamChains, true, kTeamWarps>)
+                 : DockFn(dock_kernel<persistent, kTeamChains, false, kTeamWarps>);
 }
 
 // Shared-memory floats of the dense optimiser's state: H (n x n) and the
@@ -292,7 +331,7 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     std::vector<int64_t> off(n);
     std::vector<int32_t> prefix(n + 1, 0), depth(n), steps(n);
     std::vector<uint32_t> uid(n);
-    int max_wf = 0, max_nt = 0;
+    int max_wf = 0, max_nt = 0, max_sp = 0;
     for (int i = 0; i < n; ++i) {
         st = check_ligand_maps(c, ligs[i]);
         if (st != VD_OK) return st;
@@ -305,6 +344,7 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
         max_wf = std::max(max_wf, lig_warp_floats(L) + 4 * pad4(7 + L.h.ntors) + kChainWords +
                                       (sp.dense_bfgs ? dense_floats(L.h.ntors) : 0));
         max_nt = std::max(max_nt, L.h.ntors);
+        max_sp = std::max(max_sp, L.h.sp_iters);
     }
     const int items = prefix[n];
     out.items = items;
@@ -365,33 +405,50 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     // launch shape: register budget from the caller or the autotuner, keyed
     // by form, work items and shared memory per chain
     const int wpb = 4;
-    const size_t smem = size_t(max_wf) * wpb * sizeof(float);
-    VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the docking kernel");
-    p.warps_per_block = wpb;
+    const size_t smem_warps = size_t(max_wf) * wpb * sizeof(float);
+    VD_CHECK(smem_warps <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the docking kernel");
     out.tune_key = (uint64_t(persistent) << 40) | (uint64_t(ceil_log2(uint64_t(items))) << 32) |
                    uint64_t(max_wf > 1024);  // above 4 KB per chain, shared memory caps the occupancy
     out.tune_key |= uint64_t(sp.dense_bfgs != 0) << 41;
     out.tuned = sp.launch_shape == 0;
-    out.shape = dock_shape_for(c, sp, out.tune_key);
+    // Few chains: a team of warps per chain (see kTeamChains) in the place of
+    // the 128-register shape, whose aim is the same, for a caller or an
+    // autotuner that picks that shape; the plain form, whose chains are alike,
+    // takes it without exploring.
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-    const DockFn k = sp.dense_bfgs ? (persistent ? dense_dock_fn<true>(out.shape) : dense_dock_fn<false>(out.shape))
-                                   : (persistent ? dock_fn<true>(out.shape) : dock_fn<false>(out.shape));
+    const size_t smem_team = (size_t(max_wf) + pair_team_floats(max_sp)) * sizeof(float);
+    const bool few = items <= sms * kTeamChains && smem_team <= 227 * 1024 / kTeamChains;
+    if (out.tuned && few && !persistent) {
+        out.tuned = false;
+        out.shape = kWideShape;
+    } else {
+        out.shape = dock_shape_for(c, sp, out.tune_key);
+    }
+    const bool team = few && out.shape == kWideShape;
+    const bool dense = sp.dense_bfgs != 0;
+    DockFn k;
+    if (team) k = persistent ? team_dock_fn<true>(dense) : team_dock_fn<false>(dense);
+    else if (dense) k = persistent ? dense_dock_fn<true>(out.shape) : dense_dock_fn<false>(out.shape);
+    else k = persistent ? dock_fn<true>(out.shape) : dock_fn<false>(out.shape);
+    const size_t smem = team ? smem_team : smem_warps;
+    const int threads = team ? 32 * kTeamWarps : 32 * wpb;
+    p.warps_per_block = team ? 1 : wpb;
     VD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    VD_CUDA(prefer_l1(k, c.device, kShapeBlocks[out.shape], smem));
-    int blocks = (items + wpb - 1) / wpb;
+    VD_CUDA(prefer_l1(k, c.device, team ? kTeamChains : kShapeBlocks[out.shape], smem));
+    int blocks = (items + p.warps_per_block - 1) / p.warps_per_block;
     if (persistent) {
         int per_sm = 0;
-        VD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * wpb, smem));
+        VD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem));
         blocks = std::min(sms * std::max(1, per_sm), blocks);
     }
-    out.launch = [k, blocks, wpb, smem, p](cudaStream_t stream) {
-        k<<<blocks, 32 * wpb, smem, stream>>>(p);
+    out.launch = [k, blocks, threads, smem, p](cudaStream_t stream) {
+        k<<<blocks, threads, smem, stream>>>(p);
         return cudaGetLastError();
     };
     c.stats.dock_blocks = blocks;
     c.stats.dock_shape = out.shape + 1;
-    c.stats.dock_warps_per_block = wpb;
+    c.stats.dock_warps_per_block = p.warps_per_block;
     return VD_OK;
 }
 

@@ -429,6 +429,57 @@ __device__ __forceinline__ void adjoint_phases(const LigView& L, const WarpMem& 
     __syncwarp();
 }
 
+// One entry of the search schedule (two rounds, one pair each) for this lane:
+// returns the two pairs' energies; both atoms' forces go to their
+// accumulators with atomics.
+template <bool want_grad>
+__device__ __forceinline__ float pair_rounds(const LigView& L, const WarpMem& m, const float4* smooth, float v_intra,
+                                             float fix, int2 qq) {
+    int* const qx = reinterpret_cast<int*>(m.ns);
+    int* const qy = qx + pad4(L.na);
+    int* const qz = qy + pad4(L.na);
+    const bool v0 = qq.x >= 0, v1 = qq.y >= 0;  // unused slots are negative (atoms 0, 0)
+    const int a0 = VD_DCLAMP(qq.x & 0xff, 0, L.na - 1, kChkPairAtom);
+    const int b0 = VD_DCLAMP((qq.x >> 8) & 0xff, 0, L.na - 1, kChkPairAtom);
+    const int a1 = VD_DCLAMP(qq.y & 0xff, 0, L.na - 1, kChkPairAtom);
+    const int b1 = VD_DCLAMP((qq.y >> 8) & 0xff, 0, L.na - 1, kChkPairAtom);
+    const float4 ca0 = m.c[a0], cb0 = m.c[b0], ca1 = m.c[a1], cb1 = m.c[b1];
+    const float r0x = cb0.x - ca0.x, r0y = cb0.y - ca0.y, r0z = cb0.z - ca0.z;
+    const float r1x = cb1.x - ca1.x, r1y = cb1.y - ca1.y, r1z = cb1.z - ca1.z;
+    const float d0 = r0x * r0x + r0y * r0y + r0z * r0z, d1 = r1x * r1x + r1y * r1y + r1z * r1z;
+    const float rf0 = fminf(32.f * d0, 2047.5f), rf1 = fminf(32.f * d1, 2047.5f);
+    const int i0 = VD_DCLAMP(int(rf0), 0, kBins - 2, kChkTableBin);
+    const int i1 = VD_DCLAMP(int(rf1), 0, kBins - 2, kChkTableBin);
+    const int tp0 = VD_DCLAMP(v0 ? (qq.x >> 16) : 0, 0, kPairTypes - 1, kChkPairType);
+    const int tp1 = VD_DCLAMP(v1 ? (qq.y >> 16) : 0, 0, kPairTypes - 1, kChkPairType);
+    const bool in0 = v0 && d0 < 64.f, in1 = v1 && d1 < 64.f;
+    float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
+    if (in0) t0 = __ldg(smooth + size_t(tp0) * kBins + i0);  // no gather past the cutoff
+    if (in1) t1 = __ldg(smooth + size_t(tp1) * kBins + i1);
+    const float w0 = rf0 - float(i0), w1 = rf1 - float(i1);
+    float e0 = t0.x + w0 * (t0.z - t0.x), g0 = t0.y + w0 * (t0.w - t0.y);
+    float e1 = t1.x + w1 * (t1.z - t1.x), g1 = t1.y + w1 * (t1.w - t1.y);
+    const float c0 = (e0 > 0.f) ? __fdividef(v_intra, v_intra + e0) : 1.f;
+    const float c1 = (e1 > 0.f) ? __fdividef(v_intra, v_intra + e1) : 1.f;
+    e0 = in0 ? e0 * c0 : 0.f;
+    e1 = in1 ? e1 * c1 : 0.f;
+    if (want_grad) {
+        // fixed point: fix is a power of two, so (g * fix) * r rounds exactly like (g * r) * fix
+        const float gf0 = in0 ? g0 * c0 * c0 * fix : 0.f, gf1 = in1 ? g1 * c1 * c1 * fix : 0.f;
+        if (in0) {
+            const int Fx = __float2int_rn(gf0 * r0x), Fy = __float2int_rn(gf0 * r0y), Fz = __float2int_rn(gf0 * r0z);
+            atomicAdd(&qx[a0], -Fx); atomicAdd(&qy[a0], -Fy); atomicAdd(&qz[a0], -Fz);
+            atomicAdd(&qx[b0], Fx); atomicAdd(&qy[b0], Fy); atomicAdd(&qz[b0], Fz);
+        }
+        if (in1) {
+            const int Fx = __float2int_rn(gf1 * r1x), Fy = __float2int_rn(gf1 * r1y), Fz = __float2int_rn(gf1 * r1z);
+            atomicAdd(&qx[a1], -Fx); atomicAdd(&qy[a1], -Fy); atomicAdd(&qz[a1], -Fz);
+            atomicAdd(&qx[b1], Fx); atomicAdd(&qy[b1], Fy); atomicAdd(&qz[b1], Fz);
+        }
+    }
+    return e0 + e1;
+}
+
 // pair_atomics: pairs from the search schedule, both atoms' forces by
 // atomics (no per-lane flush when the second atom changes: shorter, less
 // divergent code, which the latency-bound search prefers); otherwise the
@@ -472,52 +523,10 @@ __device__ inline float eval_pose_t(const LigView& L, const WarpMem& m, const In
     //    contiguous segment, b's coordinates and force kept in registers
     //    while b repeats, the force on a added with an atomic.
     if (pair_atomics) {
-        int* const qx = reinterpret_cast<int*>(m.ns);
-        int* const qy = qx + pad4(L.na);
-        int* const qz = qy + pad4(L.na);
         const int2* sp = L.spairs + lane;
         for (int k = 0; k < L.sp_iters; ++k, sp += 32) {
             const int2 qq = __ldg(sp);  // coalesced across the warp
-            const bool v0 = qq.x >= 0, v1 = qq.y >= 0;  // unused slots are negative (atoms 0, 0)
-            const int a0 = VD_DCLAMP(qq.x & 0xff, 0, L.na - 1, kChkPairAtom);
-            const int b0 = VD_DCLAMP((qq.x >> 8) & 0xff, 0, L.na - 1, kChkPairAtom);
-            const int a1 = VD_DCLAMP(qq.y & 0xff, 0, L.na - 1, kChkPairAtom);
-            const int b1 = VD_DCLAMP((qq.y >> 8) & 0xff, 0, L.na - 1, kChkPairAtom);
-            const float4 ca0 = m.c[a0], cb0 = m.c[b0], ca1 = m.c[a1], cb1 = m.c[b1];
-            const float r0x = cb0.x - ca0.x, r0y = cb0.y - ca0.y, r0z = cb0.z - ca0.z;
-            const float r1x = cb1.x - ca1.x, r1y = cb1.y - ca1.y, r1z = cb1.z - ca1.z;
-            const float d0 = r0x * r0x + r0y * r0y + r0z * r0z, d1 = r1x * r1x + r1y * r1y + r1z * r1z;
-            const float rf0 = fminf(32.f * d0, 2047.5f), rf1 = fminf(32.f * d1, 2047.5f);
-            const int i0 = VD_DCLAMP(int(rf0), 0, kBins - 2, kChkTableBin);
-            const int i1 = VD_DCLAMP(int(rf1), 0, kBins - 2, kChkTableBin);
-            const int tp0 = VD_DCLAMP(v0 ? (qq.x >> 16) : 0, 0, kPairTypes - 1, kChkPairType);
-            const int tp1 = VD_DCLAMP(v1 ? (qq.y >> 16) : 0, 0, kPairTypes - 1, kChkPairType);
-            const bool in0 = v0 && d0 < 64.f, in1 = v1 && d1 < 64.f;
-            float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
-            if (in0) t0 = __ldg(smooth + size_t(tp0) * kBins + i0);  // no gather past the cutoff
-            if (in1) t1 = __ldg(smooth + size_t(tp1) * kBins + i1);
-            const float w0 = rf0 - float(i0), w1 = rf1 - float(i1);
-            float e0 = t0.x + w0 * (t0.z - t0.x), g0 = t0.y + w0 * (t0.w - t0.y);
-            float e1 = t1.x + w1 * (t1.z - t1.x), g1 = t1.y + w1 * (t1.w - t1.y);
-            const float c0 = (e0 > 0.f) ? __fdividef(v_intra, v_intra + e0) : 1.f;
-            const float c1 = (e1 > 0.f) ? __fdividef(v_intra, v_intra + e1) : 1.f;
-            e0 = in0 ? e0 * c0 : 0.f;
-            e1 = in1 ? e1 * c1 : 0.f;
-            e += e0 + e1;
-            if (want_grad) {
-                // fixed point: fix is a power of two, so (g * fix) * r rounds exactly like (g * r) * fix
-                const float gf0 = in0 ? g0 * c0 * c0 * fix : 0.f, gf1 = in1 ? g1 * c1 * c1 * fix : 0.f;
-                if (in0) {
-                    const int Fx = __float2int_rn(gf0 * r0x), Fy = __float2int_rn(gf0 * r0y), Fz = __float2int_rn(gf0 * r0z);
-                    atomicAdd(&qx[a0], -Fx); atomicAdd(&qy[a0], -Fy); atomicAdd(&qz[a0], -Fz);
-                    atomicAdd(&qx[b0], Fx); atomicAdd(&qy[b0], Fy); atomicAdd(&qz[b0], Fz);
-                }
-                if (in1) {
-                    const int Fx = __float2int_rn(gf1 * r1x), Fy = __float2int_rn(gf1 * r1y), Fz = __float2int_rn(gf1 * r1z);
-                    atomicAdd(&qx[a1], -Fx); atomicAdd(&qy[a1], -Fy); atomicAdd(&qz[a1], -Fz);
-                    atomicAdd(&qx[b1], Fx); atomicAdd(&qy[b1], Fy); atomicAdd(&qz[b1], Fz);
-                }
-            }
+            e += pair_rounds<want_grad>(L, m, smooth, v_intra, fix, qq);
         }
     } else {
         const int len = (((lane + 1) * L.np) >> 5) - ((lane * L.np) >> 5);
@@ -613,6 +622,100 @@ __device__ __forceinline__ float eval_pose(const LigView& L, const WarpMem& m, c
                                            const Skip& skip = Skip()) {
     const GridInter gi{&G, ep.v_inter, ep.slope};
     return eval_pose_t<want_grad, pair_atomics>(L, m, gi, smooth, ep.v_intra, ep.fix, ep.inv_fix, lane, skip);
+}
+
+// ---------------------------------------------------------------- teams
+// A team of `warps` warps evaluates one pose: the first places the atoms,
+// looks up the grid and runs everything else; the others compute the intra
+// pairs meanwhile.  The pair energies come back through shared memory and are
+// added in the order a single warp adds them, the forces are exact integer
+// sums, so a team's results equal a single warp's bit for bit.
+//
+// Barriers of a team (its block): 1, the atoms are placed, or there is nothing
+// left to do; 2, the pair terms are in shared memory.  The first warp arrives
+// at 1 and waits at 2, the others the other way round; every thread takes part
+// in each once per evaluation, and in 1 once more at the end.
+template <int warps>
+__device__ __forceinline__ void team_sync(int id) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(32 * warps) : "memory");
+}
+template <int warps>
+__device__ __forceinline__ void team_arrive(int id) {
+    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(32 * warps) : "memory");
+}
+
+struct PairTeam {
+    float* e;   // [sp_iters][32] pair energies of the schedule's entries
+    int* work;  // 0: leave; else 1 + the index of the ligand to evaluate
+};
+__host__ __device__ inline int pair_team_floats(int sp_iters) { return 32 * sp_iters + 4; }
+__device__ __forceinline__ PairTeam pair_team(float* p) {
+    return PairTeam{p + 4, reinterpret_cast<int*>(p)};
+}
+
+// Evaluation by the team's first warp (the search's form: gradient wanted).
+template <int warps, class Inter, class Skip>
+__device__ inline float eval_pose_team(const LigView& L, const WarpMem& m, const Inter& inter, float inv_fix, int lane,
+                                       const PairTeam& tm, const Skip& skip) {
+    frames(L, m, lane);
+    int* const q = reinterpret_cast<int*>(m.ns);
+    const int a4 = pad4(L.na);
+    for (int i = lane; i < L.na; i += 32) {
+        m.c[i] = atom_position(L, m, __ldg(&L.atoms[i]));
+        q[i] = 0; q[a4 + i] = 0; q[2 * a4 + i] = 0;
+    }
+    __syncwarp();
+    team_arrive<warps>(1);
+    float e = 0.f;
+    for (int i = lane; i < L.na; i += 32) {
+        const float4 ci = m.c[i];
+        float gx, gy, gz;
+        e += inter(__float_as_int(__ldg(&L.atoms[i].w)) & 0xff, ci.x, ci.y, ci.z, gx, gy, gz);
+        m.fx[i] = gx; m.fy[i] = gy; m.fz[i] = gz;
+    }
+    __syncwarp();
+    team_sync<warps>(2);
+    for (int k = 0; k < L.sp_iters; k += 4) {
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) v[j] = k + j < L.sp_iters ? tm.e[32 * (k + j) + lane] : 0.f;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) e += v[j];
+    }
+    e = warp_sum(e);
+    if (skip(e)) return e;
+    adjoint_phases(L, m, inv_fix, lane);
+    return e;
+}
+
+// The other warps (w = 1 .. warps - 1) of a team: view(work) gives the ligand
+// and its arrays in the team's shared memory; entries w - 1, w - 1 + (warps -
+// 1), .. of its pair schedule, the first one loaded ahead of the wait.
+template <int warps, class View>
+__device__ inline void pair_team_helper(const View& view, const float4* smooth, float v_intra, float fix, int w, int lane,
+                                        const PairTeam& tm) {
+    int cur = 0;
+    LigView L;
+    WarpMem m;
+    int2 first = make_int2(-65536, -65536);
+    for (;;) {
+        team_sync<warps>(1);
+        const int work = *reinterpret_cast<volatile int*>(tm.work);
+        if (work == 0) return;
+        if (work != cur) {
+            cur = work;
+            view(work - 1, L, m);
+            if (w - 1 < L.sp_iters) first = __ldg(L.spairs + 32 * (w - 1) + lane);
+        }
+        int2 qq = first;
+        for (int k = w - 1; k < L.sp_iters; k += warps - 1) {
+            const int2 now = qq;
+            if (k + warps - 1 < L.sp_iters) qq = __ldg(L.spairs + 32 * (k + warps - 1) + lane);
+            tm.e[32 * k + lane] = pair_rounds<true>(L, m, smooth, v_intra, fix, now);
+        }
+        __syncwarp();
+        team_arrive<warps>(2);
+    }
 }
 
 }  // namespace vd

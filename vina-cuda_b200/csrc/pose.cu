@@ -65,7 +65,10 @@ __global__ void __launch_bounds__(32 * kPoseWarps, pose_min_blocks(mode)) pose_k
                 dst[3 * i + 2] = s.m.c[i].z;
             }
         } else {
-            const float e = rilc_bfgs(L, s, p.G, p.smooth, p.ep, p.max_steps, lane, evals);
+            const auto eval = [&](const SkipAbove& skip) {
+                return eval_pose<true, true>(L, s.m, p.G, p.smooth, p.ep, lane, skip);
+            };
+            const float e = rilc_bfgs(L, s, eval, p.max_steps, lane, evals);
             if (lane == 0) p.e_out[pose] = e;
             for (int i = lane; i < nc; i += 32) p.poses_out[size_t(pose) * nc + i] = s.m.x[i];
         }

@@ -455,13 +455,6 @@ __device__ __forceinline__ bool m_out(float v, double b, double e) {
 // forces are added.  Warp 0 arrives at 1 and waits at 2, the others the other
 // way round; every thread takes part in each once per evaluation, and in 1
 // once more at the end.
-__device__ __forceinline__ void team_sync(int id) {
-    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(32 * kRefineWarps) : "memory");
-}
-__device__ __forceinline__ void team_arrive(int id) {
-    asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(32 * kRefineWarps) : "memory");
-}
-
 __global__ void __launch_bounds__(32 * kRefineWarps, 1) refine_kernel(RefineParams p) {
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, pose = blockIdx.x;
@@ -492,18 +485,18 @@ __global__ void __launch_bounds__(32 * kRefineWarps, 1) refine_kernel(RefinePara
         direct_terms(L, s.m, p.R, p.smooth, 1000.f, slope, tm, wid, lane);
         pair_terms(L, s.m, p.smooth, 1000.f, p.fix, tm, threadIdx.x);
         __syncwarp();
-        team_sync(3);
+        team_sync<kRefineWarps>(3);
     };
     if (wid == 0) find_runs(L, tm, lane);
     __syncthreads();
     if (wid > 0) {
         for (;;) {
-            team_sync(1);
+            team_sync<kRefineWarps>(1);
             if (*tm.cmd == 0) break;
             terms(*tm.slope);
             run_terms(L, s.m, p.fix, tm, threadIdx.x - 32, 32 * (kRefineWarps - 1));
             __syncwarp();
-            team_arrive(2);
+            team_arrive<kRefineWarps>(2);
         }
         return;
     }
@@ -529,11 +522,11 @@ __global__ void __launch_bounds__(32 * kRefineWarps, 1) refine_kernel(RefinePara
                 *tm.slope = slope;
             }
             __syncwarp();
-            team_arrive(1);
+            team_arrive<kRefineWarps>(1);
             terms(slope);
             const float sum = sum_energy(L, tm, lane);
             __syncwarp();
-            team_sync(2);
+            team_sync<kRefineWarps>(2);
             if (skip(sum)) return sum;
             adjoint_phases(L, s.m, p.inv_fix, lane);
             return sum;
@@ -557,7 +550,7 @@ __global__ void __launch_bounds__(32 * kRefineWarps, 1) refine_kernel(RefinePara
         *tm.cmd = 0;
     }
     __syncwarp();
-    team_arrive(1);
+    team_arrive<kRefineWarps>(1);
 }
 
 // ------------------------------------------------------------ score (double)

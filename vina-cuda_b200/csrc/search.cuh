@@ -150,8 +150,10 @@ struct SearchMem {  // per-warp shared memory of the optimiser
 // entry_only: evaluate the entry pose and return its energy without
 // optimising it (the visited-history policy's skipped calls,
 // quasi_newton.cuh:1937-1939).
-__device__ inline float rilc_bfgs(const LigView& L, const SearchMem& s, const MapView& G, const float4* smooth,
-                           const EvalParams ep, int max_steps, int lane, int& evals, bool entry_only = false) {
+// eval(skip): as in dense_bfgs below.
+template <class Eval>
+__device__ inline float rilc_bfgs(const LigView& L, const SearchMem& s, const Eval& eval, int max_steps, int lane,
+                                  int& evals, bool entry_only = false) {
     const int n = 6 + L.nt, nc = 7 + L.nt;
     if (max_steps <= 0) max_steps = 1000;  // the reference's 0 means unbounded
     float fx = 0.f, fx_orig = 0.f, fxp = 0.f, step = 0.f;
@@ -165,8 +167,7 @@ __device__ inline float rilc_bfgs(const LigView& L, const SearchMem& s, const Ma
         // a trial that fails the Armijo test before the tenth reads no
         // gradient: its adjoint is skipped
         const float armijo = finit + step * dgtest;  // one value for the skip and the test below
-        fx = eval_pose<true, true>(L, s.m, G, smooth, ep, lane,
-                                   SkipAbove{(!first && count + 1 < 10) ? armijo : INFINITY});
+        fx = eval(SkipAbove{(!first && count + 1 < 10) ? armijo : INFINITY});
         ++evals;
         g = vload(s.m.g, n, lane);
         if (first) {
