@@ -9,9 +9,15 @@
 // keeps the accepted pose and energy, kernel2.cu:526-552), so it is not run
 // here: same best poses and energies, fewer evaluations.  Random
 // numbers come from a Philox stream keyed by (seed, ligand, chain), so the
-// plain (one ligand per launch, one warp per chain) and the batched
-// (persistent, work queue over (ligand, chain) items) forms compute the same
-// chains.
+// plain (one ligand per launch) and the batched form (all ligands in one
+// launch) compute the same chains.
+//
+// The launch is persistent: as many blocks as are resident, each warp taking
+// the next (ligand, chain) item from a queue when its chain ends.  With a
+// block per four chains instead, a block's slots stayed empty until its
+// slowest chain ended: 6,500 chains of one ligand, 80 registers, B200, 24
+// atoms 5.37 -> 4.91 ms, 31 atoms 12.52 -> 11.92, 44 atoms 38.6 -> 37.6 (128
+// registers: 45.1 -> 36.4).
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -47,7 +53,6 @@ struct DockParams {
     unsigned long long* evals;
     unsigned long long* lig_evals;  // [n_ligs] evaluations per ligand
     int32_t warp_floats;
-    int32_t warps_per_block;
     int32_t visited;             // QuickVina2-CUDA's visited history (RILC-BFGS only)
 };
 
@@ -75,9 +80,9 @@ enum : int { kCsItem, kCsLig, kCsChain, kCsUid, kCsDepth, kCsSteps, kCsEvals0, k
 enum : int { kCfCurrent, kCfBest };
 static_assert(kCsFloats + kCfBest + 1 <= kChainWords, "chain scalars exceed their shared words");
 
-//
-// team > 1: a block is one chain, evaluated by a team of warps (eval.cuh).
-template <bool persistent, int MINB, bool dense = false, int team = 1>
+// team > 1: a block runs one chain at a time, evaluated by a team of warps
+// (eval.cuh).
+template <int MINB, bool dense = false, int team = 1>
 __global__ void __launch_bounds__(team > 1 ? 32 * team : 128, MINB) dock_kernel(DockParams p) {
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -92,13 +97,10 @@ __global__ void __launch_bounds__(team > 1 ? 32 * team : 128, MINB) dock_kernel(
         return;
     }
     int evals = 0;
-    int item = persistent ? 0 : team > 1 ? int(blockIdx.x) : blockIdx.x * p.warps_per_block + wid;
     for (;;) {
-        if (persistent) {
-            int v = 0;
-            if (lane == 0) v = atomicAdd(p.queue, 1);
-            item = __shfl_sync(0xffffffffu, v, 0);
-        }
+        int v = 0;
+        if (lane == 0) v = atomicAdd(p.queue, 1);
+        const int item = __shfl_sync(0xffffffffu, v, 0);
         if (item >= p.total_items) break;
         const int li0 = VD_DCLAMP(find_ligand(p.prefix, p.n_ligs, item), 0, p.n_ligs - 1, kChkItem);
         const LigView L = lig_view(p.pool, __ldg(&p.lig_off[li0]));
@@ -208,7 +210,6 @@ __global__ void __launch_bounds__(team > 1 ? 32 * team : 128, MINB) dock_kernel(
             atomicAdd(&p.lig_evals[li], (unsigned long long)(evals - cs[kCsEvals0]));
         }
         __syncwarp();
-        if (!persistent) break;
     }
     if (lane == 0 && evals) atomicAdd(p.evals, (unsigned long long)evals);
     if (team > 1) {
@@ -222,27 +223,24 @@ __global__ void __launch_bounds__(team > 1 ? 32 * team : 128, MINB) dock_kernel(
 constexpr int kShapeBlocks[] = {8, 10, 12, 6, 4};
 
 using DockFn = void (*)(DockParams);
-template <bool persistent>
 DockFn dock_fn(int shape) {
     switch (shape) {
-        case 1: return dock_kernel<persistent, 10>;
-        case 2: return dock_kernel<persistent, 12>;
-        case 3: return dock_kernel<persistent, 6>;
-        case 4: return dock_kernel<persistent, 4>;
-        default: return dock_kernel<persistent, 8>;
+        case 1: return dock_kernel<10>;
+        case 2: return dock_kernel<12>;
+        case 3: return dock_kernel<6>;
+        case 4: return dock_kernel<4>;
+        default: return dock_kernel<8>;
     }
 }
 // Dense-BFGS search: built at the three register budgets the autotuner
 // explores (64 / 80 / 128); a pinned 48- or 40-register shape runs at 64.
-template <bool persistent>
 DockFn dense_dock_fn(int& shape) {
     switch (shape) {
-        case 3: return dock_kernel<persistent, 6, true>;
-        case 4: return dock_kernel<persistent, 4, true>;
-        default: shape = 0; return dock_kernel<persistent, 8, true>;
+        case 3: return dock_kernel<6, true>;
+        case 4: return dock_kernel<4, true>;
+        default: shape = 0; return dock_kernel<8, true>;
     }
 }
-
 // Few chains leave most warp slots empty and a chain is one long dependency:
 // frames, atoms, grid lookup, pairs, adjoint, optimiser.  A team of four warps
 // per chain takes the pairs off it (three warps compute them while the first
@@ -257,10 +255,8 @@ DockFn dense_dock_fn(int& shape) {
 constexpr int kTeamWarps = 4;   // warps per chain
 constexpr int kTeamChains = 7;  // chains resident per SM
 constexpr int kWideShape = 4;   // the 128-register shape
-template <bool persistent>
 DockFn team_dock_fn(bool dense) {
-    return dense ? DockFn(dock_kernel<persistent, kTeamChains, true, kTeamWarps>)
-                 : DockFn(dock_kernel<persistent, kTeamChains, false, kTeamWarps>);
+    return dense ? DockFn(dock_kernel<kTeamChains, true, kTeamWarps>) : DockFn(dock_kernel<kTeamChains, false, kTeamWarps>);
 }
 
 // Shared-memory floats of the dense optimiser's state: H (n x n) and the
@@ -275,8 +271,11 @@ int dense_floats(int ntors) {
 // The autotuner's candidates: 64, 80 and 128 registers.  The 48- and
 // 40-register shapes spill heavily and were slower on every measured
 // workload (wide-box screen, single ligand, uneven batch); they stay
-// available to callers that pin a shape.
-constexpr int kTunedShapes[] = {0, 3, 4};
+// available to callers that pin a shape.  Tried in this order: a new
+// context's first call runs the shape that is best or next to it on most
+// workloads (6,500 chains of a 31-atom ligand: 80 registers 11.9 ms, 128
+// 12.3, 64 12.5; 64 screened ligands: 793, 918, 839).
+constexpr int kTunedShapes[] = {3, 4, 0};
 constexpr int kNumTuned = int(sizeof(kTunedShapes) / sizeof(kTunedShapes[0]));
 
 int dock_shape_for(Ctx& c, const vd_search_params& sp, uint64_t key) {
@@ -427,28 +426,22 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     }
     const bool team = few && out.shape == kWideShape;
     const bool dense = sp.dense_bfgs != 0;
-    DockFn k;
-    if (team) k = persistent ? team_dock_fn<true>(dense) : team_dock_fn<false>(dense);
-    else if (dense) k = persistent ? dense_dock_fn<true>(out.shape) : dense_dock_fn<false>(out.shape);
-    else k = persistent ? dock_fn<true>(out.shape) : dock_fn<false>(out.shape);
+    const DockFn k = team ? team_dock_fn(dense) : dense ? dense_dock_fn(out.shape) : dock_fn(out.shape);
     const size_t smem = team ? smem_team : smem_warps;
     const int threads = team ? 32 * kTeamWarps : 32 * wpb;
-    p.warps_per_block = team ? 1 : wpb;
     VD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     VD_CUDA(prefer_l1(k, c.device, team ? kTeamChains : kShapeBlocks[out.shape], smem));
-    int blocks = (items + p.warps_per_block - 1) / p.warps_per_block;
-    if (persistent) {
-        int per_sm = 0;
-        VD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem));
-        blocks = std::min(sms * std::max(1, per_sm), blocks);
-    }
+    const int chains = team ? 1 : wpb;  // per block
+    int per_sm = 0;
+    VD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem));
+    const int blocks = std::min(sms * std::max(1, per_sm), (items + chains - 1) / chains);
     out.launch = [k, blocks, threads, smem, p](cudaStream_t stream) {
         k<<<blocks, threads, smem, stream>>>(p);
         return cudaGetLastError();
     };
     c.stats.dock_blocks = blocks;
     c.stats.dock_shape = out.shape + 1;
-    c.stats.dock_warps_per_block = p.warps_per_block;
+    c.stats.dock_warps_per_block = chains;
     return VD_OK;
 }
 
@@ -625,7 +618,7 @@ extern "C" vd_status vd_mc_chains_noalloc(vd_ctx* h, int32_t lig, const vd_searc
     p.out_conf = d_conf;
     p.stride = nc;
     p.out_e = d_e;
-    p.queue = nullptr;  // one warp per chain: no work queue
+    p.queue = reinterpret_cast<int32_t*>(base + 128);
     p.visited = sp->visited_history;
     p.evals = d_cnt;
     p.lig_evals = d_cnt + 1;
@@ -633,10 +626,12 @@ extern "C" vd_status vd_mc_chains_noalloc(vd_ctx* h, int32_t lig, const vd_searc
     const int wpb = 4;
     const size_t smem = size_t(p.warp_floats) * wpb * sizeof(float);
     VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "vd_mc_chains_noalloc: ligand too large for the kernel");
-    p.warps_per_block = wpb;
-    auto k = sp->dense_bfgs ? dock_kernel<false, 8, true> : dock_kernel<false, 8>;
+    auto k = sp->dense_bfgs ? dock_kernel<8, true> : dock_kernel<8>;
     VD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    k<<<(n + wpb - 1) / wpb, 32 * wpb, smem, c.stream>>>(p);
+    int sms = 148, per_sm = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    VD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * wpb, smem));
+    k<<<std::min(sms * std::max(1, per_sm), (n + wpb - 1) / wpb), 32 * wpb, smem, c.stream>>>(p);
     VD_CUDA(cudaGetLastError());
     VD_CUDA(cudaMemcpyAsync(poses_out, d_conf, size_t(n) * nc * sizeof(float), cudaMemcpyDeviceToHost, c.stream));
     VD_CUDA(cudaMemcpyAsync(e_out, d_e, size_t(n) * sizeof(float), cudaMemcpyDeviceToHost, c.stream));
