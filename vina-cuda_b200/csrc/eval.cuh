@@ -121,6 +121,19 @@ __device__ __forceinline__ WarpMem carve(float* p, int na, int nn, int np, int n
 __device__ __forceinline__ int to_fixed(float v, float fix) { return __float2int_rn(v * fix); }
 __device__ __forceinline__ float from_fixed(int v, float inv_fix) { return float(v) * inv_fix; }
 
+// trunc(v) for 0 <= v < 2^23 on the FP32 pipe: adding 2^23 rounded toward zero
+// leaves it in the low mantissa bits.  The conversions to and from integers it
+// replaces issue at a sixteenth of the rate and stand in the middle of the
+// pair phase's longest dependency.
+struct Trunc {
+    float f;  // trunc(v)
+    int i;
+};
+__device__ __forceinline__ Trunc trunc_pos(float v) {
+    const float t = __fadd_rz(v, 8388608.f);
+    return Trunc{t - 8388608.f, __float_as_int(t) - 0x4B000000};
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -236,7 +249,8 @@ __device__ __forceinline__ Corners load_corners(const MapView& G, const float* m
                                                 int a2) {
     Corners k;
     if (cell) {
-        const float* c = cell + ((size_t(a2) * (G.n[1] - 1) + a1) * (G.n[0] - 1) + a0) * 8;
+        // a map has less than 2^31 cells: 32-bit index arithmetic
+        const float* c = cell + size_t(uint32_t((a2 * (G.n[1] - 1) + a1) * (G.n[0] - 1) + a0)) * 8;
         unsigned long long w0, w1, w2, w3;
         // not allocated in L1: the cells of a 70 A box span 1.67 GB and are
         // rarely re-read from L1, where they would evict the pair table
@@ -269,9 +283,9 @@ __device__ __forceinline__ float grid_term(const MapView& G, const float* map, c
         miss += (lo + hi) * G.finv[d];
         reg[d] = (s < 0.f) ? -1.f : ((s >= G.dmo[d]) ? 1.f : 0.f);
         const float sc = fminf(fmaxf(s, 0.f), G.dmo[d]);
-        const int ai = min(int(sc), G.n[d] - 2);
-        a[d] = ai;
-        fr[d] = (s >= G.dmo[d]) ? 1.f : sc - float(ai);
+        const Trunc ai = trunc_pos(sc);  // at most n - 2 below the far face
+        a[d] = min(ai.i, G.n[d] - 2);
+        fr[d] = (s >= G.dmo[d]) ? 1.f : sc - ai.f;
     }
     const float penalty = slope * miss;
     const Corners k = load_corners(G, map, cell, a[0], a[1], a[2]);
@@ -429,6 +443,13 @@ __device__ __forceinline__ void adjoint_phases(const LigView& L, const WarpMem& 
     __syncwarp();
 }
 
+// Row of the pair table: the whole table is 5 MB, so the byte offset takes
+// 32-bit arithmetic.
+__device__ __forceinline__ const float4* table_row(const float4* smooth, int type_pair, int bin) {
+    const uint32_t off = uint32_t(type_pair) * uint32_t(kBins * sizeof(float4)) + uint32_t(bin) * uint32_t(sizeof(float4));
+    return reinterpret_cast<const float4*>(reinterpret_cast<const char*>(smooth) + off);
+}
+
 // One entry of the search schedule (two rounds, one pair each) for this lane:
 // returns the two pairs' energies; both atoms' forces go to their
 // accumulators with atomics.
@@ -448,15 +469,16 @@ __device__ __forceinline__ float pair_rounds(const LigView& L, const WarpMem& m,
     const float r1x = cb1.x - ca1.x, r1y = cb1.y - ca1.y, r1z = cb1.z - ca1.z;
     const float d0 = r0x * r0x + r0y * r0y + r0z * r0z, d1 = r1x * r1x + r1y * r1y + r1z * r1z;
     const float rf0 = fminf(32.f * d0, 2047.5f), rf1 = fminf(32.f * d1, 2047.5f);
-    const int i0 = VD_DCLAMP(int(rf0), 0, kBins - 2, kChkTableBin);
-    const int i1 = VD_DCLAMP(int(rf1), 0, kBins - 2, kChkTableBin);
+    const Trunc bin0 = trunc_pos(rf0), bin1 = trunc_pos(rf1);
+    const int i0 = VD_DCLAMP(bin0.i, 0, kBins - 2, kChkTableBin);
+    const int i1 = VD_DCLAMP(bin1.i, 0, kBins - 2, kChkTableBin);
     const int tp0 = VD_DCLAMP(v0 ? (qq.x >> 16) : 0, 0, kPairTypes - 1, kChkPairType);
     const int tp1 = VD_DCLAMP(v1 ? (qq.y >> 16) : 0, 0, kPairTypes - 1, kChkPairType);
     const bool in0 = v0 && d0 < 64.f, in1 = v1 && d1 < 64.f;
     float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
-    if (in0) t0 = __ldg(smooth + size_t(tp0) * kBins + i0);  // no gather past the cutoff
-    if (in1) t1 = __ldg(smooth + size_t(tp1) * kBins + i1);
-    const float w0 = rf0 - float(i0), w1 = rf1 - float(i1);
+    if (in0) t0 = __ldg(table_row(smooth, tp0, i0));  // no gather past the cutoff
+    if (in1) t1 = __ldg(table_row(smooth, tp1, i1));
+    const float w0 = rf0 - bin0.f, w1 = rf1 - bin1.f;
     float e0 = t0.x + w0 * (t0.z - t0.x), g0 = t0.y + w0 * (t0.w - t0.y);
     float e1 = t1.x + w1 * (t1.z - t1.x), g1 = t1.y + w1 * (t1.w - t1.y);
     const float c0 = (e0 > 0.f) ? __fdividef(v_intra, v_intra + e0) : 1.f;
@@ -564,15 +586,16 @@ __device__ inline float eval_pose_t(const LigView& L, const WarpMem& m, const In
             const float r1x = cb1.x - ca1.x, r1y = cb1.y - ca1.y, r1z = cb1.z - ca1.z;
             const float d0 = r0x * r0x + r0y * r0y + r0z * r0z, d1 = r1x * r1x + r1y * r1y + r1z * r1z;
             const float rf0 = fminf(32.f * d0, 2047.5f), rf1 = fminf(32.f * d1, 2047.5f);
-            const int i0 = VD_DCLAMP(int(rf0), 0, kBins - 2, kChkTableBin);
-            const int i1 = VD_DCLAMP(int(rf1), 0, kBins - 2, kChkTableBin);
+            const Trunc bin0 = trunc_pos(rf0), bin1 = trunc_pos(rf1);
+            const int i0 = VD_DCLAMP(bin0.i, 0, kBins - 2, kChkTableBin);
+            const int i1 = VD_DCLAMP(bin1.i, 0, kBins - 2, kChkTableBin);
             const int tp0 = VD_DCLAMP(q0.y, 0, kPairTypes - 1, kChkPairType);
             const int tp1 = VD_DCLAMP(q1.y, 0, kPairTypes - 1, kChkPairType);
             const bool in0 = d0 < 64.f, in1 = two && d1 < 64.f;
             float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
-            if (in0) t0 = __ldg(smooth + size_t(tp0) * kBins + i0);  // no gather past the cutoff
-            if (in1) t1 = __ldg(smooth + size_t(tp1) * kBins + i1);
-            const float w0 = rf0 - float(i0), w1 = rf1 - float(i1);
+            if (in0) t0 = __ldg(table_row(smooth, tp0, i0));  // no gather past the cutoff
+            if (in1) t1 = __ldg(table_row(smooth, tp1, i1));
+            const float w0 = rf0 - bin0.f, w1 = rf1 - bin1.f;
             float e0 = t0.x + w0 * (t0.z - t0.x), g0 = t0.y + w0 * (t0.w - t0.y);
             float e1 = t1.x + w1 * (t1.z - t1.x), g1 = t1.y + w1 * (t1.w - t1.y);
             const float c0 = (e0 > 0.f) ? __fdividef(v_intra, v_intra + e0) : 1.f;
