@@ -5,7 +5,8 @@ are integer sums, so nothing may differ.  Ligands: no intra pairs, fewer
 schedule entries than helper warps, more than one round of them, atoms past
 one and two per lane, the largest accepted; both searches; the plain form,
 the batched form over ligands of different sizes, and a call with no
-Monte-Carlo step.
+Monte-Carlo step.  Local optimisation picks its kernel by the number of poses:
+a pose's result may not depend on how many others there are.
 """
 import numpy as np
 import pytest
@@ -55,3 +56,16 @@ def test_team_batches_equal_single_warp_batches(env, dense, depth, visited):
     for a, b in zip(*out):
         assert a["bfgs_evals"] == b["bfgs_evals"]
         assert np.array_equal(a["energy"], b["energy"]) and np.array_equal(a["pose"], b["pose"])
+
+
+@pytest.mark.parametrize("i", [0, 2, 4, 6])
+def test_local_optimisation_does_not_depend_on_the_number_of_poses(env, i):
+    import torch
+    from vdock import synth
+    vd, ctx, ids = env
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    poses = synth.random_poses(16 * sms + 1, ctx.ntors[ids[i]], -3.0, 3.0, seed=i)
+    ref_e, ref_p, _ = ctx.local_opt(ids[i], poses, 6)
+    for n in (1, 7 * sms, 7 * sms + 1, 16 * sms):
+        e, p, _ = ctx.local_opt(ids[i], poses[:n], 6)
+        assert np.array_equal(e, ref_e[:n]) and np.array_equal(p, ref_p[:n]), n

@@ -301,9 +301,10 @@ __device__ __forceinline__ float grid_term(const MapView& G, const float* map, c
     const float t = (f > 0.f) ? __fdividef(v, v + f) : 1.f;  // curl (curl.h:31-40)
     f *= t;
     const float t2 = t * t;
-    gx = (reg[0] == 0.f) ? G.factor[0] * xg * t2 : slope * reg[0];
-    gy = (reg[1] == 0.f) ? G.factor[1] * yg * t2 : slope * reg[1];
-    gz = (reg[2] == 0.f) ? G.factor[2] * zg * t2 : slope * reg[2];
+    // (rounded products, whatever the caller adds to them)
+    gx = (reg[0] == 0.f) ? __fmul_rn(G.factor[0] * xg, t2) : slope * reg[0];
+    gy = (reg[1] == 0.f) ? __fmul_rn(G.factor[1] * yg, t2) : slope * reg[1];
+    gz = (reg[2] == 0.f) ? __fmul_rn(G.factor[2] * zg, t2) : slope * reg[2];
     return f + penalty;
 }
 
@@ -336,6 +337,23 @@ struct SkipAbove {
     float thr;
     __device__ __forceinline__ bool operator()(float e) const { return e > thr; }
 };
+
+// dE/dtorsion of body k from the force and the moment about the root origin of
+// its subtree (v); w1: its torsion axis in its own frame.
+__device__ __forceinline__ float torsion_gradient(const WarpMem& m, int k, float4 w1, float ox, float oy, float oz,
+                                                  const float (&v)[6]) {
+    const float4* nd = reinterpret_cast<const float4*>(m.nd + kNodeF * k);
+    const float4 r0 = nd[0], r1 = nd[1], r2 = nd[2];
+    const float dx = r0.w - ox, dy = r1.w - oy, dz = r2.w - oz;
+    const float T0 = v[3] - (dy * v[2] - dz * v[1]);
+    const float T1 = v[4] - (dz * v[0] - dx * v[2]);
+    const float T2 = v[5] - (dx * v[1] - dy * v[0]);
+    const float u0 = w1.x, u1 = w1.y, u2 = w1.z;
+    const float a0 = r0.x * u0 + r0.y * u1 + r0.z * u2;
+    const float a1 = r1.x * u0 + r1.y * u1 + r1.z * u2;
+    const float a2 = r2.x * u0 + r2.y * u1 + r2.z * u2;
+    return T0 * a0 + T1 * a1 + T2 * a2;
+}
 
 // Phases 6-7: the pose gradient into m.g from the atoms' grid-term forces
 // (m.fx/fy/fz), their fixed-point pair forces (m.ns) and coordinates (m.c).
@@ -427,18 +445,59 @@ __device__ __forceinline__ void adjoint_phases(const LigView& L, const WarpMem& 
         if (k == 0) {
             m.g[0] = F0; m.g[1] = F1; m.g[2] = F2; m.g[3] = M0; m.g[4] = M1; m.g[5] = M2;
         } else {
-            const float4* nd = reinterpret_cast<const float4*>(m.nd + kNodeF * k);
-            const float4 r0 = nd[0], r1 = nd[1], r2 = nd[2];
-            const float dx = r0.w - ox, dy = r1.w - oy, dz = r2.w - oz;
-            const float T0 = M0 - (dy * F2 - dz * F1);
-            const float T1 = M1 - (dz * F0 - dx * F2);
-            const float T2 = M2 - (dx * F1 - dy * F0);
-            const float u0 = w1.x, u1 = w1.y, u2 = w1.z;
-            const float a0 = r0.x * u0 + r0.y * u1 + r0.z * u2;
-            const float a1 = r1.x * u0 + r1.y * u1 + r1.z * u2;
-            const float a2 = r2.x * u0 + r2.y * u1 + r2.z * u2;
-            m.g[6 + k - 1] = T0 * a0 + T1 * a1 + T2 * a2;
+            const float v[6] = {F0, F1, F2, M0, M1, M2};
+            m.g[6 + k - 1] = torsion_gradient(m, k, w1, ox, oy, oz, v);
         }
+    }
+    __syncwarp();
+}
+
+// adjoint_phases for at most 32 heavy atoms and bodies: lane l brings atom l's
+// position and grid-term force and takes body l; the prefixes stay in
+// registers and are fetched by shuffles.  Same sums in the same order.  For
+// kernels with few warps per SM, where the chain's latency counts (a team's
+// 24-atom evaluation is 5 % shorter); in the search with full SMs the second
+// copy of this phase costs more in instruction fetches (2 % of a screen).
+__device__ __forceinline__ void adjoint_small(const LigView& L, const WarpMem& m, float inv_fix, int lane, float4 c,
+                                              float fx, float fy, float fz) {
+    const unsigned full = 0xffffffffu;
+    const bool body = lane < L.nn;
+    const float4 w1 = node_word(L.nodes, body ? lane : 0, 1);  // {axis, first atom}
+    const int e1 = VD_DCLAMP(__float_as_int(node_word(L.nodes, body ? lane : 0, 2).w), 0, L.na, kChkSubtree);
+    const int b = VD_DCLAMP(__float_as_int(w1.w), 0, e1, kChkSubtree);
+    const float4 xo4 = *reinterpret_cast<const float4*>(m.x);
+    const float ox = xo4.x, oy = xo4.y, oz = xo4.z;
+    float run[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    if (lane < L.na) {
+        const int a4 = pad4(L.na);
+        const int* q = reinterpret_cast<const int*>(m.ns);
+        const float gx = fx + from_fixed(q[lane], inv_fix), gy = fy + from_fixed(q[a4 + lane], inv_fix),
+                    gz = fz + from_fixed(q[2 * a4 + lane], inv_fix);
+        const float dx = c.x - ox, dy = c.y - oy, dz = c.z - oz;
+        run[0] = gx; run[1] = gy; run[2] = gz;
+        run[3] = dy * gz - dz * gy;
+        run[4] = dz * gx - dx * gz;
+        run[5] = dx * gy - dy * gx;
+    }
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+#pragma unroll
+        for (int j = 0; j < 6; ++j) {
+            const float o = __shfl_up_sync(full, run[j], off);
+            if (lane >= off) run[j] += o;
+        }
+    }
+    const int hi = max(e1 - 1, 0), lo = max(b - 1, 0);
+    float v[6];
+#pragma unroll
+    for (int j = 0; j < 6; ++j) {
+        const float h = __shfl_sync(full, run[j], hi), l = __shfl_sync(full, run[j], lo);
+        v[j] = e1 > b ? (b > 0 ? h - l : h) : 0.f;
+    }
+    if (lane == 0) {
+        m.g[0] = v[0]; m.g[1] = v[1]; m.g[2] = v[2]; m.g[3] = v[3]; m.g[4] = v[4]; m.g[5] = v[5];
+    } else if (body) {
+        m.g[6 + lane - 1] = torsion_gradient(m, lane, w1, ox, oy, oz, v);
     }
     __syncwarp();
 }
@@ -689,12 +748,13 @@ __device__ inline float eval_pose_team(const LigView& L, const WarpMem& m, const
     }
     __syncwarp();
     team_arrive<warps>(1);
-    float e = 0.f;
+    float e = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
+    float4 ci = make_float4(0.f, 0.f, 0.f, 0.f);
+    const bool small = L.na <= 32 && L.nn <= 32;
     for (int i = lane; i < L.na; i += 32) {
-        const float4 ci = m.c[i];
-        float gx, gy, gz;
+        ci = m.c[i];
         e += inter(__float_as_int(__ldg(&L.atoms[i].w)) & 0xff, ci.x, ci.y, ci.z, gx, gy, gz);
-        m.fx[i] = gx; m.fy[i] = gy; m.fz[i] = gz;
+        if (!small) { m.fx[i] = gx; m.fy[i] = gy; m.fz[i] = gz; }
     }
     __syncwarp();
     team_sync<warps>(2);
@@ -707,7 +767,8 @@ __device__ inline float eval_pose_team(const LigView& L, const WarpMem& m, const
     }
     e = warp_sum(e);
     if (skip(e)) return e;
-    adjoint_phases(L, m, inv_fix, lane);
+    if (small) adjoint_small(L, m, inv_fix, lane, ci, gx, gy, gz);
+    else adjoint_phases(L, m, inv_fix, lane);
     return e;
 }
 

@@ -24,57 +24,127 @@ struct PoseParams {
     float* xyz_out;     // coords only
     float* poses_out;   // local opt
     int32_t max_steps;
+    int32_t* queue;     // local opt: next pose
     unsigned long long* evals;
     int32_t warp_floats;
 };
 
-// mode 0: energy, 1: energy+gradient, 2: coordinates, 3: local optimisation.
-// Modes 0-2 are held to 64 registers (8 blocks of 4 warps per SM):
-// they fit without spills, and the adjoint (mode 1) left free takes 72 and
-// loses a block per SM.
-constexpr int pose_min_blocks(int mode) { return mode == 3 ? 1 : 8; }
+// mode 0: energy, 1: energy+gradient, 2: coordinates.  Held to 64 registers
+// (8 blocks of 4 warps per SM): they fit without spills, and the adjoint
+// (mode 1) left free takes 72 and loses a block per SM.
+constexpr int kPoseBlocks = 8;
 template <int mode>
-__global__ void __launch_bounds__(32 * kPoseWarps, pose_min_blocks(mode)) pose_kernel(PoseParams p) {
+__global__ void __launch_bounds__(32 * kPoseWarps, kPoseBlocks) pose_kernel(PoseParams p) {
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float* base = reinterpret_cast<float*>(smem4) + size_t(wid) * p.warp_floats;
     const LigView L = lig_view(p.pool, p.lig_off);
-    SearchMem s;
-    s.m = carve(base, L.na, L.nn, L.np, L.nt);
-    s.xp = base + warp_floats(L.na, L.nn, L.np, L.nt);
-    s.xo = s.xp + pad4(7 + L.nt);
+    const WarpMem m = carve(base, L.na, L.nn, L.np, L.nt);
     const int nc = 7 + L.nt, n = 6 + L.nt;
-    int evals = 0;
     for (int pose = blockIdx.x * kPoseWarps + wid; pose < p.n_poses; pose += gridDim.x * kPoseWarps) {
         const float* src = p.poses + size_t(pose) * nc;
-        for (int i = lane; i < nc; i += 32) s.m.x[i] = src[i];
+        for (int i = lane; i < nc; i += 32) m.x[i] = src[i];
         __syncwarp();
         if (mode == 0) {
-            const float e = eval_pose<false>(L, s.m, p.G, p.smooth, p.ep, lane);
+            const float e = eval_pose<false>(L, m, p.G, p.smooth, p.ep, lane);
             if (lane == 0) p.e_out[pose] = e;
         } else if (mode == 1) {
-            const float e = eval_pose<true>(L, s.m, p.G, p.smooth, p.ep, lane);
+            const float e = eval_pose<true>(L, m, p.G, p.smooth, p.ep, lane);
             if (lane == 0) p.e_out[pose] = e;
-            for (int i = lane; i < n; i += 32) p.g_out[size_t(pose) * n + i] = s.m.g[i];
-        } else if (mode == 2) {
-            kinematics(L, s.m, lane);
+            for (int i = lane; i < n; i += 32) p.g_out[size_t(pose) * n + i] = m.g[i];
+        } else {
+            kinematics(L, m, lane);
             float* dst = p.xyz_out + size_t(pose) * 3 * L.na;
             for (int i = lane; i < L.na; i += 32) {
-                dst[3 * i] = s.m.c[i].x;
-                dst[3 * i + 1] = s.m.c[i].y;
-                dst[3 * i + 2] = s.m.c[i].z;
+                dst[3 * i] = m.c[i].x;
+                dst[3 * i + 1] = m.c[i].y;
+                dst[3 * i + 2] = m.c[i].z;
             }
-        } else {
-            const auto eval = [&](const SkipAbove& skip) {
-                return eval_pose<true, true>(L, s.m, p.G, p.smooth, p.ep, lane, skip);
-            };
-            const float e = rilc_bfgs(L, s, eval, p.max_steps, lane, evals);
-            if (lane == 0) p.e_out[pose] = e;
-            for (int i = lane; i < nc; i += 32) p.poses_out[size_t(pose) * nc + i] = s.m.x[i];
         }
         __syncwarp();
     }
-    if (mode == 3 && lane == 0 && evals) atomicAdd(p.evals, (unsigned long long)evals);
+}
+
+// Local optimisation, one RILC-BFGS run per pose; poses come from a queue
+// (their numbers of evaluations differ several times over).  team > 1: a
+// block takes one pose at a time, evaluated by a team of warps.
+template <int blocks, int team>
+__global__ void __launch_bounds__(32 * (team > 1 ? team : kPoseWarps), blocks) local_opt_kernel(PoseParams p) {
+    extern __shared__ float4 smem4[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float* base = reinterpret_cast<float*>(smem4) + (team > 1 ? size_t(0) : size_t(wid) * p.warp_floats);
+    const LigView L = lig_view(p.pool, p.lig_off);
+    SearchMem s;
+    s.m = carve(base, L.na, L.nn, L.np, L.nt);
+    const PairTeam tm = pair_team(base + p.warp_floats);
+    if (team > 1 && wid > 0) {
+        const auto view = [&](int, LigView& l, WarpMem& m) {
+            l = L;
+            m = s.m;
+        };
+        pair_team_helper<team>(view, p.smooth, p.ep.v_intra, p.ep.fix, wid, lane, tm);
+        return;
+    }
+    s.xp = base + warp_floats(L.na, L.nn, L.np, L.nt);
+    s.xo = s.xp + pad4(7 + L.nt);
+    const int nc = 7 + L.nt;
+    if (team > 1 && lane == 0) *tm.work = 1;
+    int evals = 0;
+    const auto eval = [&](const SkipAbove& skip) {
+        const GridInter gi{&p.G, p.ep.v_inter, p.ep.slope};
+        if constexpr (team > 1)
+            return eval_pose_team<team>(L, s.m, gi, p.ep.inv_fix, lane, tm, skip);
+        else
+            return eval_pose_t<true, true>(L, s.m, gi, p.smooth, p.ep.v_intra, p.ep.fix, p.ep.inv_fix, lane, skip);
+    };
+    for (;;) {
+        int v = 0;
+        if (lane == 0) v = atomicAdd(p.queue, 1);
+        const int pose = __shfl_sync(0xffffffffu, v, 0);
+        if (pose >= p.n_poses) break;
+        const float* src = p.poses + size_t(pose) * nc;
+        for (int i = lane; i < nc; i += 32) s.m.x[i] = src[i];
+        __syncwarp();
+        const float e = rilc_bfgs(L, s, eval, p.max_steps, lane, evals);
+        if (lane == 0) p.e_out[pose] = e;
+        for (int i = lane; i < nc; i += 32) p.poses_out[size_t(pose) * nc + i] = s.m.x[i];
+        __syncwarp();
+    }
+    if (lane == 0 && evals) atomicAdd(p.evals, (unsigned long long)evals);
+    if (team > 1) {
+        if (lane == 0) *tm.work = 0;
+        __syncwarp();
+        team_arrive<team>(1);
+    }
+}
+
+// Launch of local_opt_kernel by the number of poses: a team of four warps per
+// pose while all poses are resident that way (7 blocks per SM, as in the
+// docking kernel), else one warp per pose, at 128 registers (4 blocks) while
+// all poses are resident, else at 80 (6 blocks).  31-atom ligand, at most 20
+// steps, us a call on B200, before (one warp a pose at 140 registers, 3 blocks
+// per SM, no queue) -> now: 50 poses 287 -> 215, 1,000 426 -> 340, 1,300 449 ->
+// 431 (80 registers: 454), 2,000 593 -> 510 (531), 2,800 644 -> 480, 8,000 1,515
+// -> 1,150; 44 atoms, 1,000 poses 669 -> 415.
+vd_status launch_local_opt(Ctx& c, const HostLigand& L, const PoseParams& p, cudaStream_t stream) {
+    constexpr int kTeam = 4, kTeamPoses = 7, kWide = 4, kNarrow = 6;
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    const size_t smem_team = (size_t(p.warp_floats) + pair_team_floats(L.h.sp_iters)) * sizeof(float);
+    const bool team = p.n_poses <= sms * kTeamPoses && smem_team <= 227 * 1024 / kTeamPoses;
+    const bool wide = p.n_poses <= sms * kWide * kPoseWarps;
+    const size_t smem = team ? smem_team : size_t(p.warp_floats) * kPoseWarps * sizeof(float);
+    VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the pose kernel");
+    auto k = team ? local_opt_kernel<kTeamPoses, kTeam> : wide ? local_opt_kernel<kWide, 1> : local_opt_kernel<kNarrow, 1>;
+    const int threads = 32 * (team ? kTeam : kPoseWarps), poses = team ? 1 : kPoseWarps;  // per block
+    VD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    VD_CUDA(prefer_l1(k, c.device, team ? kTeamPoses : wide ? kWide : kNarrow, smem));
+    int per_sm = 0;
+    VD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem));
+    const int blocks = std::min(sms * std::max(1, per_sm), (p.n_poses + poses - 1) / poses);
+    k<<<blocks, threads, smem, stream>>>(p);
+    VD_CUDA(cudaGetLastError());
+    return VD_OK;
 }
 
 template <int mode>
@@ -108,18 +178,23 @@ vd_status run_pose_kernel(Ctx& c, int lig, int n_poses, const float* d_poses, co
     p.poses_out = d_out;
     p.max_steps = max_steps;
     p.evals = reinterpret_cast<unsigned long long*>(c.d_counter + 8);
-    p.warp_floats = lig_warp_floats(L) + 2 * pad4(7 + L.h.ntors);
-    const size_t smem = size_t(p.warp_floats) * kPoseWarps * sizeof(float);
-    VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the pose kernel");
-    auto kern = pose_kernel<mode>;
-    VD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    if (mode != 3) VD_CUDA(prefer_l1(kern, c.device, pose_min_blocks(mode), smem));
-    int dev_sms = 148;
-    cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c.device);
-    const int blocks = std::min((n_poses + kPoseWarps - 1) / kPoseWarps, dev_sms * 16);
-    kern<<<blocks, 32 * kPoseWarps, smem, stream>>>(p);
-    VD_CUDA(cudaGetLastError());
-    return VD_OK;
+    p.queue = c.d_counter + 10;
+    p.warp_floats = lig_warp_floats(L) + (mode == 3 ? 2 * pad4(7 + L.h.ntors) : 0);
+    if constexpr (mode == 3) {
+        return launch_local_opt(c, L, p, stream);
+    } else {
+        const size_t smem = size_t(p.warp_floats) * kPoseWarps * sizeof(float);
+        VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the pose kernel");
+        auto kern = pose_kernel<mode>;
+        VD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        VD_CUDA(prefer_l1(kern, c.device, kPoseBlocks, smem));
+        int dev_sms = 148;
+        cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c.device);
+        const int blocks = std::min((n_poses + kPoseWarps - 1) / kPoseWarps, dev_sms * 16);
+        kern<<<blocks, 32 * kPoseWarps, smem, stream>>>(p);
+        VD_CUDA(cudaGetLastError());
+        return VD_OK;
+    }
 }
 
 }  // namespace
@@ -168,7 +243,7 @@ static vd_status pose_host(vd_ctx* h, int32_t lig, int32_t n, const float* poses
     float* d_g = reinterpret_cast<float*>(s + 2 * b_pose + b_e);
     float* d_x = reinterpret_cast<float*>(s + 2 * b_pose + b_e + b_g);
     VD_CUDA(cudaMemcpyAsync(d_pose, poses, n * nc * 4, cudaMemcpyHostToDevice, c.stream));
-    if (mode == 3) VD_CUDA(cudaMemsetAsync(c.d_counter + 8, 0, 8, c.stream));
+    if (mode == 3) VD_CUDA(cudaMemsetAsync(c.d_counter + 8, 0, 12, c.stream));  // evaluations, queue
     switch (mode) {
         case 0: st = run_pose_kernel<0>(c, lig, n, d_pose, ep, d_e, nullptr, nullptr, nullptr, 0, c.stream); break;
         case 1: st = run_pose_kernel<1>(c, lig, n, d_pose, ep, d_e, d_g, nullptr, nullptr, 0, c.stream); break;
