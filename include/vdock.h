@@ -179,8 +179,8 @@ vd_status vd_grid_dims(vd_ctx* ctx, int32_t npts[3], double begin[3], double end
 /* ---- grid maps: replaces kernel_grid (kernel1.cu:202-249) ----------------- */
 /* Builds one FP32 map per listed XS type over the box; maps stay on device. */
 vd_status vd_build_grids(vd_ctx* ctx, const int32_t* xs_types, int32_t n_types);
-/* Grid tile of later builds: 0 = autotuned (the first build of each box size
- * times both tiles), 1 = 16x8x8 points per 256 threads, 2 = 16x8x4 per 128.
+/* Grid tile of later builds: 1 = 16x8x8 points per 256 threads, 2 = 16x8x4 per
+ * 128, 0 = the default (16x8x4).
  * The maps are bit-identical for every tile. */
 vd_status vd_set_grid_shape(vd_ctx* ctx, int32_t shape);
 /* Copies one map to the host, x fastest: out[x + nx*(y + ny*z)]. */

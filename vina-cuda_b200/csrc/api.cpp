@@ -37,6 +37,11 @@ vd_status dev_alloc(Ctx& c, void** p, size_t bytes, const char* what) {
     return VD_OK;
 }
 
+bool dev_keeps(const Ctx& c, const void* p, size_t bytes) {
+    const auto it = c.dev_bytes.find(const_cast<void*>(p));
+    return p && it != c.dev_bytes.end() && it->second == bytes && (c.dev_cap == 0 || c.dev_used <= c.dev_cap);
+}
+
 void dev_free(Ctx& c, void* p) {
     if (!p) return;
     auto it = c.dev_bytes.find(p);

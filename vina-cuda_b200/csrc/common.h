@@ -175,6 +175,8 @@ struct Ctx {
     // executable CUDA graph it is recorded into (updated in place per call)
     void* h_stage = nullptr;
     size_t h_stage_bytes = 0;
+    std::vector<char> h_slab;             // vd_get_grid: rows on their way out (about 1 MB at most)
+    int slab_reads = 0;                   // maps read through it
     cudaGraphExec_t pipe_exec = nullptr;
     vd_stats stats{};
     // device memory owned by the context (dev_alloc / dev_free): bytes in use
@@ -182,8 +184,8 @@ struct Ctx {
     // past it into VD_ERR_NOMEM
     std::unordered_map<void*, size_t> dev_bytes;
     size_t dev_used = 0, dev_cap = 0;
-    // launch-shape autotuners (tune.h); grid_shape_fixed > 0 pins the grid tile
-    Tuner dock_tune, grid_tune;
+    // launch-shape autotuner (tune.h); grid_shape_fixed > 0 pins the grid tile
+    Tuner dock_tune;
     int grid_shape_fixed = 0;
 };
 
@@ -226,6 +228,9 @@ vd_status dev_alloc(Ctx& c, T** p, size_t bytes, const char* what) {
     *p = static_cast<T*>(q);
     return st;
 }
+// Whether an allocation of dev_alloc serves a new need of `bytes` as it is:
+// the same size, and the context within its cap.
+bool dev_keeps(const Ctx& c, const void* p, size_t bytes);
 // Frees a dev_alloc allocation (null is fine) and sets the pointer to null.
 void dev_free(Ctx& c, void* p);
 template <class T>

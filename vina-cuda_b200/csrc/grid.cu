@@ -8,8 +8,8 @@
 // evaluated in double with explicitly rounded operations (no FMA
 // contraction); the table values are FP32 and the sums are FP32.
 //
-// Launch: one CTA per tile of 16(x) x 8(y) x TZ(z) points (TZ = 8 or 4,
-// autotuned), 32*TZ threads, each thread owning 4 consecutive x points so
+// Launch: one CTA per tile of 16(x) x 8(y) x TZ(z) points (TZ = 4, or 8 when
+// pinned), 32*TZ threads, each thread owning 4 consecutive x points so
 // every map store is one 128-bit store; one launch per group of up to 8 maps.  The CTA stages, in shared
 // memory, the receptor atoms whose brick distance to the tile is below the
 // cutoff, taken from per-type 4 A cell lists in deterministic (receptor type,
@@ -28,7 +28,7 @@
 namespace vd {
 namespace {
 
-constexpr int kTileX = 16, kTileY = 8;  // z tile (TZ = 8 or 4) is a launch shape; threads = 32 * TZ
+constexpr int kTileX = 16, kTileY = 8;  // z tile TZ: 4, or 8 when pinned; threads = 32 * TZ
 constexpr int kStageCap = 128;    // atoms staged per chunk (4 KB; a 70 A tile keeps ~60, larger counts loop)
 constexpr double kCellSize = 4.0;
 constexpr int kLutRows = kBins + 1;  // table rows per receptor type; the last (zero) row is padding
@@ -259,29 +259,67 @@ __global__ void __launch_bounds__(32 * TZ, 16 / TZ) grid_build_kernel(GridParams
     }
 }
 
+// Table slices of a build, per group of up to 8 maps [receptor types present]
+// [kLutRows][w] (w = 8, or 4 for a last group of at most 4 maps), gathered from
+// the FP32 pair table on the device (4 us; building them on the host and
+// copying them took ~0.3 ms).  One thread per row.
+struct LutParams {
+    const float* fast;      // [153][kBins]
+    float* lut;
+    int32_t n_present, n_maps;
+    int32_t present[kTypes], needed[kTypes];
+};
+__global__ void __launch_bounds__(256) lut_kernel(LutParams p) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x, ti = r / kLutRows, i = r - ti * kLutRows;
+    if (ti >= p.n_present) return;
+    const int g0 = 8 * blockIdx.y, w = p.n_maps - g0 <= 4 ? 4 : 8;  // groups before this one are 8 wide
+    float* row = p.lut + size_t(g0) * p.n_present * kLutRows + size_t(r) * w;
+    const int t1 = p.present[ti];
+    for (int j = 0; j < w; ++j) {
+        float v = 0.f;
+        if (i < kBins && g0 + j < p.n_maps) {
+            const int t2 = p.needed[g0 + j], a = min(t1, t2), b = max(t1, t2);
+            v = __ldg(&p.fast[size_t(a + b * (b + 1) / 2) * kBins + i]);
+        }
+        row[j] = v;
+    }
+}
+
 // Corner cells for the evaluation kernels: cell (x, y, z) of map j holds the
 // map values at its 8 corners (x fastest, then y, then z), 32 bytes, so a
-// trilinear lookup reads one sector instead of eight scattered floats.  One
-// thread per cell; consecutive threads write consecutive cells.
+// trilinear lookup reads one sector instead of eight scattered floats.
+// Bound by the cells' write: one thread per column of kCellZ cells, which
+// loads each of its planes once, with 32-bit indices and one 256-bit store per
+// cell (consecutive threads write consecutive cells).  With a 64-bit division
+// per cell and two 128-bit stores the 188^3 x 8 maps of a 70 A box took
+// 505 us (3.7 TB/s); now 294 us (6.4 TB/s, 98 % of a plain copy's rate).
+constexpr int kCellZ = 4;
 __global__ void __launch_bounds__(256) corner_cells_kernel(const float* maps, size_t map_stride, float* cells,
-                                                           size_t cell_stride, int n_maps, int nx, int ny, int nz,
-                                                           int pitch) {
-    const int cx = nx - 1, cy = ny - 1, cz = nz - 1;
-    const size_t per_map = size_t(cx) * cy * cz;
-    const size_t total = per_map * size_t(n_maps);
-    for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < total; i += size_t(gridDim.x) * blockDim.x) {
-        const int j = int(i / per_map);
-        const size_t r = i - size_t(j) * per_map;
-        const int x = int(r % size_t(cx));
-        const size_t yz = r / size_t(cx);
-        const int y = int(yz % size_t(cy)), z = int(yz / size_t(cy));
-        const float* b = maps + size_t(j) * map_stride + (size_t(z) * ny + y) * pitch + x;
-        const size_t row = size_t(pitch), plane = row * size_t(ny);
-        const float4 lo = make_float4(b[0], b[1], b[row], b[row + 1]);
-        const float4 hi = make_float4(b[plane], b[plane + 1], b[plane + row], b[plane + row + 1]);
-        float4* d = reinterpret_cast<float4*>(cells + size_t(j) * cell_stride + r * 8);
-        d[0] = lo;
-        d[1] = hi;
+                                                           size_t cell_stride, int nx, int ny, int nz, int pitch) {
+    const uint32_t cx = nx - 1, cy = ny - 1, cz = nz - 1, plane = cx * cy;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= plane) return;
+    const uint32_t y = i / cx, x = i - y * cx;
+    const size_t map_plane = size_t(ny) * pitch;
+    auto load = [&](const float* q) { return make_float4(__ldg(q), __ldg(q + 1), __ldg(q + pitch), __ldg(q + pitch + 1)); };
+    auto pack = [](float lo, float hi) {
+        return (static_cast<unsigned long long>(__float_as_uint(hi)) << 32) | __float_as_uint(lo);
+    };
+    for (uint32_t z0 = blockIdx.y * kCellZ; z0 < cz; z0 += gridDim.y * kCellZ) {
+        const float* b = maps + size_t(blockIdx.z) * map_stride + (size_t(z0) * ny + y) * pitch + x;
+        float* d = cells + size_t(blockIdx.z) * cell_stride + (size_t(z0) * plane + i) * 8;
+        float4 v[kCellZ + 1];
+#pragma unroll
+        for (int k = 0; k <= kCellZ; ++k)
+            if (z0 + k <= cz) v[k] = load(b + k * map_plane);
+#pragma unroll
+        for (int k = 0; k < kCellZ; ++k) {
+            if (z0 + k >= cz) break;
+            asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(d + size_t(k) * plane * 8),
+                         "l"(pack(v[k].x, v[k].y)), "l"(pack(v[k].z, v[k].w)), "l"(pack(v[k + 1].x, v[k + 1].y)),
+                         "l"(pack(v[k + 1].z, v[k + 1].w))
+                         : "memory");
+        }
     }
 }
 
@@ -337,74 +375,71 @@ vd_status vd_build_grids(vd_ctx* h, const int32_t* types, int32_t n_types) {
         cell_of.push_back(ci[0] + cd[0] * (ci[1] + cd[1] * ci[2]));
     }
     // per receptor type present: cell list over the same cells, atoms sorted
-    // by (type, cell) so a tile stages them type by type
+    // by (type, cell) so a tile stages them type by type: one counting sort
     const int n_cells = cd[0] * cd[1] * cd[2];
+    bool has[kTypes] = {};
+    for (const auto& a : rel) has[a.type] = true;
     std::vector<int> present;
+    int row_of[kTypes] = {};  // table rows of the present types
     for (int tr = 0; tr < kTypes; ++tr)
-        for (const auto& a : rel)
-            if (a.type == tr) { present.push_back(tr); break; }
+        if (has[tr]) {
+            row_of[tr] = int(present.size());
+            present.push_back(tr);
+        }
     if (present.empty()) present.push_back(0);
     std::vector<int32_t> start(present.size() * size_t(n_cells + 1), 0);
     std::vector<StagedAtom> sorted(rel.size());
     {
-        size_t base_atom = 0;
-        for (size_t ti = 0; ti < present.size(); ++ti) {
-            int32_t* st = &start[ti * size_t(n_cells + 1)];
-            for (size_t i = 0; i < rel.size(); ++i)
-                if (rel[i].type == present[ti]) st[cell_of[i] + 1]++;
-            st[0] = int32_t(base_atom);
-            for (int i = 0; i < n_cells; ++i) st[i + 1] += st[i];
-            std::vector<int32_t> fill(st, st + n_cells);
-            for (size_t i = 0; i < rel.size(); ++i)
-                if (rel[i].type == present[ti]) sorted[fill[cell_of[i]]++] = rel[i];
-            base_atom = size_t(st[n_cells]);
+        // counts one place on, so that the running sums are each cell's start
+        for (size_t i = 0; i < rel.size(); ++i) {
+            rel[i].type = row_of[rel[i].type];
+            ++start[size_t(rel[i].type) * (n_cells + 1) + cell_of[i] + 1];
         }
+        int32_t run = 0;
+        for (int32_t& s : start) s = run += s;
+        std::vector<int32_t> fill(start);
+        for (size_t i = 0; i < rel.size(); ++i)
+            sorted[fill[size_t(rel[i].type) * (n_cells + 1) + cell_of[i]]++] = rel[i];
     }
-    // remap staged atom types to table rows of the present types
-    std::vector<int> row_of(kTypes, 0);
-    for (size_t ti = 0; ti < present.size(); ++ti) row_of[present[ti]] = int(ti);
-    for (auto& a : sorted) a.type = row_of[a.type];
-    // Table slices per group of up to 8 maps: [receptor types present][kLutRows][w]
-    // with w = 8, or 4 for a last group of at most 4 maps.
-    std::vector<int> grp_w, grp_off;
-    size_t lut_floats = 0;
-    for (int g0 = 0; g0 < nt; g0 += 8) {
-        grp_w.push_back(nt - g0 <= 4 ? 4 : 8);
-        grp_off.push_back(int(lut_floats));
-        lut_floats += present.size() * kLutRows * size_t(grp_w.back());
-    }
-    std::vector<float> lut(lut_floats, 0.f);
-    for (size_t gi = 0; gi < grp_w.size(); ++gi) {
-        const int w = grp_w[gi];
-        for (size_t ti = 0; ti < present.size(); ++ti)
-            for (int j = 0; j < w && 8 * int(gi) + j < nt; ++j) {
-                const size_t b = size_t(tri_index(present[ti], needed[8 * gi + j])) * kN;
-                for (int i = 0; i < kBins; ++i)
-                    lut[grp_off[gi] + (ti * kLutRows + i) * w + j] = float(c.fast[b + i]);
-            }
-    }
+    const size_t lut_floats = present.size() * kLutRows * size_t(nt % 8 == 0 ? nt : nt / 8 * 8 + (nt % 8 <= 4 ? 4 : 8));
 
     const size_t map_stride = size_t(g.pitch) * g.n[1] * g.n[2];
     const size_t bytes_maps = map_stride * nt * sizeof(float);
-    const size_t bytes_atoms = std::max<size_t>(1, sorted.size()) * sizeof(StagedAtom);
-    const size_t bytes_start = start.size() * sizeof(int32_t);
-    const size_t bytes_lut = lut.size() * sizeof(float);
-    dev_release(c, c.d_maps);
-    dev_release(c, c.d_cells);
+    const size_t n_cells_map = size_t(g.n[0] - 1) * (g.n[1] - 1) * (g.n[2] - 1);
+    const size_t bytes_cells = n_cells_map * 8 * sizeof(float) * nt;
+    const bool with_cells = bytes_cells <= kMaxCellBytes;
+    const size_t bytes_atoms = (std::max<size_t>(1, sorted.size()) * sizeof(StagedAtom) + 255) & ~size_t(255);
+    const size_t bytes_start = (start.size() * sizeof(int32_t) + 255) & ~size_t(255);
+    const size_t bytes_lut = lut_floats * sizeof(float);
     c.n_maps = 0;
     for (int i = 0; i < kTypes; ++i) c.map_slot[i] = -1;
-    vd_status st0 = dev_alloc(c, &c.d_maps, bytes_maps, "vd_build_grids: maps");
-    if (st0 != VD_OK) return st0;
-    vd_status st = ensure_scratch(&c, bytes_atoms + bytes_start + bytes_lut + 256);
+    // Maps and cells of the same size as the last build's stay allocated
+    // (allocating and freeing 1.9 GB took ~3 of the 4.4 ms of a 70 A build); others are
+    // all given back first.
+    if (!dev_keeps(c, c.d_maps, bytes_maps)) dev_release(c, c.d_maps);
+    if (!with_cells || !dev_keeps(c, c.d_cells, bytes_cells)) dev_release(c, c.d_cells);
+    vd_status st = VD_OK;
+    if (!c.d_maps && (st = dev_alloc(c, &c.d_maps, bytes_maps, "vd_build_grids: maps")) != VD_OK) return st;
+    st = ensure_scratch(&c, bytes_atoms + bytes_start + bytes_lut);
     if (st != VD_OK) return st;
+    // atoms and cell starts in one upload
     char* s = static_cast<char*>(c.d_scratch);
     StagedAtom* d_atoms = reinterpret_cast<StagedAtom*>(s);
-    int32_t* d_start = reinterpret_cast<int32_t*>(s + ((bytes_atoms + 255) & ~size_t(255)));
-    float* d_lut = reinterpret_cast<float*>(reinterpret_cast<char*>(d_start) + ((bytes_start + 255) & ~size_t(255)));
-    if (!sorted.empty())
-        VD_CUDA(cudaMemcpyAsync(d_atoms, sorted.data(), sorted.size() * sizeof(StagedAtom), cudaMemcpyHostToDevice, c.stream));
-    VD_CUDA(cudaMemcpyAsync(d_start, start.data(), bytes_start, cudaMemcpyHostToDevice, c.stream));
-    VD_CUDA(cudaMemcpyAsync(d_lut, lut.data(), bytes_lut, cudaMemcpyHostToDevice, c.stream));
+    int32_t* d_start = reinterpret_cast<int32_t*>(s + bytes_atoms);
+    float* d_lut = reinterpret_cast<float*>(s + bytes_atoms + bytes_start);
+    std::vector<char> up(bytes_atoms + bytes_start);
+    std::memcpy(up.data(), sorted.data(), sorted.size() * sizeof(StagedAtom));
+    std::memcpy(up.data() + bytes_atoms, start.data(), start.size() * sizeof(int32_t));
+    VD_CUDA(cudaMemcpyAsync(s, up.data(), up.size(), cudaMemcpyHostToDevice, c.stream));
+    LutParams lp{};
+    lp.fast = c.d_fast;
+    lp.lut = d_lut;
+    lp.n_present = int(present.size());
+    lp.n_maps = nt;
+    std::copy(present.begin(), present.end(), lp.present);
+    std::copy(needed.begin(), needed.end(), lp.needed);
+    lut_kernel<<<dim3((lp.n_present * kLutRows + 255) / 256, (nt + 7) / 8), 256, 0, c.stream>>>(lp);
+    VD_CUDA(cudaGetLastError());
 
     GridParams p{};
     for (int d = 0; d < 3; ++d) {
@@ -423,77 +458,56 @@ vd_status vd_build_grids(vd_ctx* h, const int32_t* types, int32_t n_types) {
     for (int d = 1; d < 3; ++d)  // cell rows a tile can touch in y and z: floor(span / cell) + 2 <= 6
         VD_CHECK(int(std::floor(((kTileY - 1) * g.finv[d] + 16.0) / kCellSize)) + 2 <= 6, VD_ERR_CAPACITY,
                  "vd_build_grids: grid spacing too large for the tile");
-    // Launch shapes (z tile 8 or 4) give bit-identical maps: a point sums its
-    // atoms in global (type, cell, index) order whatever the tile.  The first
-    // build of a box size times both and keeps the faster.
-    const uint64_t key = (uint64_t(ceil_log2(uint64_t(g.n[0]) * g.n[1] * g.n[2])) << 8) | uint64_t((nt + 7) / 8);
-    std::vector<int> shapes;
-    if (c.grid_shape_fixed > 0) shapes.push_back(c.grid_shape_fixed - 1);
-    else if (c.grid_tune.best(key) >= 0) shapes.push_back(c.grid_tune.best(key));
-    else shapes = {0, 1};
+    // z tile: 4, unless the caller pinned 8 (bit-identical maps: a point sums its
+    // atoms in global (type, cell, index) order whatever the tile).  us at 4
+    // and 8 for boxes of 20 / 30 / 40 / 45 / 70 A: 22.6 / 26.6, 60 / 64, 106 /
+    // 104, 152 / 154, 565 / 563; timing both on a box's first build cost more
+    // than it could find.
+    const int shape = c.grid_shape_fixed > 0 ? c.grid_shape_fixed - 1 : 1;
+    const int tz = shape == 0 ? 8 : 4;
     // shared-memory carve-out for the blocks each tile keeps resident (2 of
     // 256 threads or 4 of 128), the rest of the SM's data memory as L1
-    auto carve = [&](auto kern, int blocks) -> cudaError_t {
+    using GridFn = void (*)(GridParams);
+    const GridFn wide = tz == 8 ? grid_build_kernel<8, 8> : grid_build_kernel<8, 4>;
+    const GridFn narrow = tz == 8 ? grid_build_kernel<4, 8> : grid_build_kernel<4, 4>;
+    auto carve = [&](GridFn kern) -> cudaError_t {
         cudaFuncAttributes fa{};
         const cudaError_t r = cudaFuncGetAttributes(&fa, kern);
-        return r != cudaSuccess ? r : prefer_l1(kern, c.device, blocks, fa.sharedSizeBytes);
+        return r != cudaSuccess ? r : prefer_l1(kern, c.device, 16 / tz, fa.sharedSizeBytes);
     };
-    VD_CUDA(carve(grid_build_kernel<4, 8>, 2));
-    VD_CUDA(carve(grid_build_kernel<8, 8>, 2));
-    VD_CUDA(carve(grid_build_kernel<4, 4>, 4));
-    VD_CUDA(carve(grid_build_kernel<8, 4>, 4));
-    float best_ms = -1;
-    for (int shape : shapes) {
-        const int tz = shape == 0 ? 8 : 4;
-        dim3 grid((g.n[0] + kTileX - 1) / kTileX, (g.n[1] + kTileY - 1) / kTileY, (g.n[2] + tz - 1) / tz);
-        VD_CUDA(cudaEventRecord(c.ev0, c.stream));
-        for (int g0 = 0; g0 < nt; g0 += 8) {
-            p.maps = c.d_maps + size_t(g0) * map_stride;
-            p.lut = d_lut + grp_off[g0 / 8];
-            p.n_out = std::min(8, nt - g0);
-            const bool narrow = nt - g0 <= 4;
-            if (shape == 0) {
-                if (narrow) grid_build_kernel<4, 8><<<grid, 256, 0, c.stream>>>(p);
-                else grid_build_kernel<8, 8><<<grid, 256, 0, c.stream>>>(p);
-            } else {
-                if (narrow) grid_build_kernel<4, 4><<<grid, 128, 0, c.stream>>>(p);
-                else grid_build_kernel<8, 4><<<grid, 128, 0, c.stream>>>(p);
-            }
-            VD_CUDA(cudaGetLastError());
-        }
-        VD_CUDA(cudaEventRecord(c.ev1, c.stream));
-        VD_CUDA(cudaEventSynchronize(c.ev1));
-        if ((st = take_device_checks("grid kernel")) != VD_OK) return st;
-        float ms = 0;
-        VD_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
-        c.grid_tune.pick(key, 2);
-        c.grid_tune.report(key, shape, ms);
-        if (best_ms < 0 || ms < best_ms) best_ms = ms;
-        c.stats.grid_shape = shape + 1;
-    }
-    c.stats.grid_ms = best_ms;
-    // corner cells of the new maps (timed separately: cells_ms)
-    const size_t n_cells_map = size_t(g.n[0] - 1) * (g.n[1] - 1) * (g.n[2] - 1);
-    const size_t bytes_cells = n_cells_map * 8 * sizeof(float) * nt;
-    c.stats.cells_ms = 0;
-    if (bytes_cells <= kMaxCellBytes) {
-        st = dev_alloc(c, &c.d_cells, bytes_cells, "vd_build_grids: corner cells");
-        if (st != VD_OK) return st;
-        c.cell_stride = n_cells_map * 8;
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
-        const size_t total = n_cells_map * nt;
-        const int blocks = int(std::min<size_t>((total + 255) / 256, size_t(sms) * 8));
-        VD_CUDA(cudaEventRecord(c.ev0, c.stream));
-        corner_cells_kernel<<<blocks, 256, 0, c.stream>>>(c.d_maps, map_stride, c.d_cells, c.cell_stride, nt, g.n[0],
-                                                            g.n[1], g.n[2], g.pitch);
+    if (nt > 4) VD_CUDA(carve(wide));
+    if (nt % 8 >= 1 && nt % 8 <= 4) VD_CUDA(carve(narrow));
+    const dim3 grid((g.n[0] + kTileX - 1) / kTileX, (g.n[1] + kTileY - 1) / kTileY, (g.n[2] + tz - 1) / tz);
+    VD_CUDA(cudaEventRecord(c.ev0, c.stream));
+    for (int g0 = 0; g0 < nt; g0 += 8) {
+        p.maps = c.d_maps + size_t(g0) * map_stride;
+        p.lut = d_lut + size_t(g0) * present.size() * kLutRows;
+        p.n_out = std::min(8, nt - g0);
+        (nt - g0 <= 4 ? narrow : wide)<<<grid, 32 * tz, 0, c.stream>>>(p);
         VD_CUDA(cudaGetLastError());
-        VD_CUDA(cudaEventRecord(c.ev1, c.stream));
-        VD_CUDA(cudaEventSynchronize(c.ev1));
-        float ms = 0;
-        VD_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
-        c.stats.cells_ms = ms;
     }
+    VD_CUDA(cudaEventRecord(c.ev1, c.stream));
+    // corner cells of the new maps (cells_ms)
+    if (with_cells) {
+        if (!c.d_cells && (st = dev_alloc(c, &c.d_cells, bytes_cells, "vd_build_grids: corner cells")) != VD_OK) {
+            VD_CUDA(cudaStreamSynchronize(c.stream));
+            return st;
+        }
+        c.cell_stride = n_cells_map * 8;
+        const dim3 cells((size_t(g.n[0] - 1) * (g.n[1] - 1) + 255) / 256, std::min((g.n[2] - 1 + kCellZ - 1) / kCellZ, 65535), nt);
+        corner_cells_kernel<<<cells, 256, 0, c.stream>>>(c.d_maps, map_stride, c.d_cells, c.cell_stride, g.n[0], g.n[1],
+                                                         g.n[2], g.pitch);
+        VD_CUDA(cudaGetLastError());
+    }
+    VD_CUDA(cudaEventRecord(c.ev2, c.stream));
+    VD_CUDA(cudaEventSynchronize(c.ev2));
+    if ((st = take_device_checks("grid kernel")) != VD_OK) return st;
+    float grid_ms = 0, cells_ms = 0;
+    VD_CUDA(cudaEventElapsedTime(&grid_ms, c.ev0, c.ev1));
+    VD_CUDA(cudaEventElapsedTime(&cells_ms, c.ev1, c.ev2));
+    c.stats.grid_shape = shape + 1;
+    c.stats.grid_ms = grid_ms;
+    c.stats.cells_ms = with_cells ? cells_ms : 0;
     c.map_stride = map_stride;
     c.n_maps = nt;
     for (int i = 0; i < kTypes; ++i) c.map_slot[i] = -1;
@@ -514,10 +528,29 @@ vd_status vd_get_grid(vd_ctx* h, int32_t t, float* out) {
     VD_CUDA(cudaSetDevice(c.device));
     const GridGeom& g = c.geom;
     const float* src = c.d_maps + size_t(c.map_slot[t]) * c.map_stride;
-    VD_CUDA(cudaMemcpy2DAsync(out, size_t(g.n[0]) * sizeof(float), src, size_t(g.pitch) * sizeof(float),
-                              size_t(g.n[0]) * sizeof(float), size_t(g.n[1]) * g.n[2], cudaMemcpyDeviceToHost,
-                              c.stream));
-    VD_CUDA(cudaStreamSynchronize(c.stream));
+    // Slabs of padded rows come in one piece each into host memory that stays
+    // with the context, and the rows are copied out from there: 220 us a call
+    // for a 61 x 50 x 71 map, 120 us through pinned memory; a row-wise 2D copy
+    // took ~800 us, one piece straight into memory that the caller has not
+    // touched yet 240 us.  Pinned memory takes 4 ms to allocate, what it saves
+    // on 40 such calls: a context allocates it once it has made that many.
+    constexpr size_t kSlab = size_t(1) << 20;
+    constexpr int kPinAfter = 40;
+    const size_t row = size_t(g.n[0]) * sizeof(float), pitch = size_t(g.pitch) * sizeof(float);
+    const size_t rows = size_t(g.n[1]) * g.n[2], per = std::max<size_t>(1, std::min(rows, kSlab / pitch));
+    char* slab = nullptr;
+    if (c.h_stage_bytes >= per * pitch || (++c.slab_reads > kPinAfter && ensure_host_stage(&c, per * pitch) == VD_OK)) {
+        slab = static_cast<char*>(c.h_stage);
+    } else {
+        if (c.h_slab.size() < per * pitch) c.h_slab.resize(per * pitch);
+        slab = c.h_slab.data();
+    }
+    for (size_t r0 = 0; r0 < rows; r0 += per) {
+        const size_t n = std::min(per, rows - r0);
+        VD_CUDA(cudaMemcpyAsync(slab, src + r0 * g.pitch, n * pitch, cudaMemcpyDeviceToHost, c.stream));
+        VD_CUDA(cudaStreamSynchronize(c.stream));
+        for (size_t r = 0; r < n; ++r) std::memcpy(out + (r0 + r) * g.n[0], slab + r * pitch, row);
+    }
     return VD_OK;
 }
 

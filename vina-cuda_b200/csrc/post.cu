@@ -1231,12 +1231,20 @@ vd_status dock_pipeline(Ctx& c, const std::vector<int>& ligs, const vd_search_pa
     PostPlan pp;
     st = prepare_post(c, ligs, sp, db, pp);
     if (st != VD_OK) return st;
-    // pinned stage: [dock params | post params | results | counters]
+    // stage: [dock params | post params | results | counters]; pinned for the
+    // recorded form, which needs it, plain host memory for the direct one (a
+    // few KB; allocating pinned memory took 4 ms of a context's first call)
     const size_t b_dp = al256(db.h_params.size()), b_pp = al256(pp.h_params.size());
     const size_t b_res = al256(n * sizeof(vd_dock_result)), b_cnt = al256((2 + n) * sizeof(unsigned long long));
-    st = ensure_host_stage(&c, b_dp + b_pp + b_res + b_cnt);
-    if (st != VD_OK) return st;
-    unsigned char* hs = static_cast<unsigned char*>(c.h_stage);
+    std::vector<unsigned char> local;
+    if (persistent) {
+        st = ensure_host_stage(&c, b_dp + b_pp + b_res + b_cnt);
+        if (st != VD_OK) return st;
+    } else {
+        local.resize(b_dp + b_pp + b_res + b_cnt + 256);
+    }
+    unsigned char* hs = persistent ? static_cast<unsigned char*>(c.h_stage)
+                                   : local.data() + (-reinterpret_cast<uintptr_t>(local.data()) & 255);
     std::memcpy(hs, db.h_params.data(), db.h_params.size());
     std::memcpy(hs + b_dp, pp.h_params.data(), pp.h_params.size());
     vd_dock_result* h_res = reinterpret_cast<vd_dock_result*>(hs + b_dp + b_pp);
