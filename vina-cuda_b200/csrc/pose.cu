@@ -65,6 +65,343 @@ __global__ void __launch_bounds__(32 * kPoseWarps, kPoseBlocks) pose_kernel(Pose
     }
 }
 
+// ---------------------------------------------------------------- pose tiles
+// A block evaluates a tile of PL poses: a lane is one pose (lane mod PL) in one
+// of S slots (warps x 32 / PL), and bodies, atoms and pairs are dealt to the
+// slots.  Arrays in shared memory are [row][PL], rows being components of
+// bodies or atoms.  With a warp per pose (pose_kernel) a pair's atoms lie at
+// random places of shared memory and the lanes past a ligand's bodies and
+// atoms idle: 1,198 L1 wavefronts and 3,241 warp instructions per evaluation
+// of 40 atoms / 595 pairs at 65,536 poses, 90 % of the L1 data pipe.  With
+// lanes as poses the loads are conflict-free and the pair list is uniform:
+// 605 and 2,218; what is left is the table gathers, about one wavefront per
+// lane, and L1 hit rate decides (33 % at 4 tiles per SM), so large ligands
+// take 16 warps per tile and two tiles per SM.
+template <int PL>
+struct Tile {
+    int p, slot, slots;
+    __device__ __forceinline__ Tile() {
+        const int lane = threadIdx.x & 31;
+        p = lane % PL;
+        slot = (threadIdx.x >> 5) * (32 / PL) + lane / PL;
+        slots = (blockDim.x >> 5) * (32 / PL);
+    }
+};
+// Rows of a tile: coordinates [3][na]; pair forces [3][na] after the poses'
+// components [7 + nt] and the bodies' local rotations [nn][4]; per body its
+// axis and origin [6], then its part of the gradient; a partial energy per warp.
+__host__ __device__ inline int tile_rows(int mode, int na, int nn, int nt, int warps) {
+    const int early = 7 + nt + 4 * nn;
+    const int forces = mode == 1 && 3 * na > early ? 3 * na : early;
+    return 3 * na + forces + (mode == 1 ? 6 * nn : 0) + (mode == 2 ? 0 : warps);
+}
+// Before them: the pairs as 32-bit words, an even number.
+__host__ __device__ inline int tile_words(int mode, int np) { return mode == 2 ? 0 : pad4(np); }
+
+// Kinematics of the tile kernel.  Its coordinates equal frames() and
+// atom_position() bit for bit: the trilinear gradient jumps at cell faces and
+// the penalty's at the box, so a coordinate an ulp off would now and then give
+// another gradient than the other kernels do.  Where a sum of two products
+// leaves the compiler the choice of which one to fuse, the choice it makes
+// there is spelled out here (dot2: the first one).
+__device__ __forceinline__ float dot2(float a, float b, float c, float d) {  // a b + c d
+    return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+// a_j P of the walk up the ancestors
+__device__ __forceinline__ float4 walk_qmul(float4 a, float4 b) {
+    return make_float4(__fmaf_rn(-a.w, b.w, __fmaf_rn(-a.z, b.z, dot2(a.x, b.x, -a.y, b.y))),
+                       __fmaf_rn(-a.w, b.z, __fmaf_rn(a.z, b.w, dot2(a.x, b.y, a.y, b.x))),
+                       __fmaf_rn(a.w, b.y, __fmaf_rn(a.z, b.x, dot2(a.x, b.z, -a.y, b.w))),
+                       __fmaf_rn(a.w, b.x, __fmaf_rn(-a.z, b.y, dot2(a.x, b.w, a.y, b.z))));
+}
+// q_root P
+__device__ __forceinline__ float4 root_qmul(float4 a, float4 b) {
+    return make_float4(__fmaf_rn(-a.w, b.w, __fmaf_rn(-a.z, b.z, dot2(a.x, b.x, -a.y, b.y))),
+                       __fmaf_rn(-a.w, b.z, __fmaf_rn(a.z, b.w, dot2(a.y, b.x, a.x, b.y))),
+                       __fmaf_rn(a.w, b.y, __fmaf_rn(a.z, b.x, dot2(a.x, b.z, -a.y, b.w))),
+                       __fmaf_rn(a.w, b.x, __fmaf_rn(-a.z, b.y, dot2(a.y, b.z, a.x, b.w))));
+}
+__device__ __forceinline__ float3 tile_qrot(float4 q, float3 v) {
+    const float tx = __fmaf_rn(q.x, v.x, dot2(q.z, v.z, -q.w, v.y));
+    const float ty = __fmaf_rn(q.x, v.y, dot2(q.w, v.x, -q.y, v.z));
+    const float tz = __fmaf_rn(q.x, v.z, dot2(q.y, v.y, -q.z, v.x));
+    return make_float3(__fmaf_rn(2.f, dot2(q.z, tz, -q.w, ty), v.x), __fmaf_rn(2.f, dot2(q.w, tx, -q.y, tz), v.y),
+                       __fmaf_rn(2.f, dot2(q.y, ty, -q.z, tx), v.z));
+}
+// Rotation matrix rows and origin of a unit quaternion's frame
+struct TileFrame {
+    float r[3][3], o[3];
+    __device__ __forceinline__ TileFrame(float4 q, float3 origin) : o{origin.x, origin.y, origin.z} {
+        const float inv = rsqrtf(__fmaf_rn(q.w, q.w, __fmaf_rn(q.z, q.z, dot2(q.x, q.x, q.y, q.y))));
+        const float a = __fmul_rn(q.x, inv), b = __fmul_rn(q.y, inv), c = __fmul_rn(q.z, inv), d = __fmul_rn(q.w, inv);
+        r[0][0] = __fmaf_rn(-d, d, __fmaf_rn(-c, c, dot2(a, a, b, b)));
+        r[0][1] = 2.f * dot2(b, c, -a, d);
+        r[0][2] = 2.f * dot2(a, c, b, d);
+        r[1][0] = 2.f * dot2(b, c, a, d);
+        r[1][1] = __fmaf_rn(-d, d, __fmaf_rn(c, c, dot2(a, a, -b, b)));
+        r[1][2] = 2.f * dot2(c, d, -a, b);
+        r[2][0] = 2.f * dot2(-a, c, b, d);
+        r[2][1] = 2.f * dot2(c, d, a, b);
+        r[2][2] = __fmaf_rn(d, d, __fmaf_rn(-c, c, dot2(a, a, -b, b)));
+    }
+    __device__ __forceinline__ float direction(int i, float x, float y, float z) const {
+        return __fmaf_rn(r[i][2], z, dot2(r[i][0], x, r[i][1], y));
+    }
+    __device__ __forceinline__ float point(int i, float4 a) const { return __fadd_rn(o[i], direction(i, a.x, a.y, a.z)); }
+};
+
+template <int mode, int PL>
+__global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
+    extern __shared__ float4 smem4[];
+    const Tile<PL> T;
+    const LigView L = lig_view(p.pool, p.lig_off);
+    const int nc = 7 + L.nt, na = L.na;
+    uint32_t* const W = reinterpret_cast<uint32_t*>(smem4);      // pairs: a | b << 8 | type pair << 16
+    float* const C = reinterpret_cast<float*>(W + tile_words(mode, L.np));  // [3][na]
+    float* const X = C + 3 * na * PL;                            // [nc], then
+    float* const A = X + nc * PL;                                // [nn][4]
+    int* const Q = reinterpret_cast<int*>(X);                    // [3][na], later
+    float* const B = X + PL * (mode == 1 ? max(3 * na, nc + 4 * L.nn) : nc + 4 * L.nn);  // [nn][6]
+    float* const E = B + (mode == 1 ? 6 * L.nn * PL : 0);        // [warps]
+    const int first = blockIdx.x * PL, here = min(PL, p.n_poses - first);
+
+    // poses, transposed; a short last tile repeats its last pose
+    for (int i = threadIdx.x; i < PL * nc; i += blockDim.x) {
+        const int q = i / nc, c = i - q * nc;
+        X[c * PL + q] = p.poses[size_t(first + min(q, here - 1)) * nc + c];
+    }
+    if (mode != 2)
+        for (int i = threadIdx.x; i < L.np; i += blockDim.x) {
+            const int2 q = __ldg(&L.pairs[i]);
+            W[i] = uint32_t(q.x & 0xff) | uint32_t(q.x >> 16) << 8 | uint32_t(q.y) << 16;
+        }
+    __syncthreads();
+    // local rotations, frames and coordinates: the arithmetic of frames() and
+    // atom_position(), a slot per body
+    for (int k = T.slot; k < L.nn; k += T.slots) {
+        float4 aa = make_float4(1.f, 0.f, 0.f, 0.f);
+        if (k > 0) {
+            float s, c;
+            __sincosf(0.5f * X[(7 + k - 1) * PL + T.p], &s, &c);
+            const float4 ax = node_word(L.nodes, k, 1);
+            aa = make_float4(c, __fmul_rn(s, ax.x), __fmul_rn(s, ax.y), __fmul_rn(s, ax.z));
+        }
+        float* const d = A + 4 * k * PL + T.p;
+        d[0] = aa.x; d[PL] = aa.y; d[2 * PL] = aa.z; d[3 * PL] = aa.w;
+    }
+    __syncthreads();
+    auto rotation = [&](int k) {
+        const float* d = A + 4 * k * PL + T.p;
+        return make_float4(d[0], d[PL], d[2 * PL], d[3 * PL]);
+    };
+    for (int k = T.slot; k < L.nn; k += T.slots) {
+        float4 P = make_float4(1.f, 0.f, 0.f, 0.f);
+        float3 w = make_float3(0.f, 0.f, 0.f);
+        if (k > 0) {
+            P = rotation(k);
+            const float4 ok = node_word(L.nodes, k, 0);
+            w = make_float3(ok.x, ok.y, ok.z);
+            int j = VD_DCLAMP(__float_as_int(ok.w), 0, k - 1, kChkParent);
+            while (j > 0) {
+                const float4 aj = rotation(j);
+                const float4 oj = node_word(L.nodes, j, 0);
+                const float3 r = tile_qrot(aj, w);
+                w = make_float3(__fadd_rn(oj.x, r.x), __fadd_rn(oj.y, r.y), __fadd_rn(oj.z, r.z));
+                P = walk_qmul(aj, P);
+                j = VD_DCLAMP(__float_as_int(oj.w), 0, j - 1, kChkParent);
+            }
+        }
+        const float4 qr = make_float4(X[3 * PL + T.p], X[4 * PL + T.p], X[5 * PL + T.p], X[6 * PL + T.p]);
+        const float3 ro = tile_qrot(qr, w);
+        const TileFrame f(root_qmul(qr, P), make_float3(__fadd_rn(X[T.p], ro.x), __fadd_rn(X[PL + T.p], ro.y),
+                                                        __fadd_rn(X[2 * PL + T.p], ro.z)));
+        const float4 w1 = node_word(L.nodes, k, 1);
+        const int i1 = __float_as_int(node_word(L.nodes, k, 2).x);
+        for (int i = __float_as_int(w1.w); i < i1; ++i) {
+            const float4 a = __ldg(&L.atoms[i]);
+#pragma unroll
+            for (int d = 0; d < 3; ++d) C[(d * na + i) * PL + T.p] = f.point(d, a);
+        }
+        if (mode == 1) {
+            float* const b = B + 6 * k * PL + T.p;
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                b[d * PL] = f.direction(d, w1.x, w1.y, w1.z);
+                b[(3 + d) * PL] = f.o[d];
+            }
+        }
+    }
+    __syncthreads();
+    if constexpr (mode == 2) {
+        for (int i = threadIdx.x; i < here * 3 * na; i += blockDim.x) {
+            const int q = i / (3 * na), c = i - q * 3 * na, a = c / 3;
+            p.xyz_out[size_t(first) * 3 * na + i] = C[((c - 3 * a) * na + a) * PL + q];
+        }
+    } else {
+        if (mode == 1) {
+            for (int i = threadIdx.x; i < 3 * na * PL; i += blockDim.x) Q[i] = 0;
+            __syncthreads();
+        }
+        auto coords = [&](int i) {
+            return make_float3(C[i * PL + T.p], C[(na + i) * PL + T.p], C[(2 * na + i) * PL + T.p]);
+        };
+        // intra pairs: a slot takes a stretch of the pair list (sorted by second
+        // atom), the second atom's position and force in registers while it repeats
+        float e = 0.f;
+        {
+            const int twos = (L.np + 1) >> 1;  // two pairs at a time
+            const int q1 = min(L.np, 2 * int(uint32_t(T.slot + 1) * uint32_t(twos) / uint32_t(T.slots)));
+            int cur = -1;
+            float3 cb = make_float3(0.f, 0.f, 0.f);
+            float bx = 0.f, by = 0.f, bz = 0.f;  // in fixed-point units: fix is a power of two
+            auto add_to = [&](int i, float x, float y, float z) {
+                int* const d = Q + i * PL + T.p;
+                atomicAdd(d, __float2int_rn(x));
+                atomicAdd(d + na * PL, __float2int_rn(y));
+                atomicAdd(d + 2 * na * PL, __float2int_rn(z));
+            };
+            auto turn_to = [&](int b) {
+                if (mode == 1 && cur >= 0) add_to(cur, bx, by, bz);
+                cur = b;
+                bx = by = bz = 0.f;
+            };
+            for (int q = 2 * int(uint32_t(T.slot) * uint32_t(twos) / uint32_t(T.slots)); q < q1; q += 2) {
+                const bool two = q + 1 < q1;
+                const uint2 w = *reinterpret_cast<const uint2*>(W + q);
+                const uint32_t w1 = two ? w.y : w.x;
+                const int a0 = VD_DCLAMP(int(w.x & 0xff), 0, na - 1, kChkPairAtom), b0 = VD_DCLAMP(int(w.x >> 8 & 0xff), 0, na - 1, kChkPairAtom);
+                const int a1 = VD_DCLAMP(int(w1 & 0xff), 0, na - 1, kChkPairAtom), b1 = VD_DCLAMP(int(w1 >> 8 & 0xff), 0, na - 1, kChkPairAtom);
+                if (b0 != cur) {
+                    turn_to(b0);
+                    cb = coords(b0);
+                }
+                float3 cb1 = cb;
+                if (b1 != b0) cb1 = coords(b1);
+                const float3 ca0 = coords(a0), ca1 = coords(a1);
+                const float r0x = cb.x - ca0.x, r0y = cb.y - ca0.y, r0z = cb.z - ca0.z;
+                const float r1x = cb1.x - ca1.x, r1y = cb1.y - ca1.y, r1z = cb1.z - ca1.z;
+                const float d0 = r0x * r0x + r0y * r0y + r0z * r0z, d1 = r1x * r1x + r1y * r1y + r1z * r1z;
+                const float rf0 = fminf(32.f * d0, 2047.5f), rf1 = fminf(32.f * d1, 2047.5f);
+                const Trunc bin0 = trunc_pos(rf0), bin1 = trunc_pos(rf1);
+                const bool in0 = d0 < 64.f, in1 = two && d1 < 64.f;
+                float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
+                if (in0) t0 = __ldg(table_row(p.smooth, VD_DCLAMP(int(w.x >> 16), 0, kPairTypes - 1, kChkPairType), VD_DCLAMP(bin0.i, 0, kBins - 2, kChkTableBin)));
+                if (in1) t1 = __ldg(table_row(p.smooth, VD_DCLAMP(int(w1 >> 16), 0, kPairTypes - 1, kChkPairType), VD_DCLAMP(bin1.i, 0, kBins - 2, kChkTableBin)));
+                const float m0 = rf0 - bin0.f, m1 = rf1 - bin1.f, v = p.ep.v_intra;
+                const float e0 = t0.x + m0 * (t0.z - t0.x), g0 = t0.y + m0 * (t0.w - t0.y);
+                const float e1 = t1.x + m1 * (t1.z - t1.x), g1 = t1.y + m1 * (t1.w - t1.y);
+                const float c0 = (e0 > 0.f) ? __fdividef(v, v + e0) : 1.f, c1 = (e1 > 0.f) ? __fdividef(v, v + e1) : 1.f;
+                e += e0 * c0 + e1 * c1;  // zero past the cutoff
+                if (mode == 1) {
+                    if (in0) {
+                        const float h = g0 * c0 * c0 * p.ep.fix, Fx = h * r0x, Fy = h * r0y, Fz = h * r0z;
+                        add_to(a0, -Fx, -Fy, -Fz);
+                        bx += Fx; by += Fy; bz += Fz;
+                    }
+                    if (b1 != b0) turn_to(b1);
+                    if (in1) {
+                        const float h = g1 * c1 * c1 * p.ep.fix, Fx = h * r1x, Fy = h * r1y, Fz = h * r1z;
+                        add_to(a1, -Fx, -Fy, -Fz);
+                        bx += Fx; by += Fy; bz += Fz;
+                    }
+                } else {
+                    cur = b1;
+                }
+                cb = cb1;
+            }
+            turn_to(-1);
+        }
+        if (mode == 1) __syncthreads();
+        // grid terms; an atom's total force takes the place of its pair force
+        const GridInter inter{&p.G, p.ep.v_inter, p.ep.slope};
+        for (int i = T.slot; i < na; i += T.slots) {
+            const float3 c = coords(i);
+            float g[3];
+            e += inter(__float_as_int(__ldg(&L.atoms[i].w)) & 0xff, c.x, c.y, c.z, g[0], g[1], g[2]);
+            if (mode == 1)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    int* const f = Q + (d * na + i) * PL + T.p;
+                    *reinterpret_cast<float*>(f) = g[d] + from_fixed(*f, p.ep.inv_fix);
+                }
+        }
+#pragma unroll
+        for (int o = 16; o >= PL; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);  // the warp's slots
+        if ((threadIdx.x & 31) < PL) E[(threadIdx.x >> 5) * PL + T.p] = e;
+        __syncthreads();
+        if (threadIdx.x < here) {
+            float sum = 0.f;
+            for (int s = 0; s < blockDim.x >> 5; ++s) sum += E[s * PL + threadIdx.x];
+            p.e_out[first + threadIdx.x] = sum;
+        }
+        if constexpr (mode == 1) {
+            // a body's force and torque about its origin: the atoms of its subtree
+            for (int k = T.slot; k < L.nn; k += T.slots) {
+                float* const b = B + 6 * k * PL + T.p;
+                const float ox = b[3 * PL], oy = b[4 * PL], oz = b[5 * PL];
+                const float* const F = reinterpret_cast<const float*>(Q) + T.p;
+                float fx = 0.f, fy = 0.f, fz = 0.f, tx = 0.f, ty = 0.f, tz = 0.f;
+                const int i1 = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 2).w), 0, na, kChkSubtree);
+                for (int i = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 1).w), 0, na, kChkSubtree); i < i1; ++i) {
+                    const float3 c = coords(i);
+                    const float x = F[i * PL], y = F[(na + i) * PL], z = F[(2 * na + i) * PL];
+                    const float dx = c.x - ox, dy = c.y - oy, dz = c.z - oz;
+                    fx += x; fy += y; fz += z;
+                    tx += dy * z - dz * y;
+                    ty += dz * x - dx * z;
+                    tz += dx * y - dy * x;
+                }
+                if (k == 0) {
+                    b[0] = fx; b[PL] = fy; b[2 * PL] = fz; b[3 * PL] = tx; b[4 * PL] = ty; b[5 * PL] = tz;
+                } else {
+                    b[0] = tx * b[0] + ty * b[PL] + tz * b[2 * PL];
+                }
+            }
+            __syncthreads();
+            const int n = 6 + L.nt;
+            for (int i = threadIdx.x; i < here * n; i += blockDim.x) {
+                const int q = i / n, c = i - q * n;
+                p.g_out[size_t(first) * n + i] = B[(c < 6 ? c : 6 * (c - 5)) * PL + q];
+            }
+        }
+    }
+}
+
+// Which kernel, and tile, by measurement (us on B200, energy + gradient | energy,
+// warp per pose -> tile):
+//   24 atoms / 5 torsions (~200 pairs): 64 poses 8.8 -> 9.7, 1,000 8.5 -> 10.5,
+//     3,000 10.6 -> 12.4, 10,000 22.8 -> 17.7 | 16.7 -> 14.6, 65,536 105 -> 60 | 66 -> 50
+//   33 / 9: 10,007 poses 41.4 -> 31.0 | 29.9 -> 27.0
+//   40 / 10 (595 pairs): 64 poses 13.6 -> 10.6, 300 14.6 -> 12.6, 1,000 14.7 -> 13.6,
+//     4,096 22.9 -> 21.1, 65,536 256 -> 175 | 198 -> 139
+//   90 / 32 (~3,500 pairs): 64 poses 47.6 -> 16.7, 500 49.5 -> 22.8, 3,001 78 -> 62 | 74 -> 55
+// A small ligand's evaluation in one warp is as short as a tile's phases, so
+// below kTilePairs pairs it takes 64 poses per SM (two tiles of 32) for the
+// tiles to pay.  Poses per tile: as many as leave two tiles per SM.
+constexpr int kTilePairs = 400;
+
+template <int mode>
+vd_status launch_tile(Ctx& c, const HostLigand& L, const PoseParams& p, int sms, cudaStream_t stream) {
+    const int np = L.h.n_pairs;
+    const double per_sm = double(p.n_poses) / (2.0 * sms);  // poses per tile for two tiles per SM
+    const int poses = per_sm >= 32 ? 32 : per_sm >= 16 ? 16 : per_sm >= 8 ? 8 : per_sm >= 1.5 ? 4 : 1;
+    int warps = (poses == 32 && np >= kTilePairs) || (poses <= 4 && np >= 1500) ? 16 : 8;
+    auto bytes = [&](int w) {
+        return (size_t(tile_words(mode, np)) + size_t(tile_rows(mode, L.h.n_atoms, L.h.n_nodes, L.h.ntors, w)) * poses) *
+               sizeof(float);
+    };
+    const size_t smem = bytes(warps);
+    VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the pose kernel");
+    auto k = poses == 32 ? tile_kernel<mode, 32> : poses == 16 ? tile_kernel<mode, 16> : poses == 8 ? tile_kernel<mode, 8>
+             : poses == 4 ? tile_kernel<mode, 4> : tile_kernel<mode, 1>;
+    VD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    const int resident = std::max(1, std::min(int(227 * 1024 / (smem + 1024)), 32 / warps));  // 64 registers
+    VD_CUDA(prefer_l1(k, c.device, resident, smem));
+    k<<<(p.n_poses + poses - 1) / poses, 32 * warps, smem, stream>>>(p);
+    VD_CUDA(cudaGetLastError());
+    return VD_OK;
+}
+
 // Local optimisation, one RILC-BFGS run per pose; poses come from a queue
 // (their numbers of evaluations differ several times over).  team > 1: a
 // block takes one pose at a time, evaluated by a team of warps.
@@ -183,13 +520,14 @@ vd_status run_pose_kernel(Ctx& c, int lig, int n_poses, const float* d_poses, co
     if constexpr (mode == 3) {
         return launch_local_opt(c, L, p, stream);
     } else {
+        int dev_sms = 148;
+        cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c.device);
+        if (L.h.n_pairs >= kTilePairs || n_poses >= 64 * dev_sms) return launch_tile<mode>(c, L, p, dev_sms, stream);
         const size_t smem = size_t(p.warp_floats) * kPoseWarps * sizeof(float);
         VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the pose kernel");
         auto kern = pose_kernel<mode>;
         VD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
         VD_CUDA(prefer_l1(kern, c.device, kPoseBlocks, smem));
-        int dev_sms = 148;
-        cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c.device);
         const int blocks = std::min((n_poses + kPoseWarps - 1) / kPoseWarps, dev_sms * 16);
         kern<<<blocks, 32 * kPoseWarps, smem, stream>>>(p);
         VD_CUDA(cudaGetLastError());
