@@ -104,6 +104,9 @@ vd_status vd_create(vd_ctx** out, int device) {
     vd_ctx* h = new vd_ctx();
     Ctx& c = h->c;
     c.device = device;
+    c.sms = prop.multiProcessorCount;
+    c.smem_sm = int(prop.sharedMemPerMultiprocessor);
+    c.smem_reserved = int(prop.reservedSharedMemPerBlock);
     for (int i = 0; i < kTypes; ++i) c.map_slot[i] = -1;
     if (cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreate(&c.ev0) != cudaSuccess || cudaEventCreate(&c.ev1) != cudaSuccess ||

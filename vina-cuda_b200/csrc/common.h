@@ -4,6 +4,7 @@
 #include <cstddef>
 #include <cstdint>
 #include <cstdio>
+#include <algorithm>
 #include <string>
 #include <unordered_map>
 #include <vector>
@@ -113,6 +114,7 @@ struct HostLigand {
     // host-side copies for helpers
     std::vector<int32_t> heavy_index;  // device atom -> input atom index
     int32_t n_all_atoms = 0;
+    int32_t max_partners = 0;          // most intra pairs of one heavy atom
     int64_t pool_offset = 0;       // in float4 words
     double num_tors = 0;
 };
@@ -127,6 +129,10 @@ struct GridGeom {
 
 struct Ctx {
     int device = 0;
+    int sms = 148, smem_sm = 0, smem_reserved = 0;  // device attributes: SMs, shared memory per SM, per block for the driver
+    // Launch settings this context has given its kernels (set_launch): the
+    // driver is asked again only when they change.
+    std::unordered_map<const void*, int> carveout;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     bool scoring = false;
@@ -199,22 +205,33 @@ inline cudaError_t record_event(cudaEvent_t e, cudaStream_t s) {
                                                : cudaEventRecord(e, s);
 }
 
+// Launch settings of a kernel that takes `smem` bytes of dynamic shared memory.
+//
+// The most a block may ask for is always set to the same value, the SM's
+// whole, whatever this launch needs: kernels belong to the process, and a
+// context that set only its own need could take another's away.
+//
 // Each SM's on-chip data memory is split between shared memory and L1.  Asks
 // for the smallest shared-memory carve-out that holds `blocks` resident
-// blocks of `smem` bytes each (plus the driver's per-block reservation); the
-// percentage is rounded up and the driver rounds it up again to a capacity
-// it supports.  The rest is L1, which caches the kernels' table and grid
-// gathers.
+// blocks (plus the driver's per-block reservation); the percentage is rounded
+// up and the driver rounds it up again to a capacity it supports.  The rest
+// is L1, which caches the kernels' table and grid gathers.  It is a hint: two
+// contexts that want different ones only lose some L1.  Each of the two
+// driver calls costs about 0.6 us, of 6 for a small pose batch.
 template <class K>
-inline cudaError_t prefer_l1(K kernel, int device, int blocks, size_t smem) {
-    int max_sm = 0, reserved = 0;
-    cudaError_t r = cudaDeviceGetAttribute(&max_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, device);
-    if (r == cudaSuccess) r = cudaDeviceGetAttribute(&reserved, cudaDevAttrReservedSharedMemoryPerBlock, device);
-    if (r != cudaSuccess || max_sm <= 0) return r;
-    const size_t need = size_t(blocks) * (smem + size_t(reserved));
-    size_t pct = (need * 100 + size_t(max_sm) - 1) / size_t(max_sm);
-    if (pct > 100) pct = 100;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, int(pct));
+inline cudaError_t set_launch(Ctx& c, K kernel, int blocks, size_t smem, size_t static_smem = 0) {
+    int pct = -1;
+    if (blocks > 0 && c.smem_sm > 0) {
+        const size_t need = size_t(blocks) * (smem + static_smem + size_t(c.smem_reserved));
+        pct = int(std::min<size_t>(100, (need * 100 + size_t(c.smem_sm) - 1) / size_t(c.smem_sm)));
+    }
+    const void* const key = reinterpret_cast<const void*>(kernel);
+    const auto it = c.carveout.find(key);
+    if (it != c.carveout.end() && it->second == pct) return cudaSuccess;
+    cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(227 * 1024 - static_smem));
+    if (r == cudaSuccess && pct >= 0) r = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+    if (r == cudaSuccess) c.carveout[key] = pct;
+    return r;
 }
 
 vd_status ensure_scratch(Ctx* c, size_t bytes);

@@ -414,8 +414,7 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     // the 128-register shape, whose aim is the same, for a caller or an
     // autotuner that picks that shape; the plain form, whose chains are alike,
     // takes it without exploring.
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    const int sms = c.sms;
     const size_t smem_team = (size_t(max_wf) + pair_team_floats(max_sp)) * sizeof(float);
     const bool few = items <= sms * kTeamChains && smem_team <= 227 * 1024 / kTeamChains;
     if (out.tuned && few && !persistent) {
@@ -429,8 +428,7 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     const DockFn k = team ? team_dock_fn(dense) : dense ? dense_dock_fn(out.shape) : dock_fn(out.shape);
     const size_t smem = team ? smem_team : smem_warps;
     const int threads = team ? 32 * kTeamWarps : 32 * wpb;
-    VD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    VD_CUDA(prefer_l1(k, c.device, team ? kTeamChains : kShapeBlocks[out.shape], smem));
+    VD_CUDA(set_launch(c, k, team ? kTeamChains : kShapeBlocks[out.shape], smem));
     const int chains = team ? 1 : wpb;  // per block
     int per_sm = 0;
     VD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem));
@@ -627,11 +625,10 @@ extern "C" vd_status vd_mc_chains_noalloc(vd_ctx* h, int32_t lig, const vd_searc
     const size_t smem = size_t(p.warp_floats) * wpb * sizeof(float);
     VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "vd_mc_chains_noalloc: ligand too large for the kernel");
     auto k = sp->dense_bfgs ? dock_kernel<8, true> : dock_kernel<8>;
-    VD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int sms = 148, per_sm = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    VD_CUDA(set_launch(c, k, kShapeBlocks[0], smem));
+    int per_sm = 0;
     VD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, 32 * wpb, smem));
-    k<<<std::min(sms * std::max(1, per_sm), (n + wpb - 1) / wpb), 32 * wpb, smem, c.stream>>>(p);
+    k<<<std::min(c.sms * std::max(1, per_sm), (n + wpb - 1) / wpb), 32 * wpb, smem, c.stream>>>(p);
     VD_CUDA(cudaGetLastError());
     VD_CUDA(cudaMemcpyAsync(poses_out, d_conf, size_t(n) * nc * sizeof(float), cudaMemcpyDeviceToHost, c.stream));
     VD_CUDA(cudaMemcpyAsync(e_out, d_e, size_t(n) * sizeof(float), cudaMemcpyDeviceToHost, c.stream));

@@ -60,22 +60,24 @@ struct LigView {
     float num_tors;
 };
 
+__device__ __forceinline__ LigView lig_view(const float4* b, const LigHeader& h) {
+    LigView L;
+    L.na = h.n_atoms;
+    L.nn = h.n_nodes;
+    L.np = h.n_pairs;
+    L.nt = h.ntors;
+    L.num_tors = h.num_tors;
+    L.atoms = b + h.off_atoms;
+    L.nodes = reinterpret_cast<const NodeRec*>(b + h.off_nodes);
+    L.pairs = reinterpret_cast<const int2*>(b + h.off_pairs);
+    L.lpairs = reinterpret_cast<const int4*>(b + h.off_lpairs);
+    L.spairs = reinterpret_cast<const int2*>(b + h.off_spairs);
+    L.sp_iters = h.sp_iters;
+    return L;
+}
 __device__ __forceinline__ LigView lig_view(const float4* pool, int64_t off) {
     const float4* b = pool + off;
-    const LigHeader* h = reinterpret_cast<const LigHeader*>(b);
-    LigView L;
-    L.na = h->n_atoms;
-    L.nn = h->n_nodes;
-    L.np = h->n_pairs;
-    L.nt = h->ntors;
-    L.num_tors = h->num_tors;
-    L.atoms = b + h->off_atoms;
-    L.nodes = reinterpret_cast<const NodeRec*>(b + h->off_nodes);
-    L.pairs = reinterpret_cast<const int2*>(b + h->off_pairs);
-    L.lpairs = reinterpret_cast<const int4*>(b + h->off_lpairs);
-    L.spairs = reinterpret_cast<const int2*>(b + h->off_spairs);
-    L.sp_iters = h->sp_iters;
-    return L;
+    return lig_view(b, *reinterpret_cast<const LigHeader*>(b));
 }
 
 // Body frame in shared memory, 20 floats: three rows [R(i,0) R(i,1) R(i,2) o_i]
@@ -775,22 +777,25 @@ __device__ inline float eval_pose_team(const LigView& L, const WarpMem& m, const
 // The other warps (w = 1 .. warps - 1) of a team: view(work) gives the ligand
 // and its arrays in the team's shared memory; entries w - 1, w - 1 + (warps -
 // 1), .. of its pair schedule, the first one loaded ahead of the wait.
+// known: the work of the first evaluation where it is known before the wait, or 0.
 template <int warps, class View>
 __device__ inline void pair_team_helper(const View& view, const float4* smooth, float v_intra, float fix, int w, int lane,
-                                        const PairTeam& tm) {
+                                        const PairTeam& tm, int known = 0) {
     int cur = 0;
     LigView L;
     WarpMem m;
     int2 first = make_int2(-65536, -65536);
+    auto turn_to = [&](int work) {
+        cur = work;
+        view(work - 1, L, m);
+        if (w - 1 < L.sp_iters) first = __ldg(L.spairs + 32 * (w - 1) + lane);
+    };
+    if (known) turn_to(known);
     for (;;) {
         team_sync<warps>(1);
         const int work = *reinterpret_cast<volatile int*>(tm.work);
         if (work == 0) return;
-        if (work != cur) {
-            cur = work;
-            view(work - 1, L, m);
-            if (w - 1 < L.sp_iters) first = __ldg(L.spairs + 32 * (w - 1) + lane);
-        }
+        if (work != cur) turn_to(work);
         int2 qq = first;
         for (int k = w - 1; k < L.sp_iters; k += warps - 1) {
             const int2 now = qq;

@@ -471,9 +471,10 @@ vd_status vd_build_grids(vd_ctx* h, const int32_t* types, int32_t n_types) {
     const GridFn wide = tz == 8 ? grid_build_kernel<8, 8> : grid_build_kernel<8, 4>;
     const GridFn narrow = tz == 8 ? grid_build_kernel<4, 8> : grid_build_kernel<4, 4>;
     auto carve = [&](GridFn kern) -> cudaError_t {
+        if (c.carveout.count(reinterpret_cast<const void*>(kern))) return cudaSuccess;
         cudaFuncAttributes fa{};
         const cudaError_t r = cudaFuncGetAttributes(&fa, kern);
-        return r != cudaSuccess ? r : prefer_l1(kern, c.device, 16 / tz, fa.sharedSizeBytes);
+        return r != cudaSuccess ? r : set_launch(c, kern, 16 / tz, 0, fa.sharedSizeBytes);
     };
     if (nt > 4) VD_CUDA(carve(wide));
     if (nt % 8 >= 1 && nt % 8 <= 4) VD_CUDA(carve(narrow));

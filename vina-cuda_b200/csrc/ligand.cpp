@@ -254,6 +254,8 @@ vd_status build_ligand(const vd_ligand_desc* d, HostLigand& L) {
     if (!spairs.empty()) std::memcpy(base + 16 * size_t(H.off_spairs), spairs.data(), spairs.size() * sizeof(int2));
     L.heavy_index = heavy_index;
     L.n_all_atoms = na;
+    std::vector<int> partners(nh, 0);
+    for (const int2& q : pairs) L.max_partners = std::max({L.max_partners, ++partners[q.x & 0xffff], ++partners[q.x >> 16]});
     L.num_tors = d->num_tors;
     return VD_OK;
 }

@@ -12,8 +12,8 @@ namespace {
 constexpr int kPoseWarps = 4;
 
 struct PoseParams {
-    const float4* pool;
-    int64_t lig_off;
+    const float4* lig;  // the ligand's blob
+    LigHeader h;        // and its header: a call has one ligand, so no block waits for it
     MapView G;
     const float4* smooth;
     EvalParams ep;
@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(32 * kPoseWarps, kPoseBlocks) pose_kernel(Pose
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float* base = reinterpret_cast<float*>(smem4) + size_t(wid) * p.warp_floats;
-    const LigView L = lig_view(p.pool, p.lig_off);
+    const LigView L = lig_view(p.lig, p.h);
     const WarpMem m = carve(base, L.na, L.nn, L.np, L.nt);
     const int nc = 7 + L.nt, n = 6 + L.nt;
     for (int pose = blockIdx.x * kPoseWarps + wid; pose < p.n_poses; pose += gridDim.x * kPoseWarps) {
@@ -63,6 +63,46 @@ __global__ void __launch_bounds__(32 * kPoseWarps, kPoseBlocks) pose_kernel(Pose
         }
         __syncwarp();
     }
+}
+
+// Modes 0 and 1 for few poses of a small ligand: a team of four warps per pose
+// (eval.cuh), one evaluation and out.  Latency is all of it: us per launch in a
+// graph on B200, a warp per pose -> a team, 64 poses of 8 / 16 / 24 / 30 atoms:
+// 4.1 / 4.6 / 5.8 / 7.5 -> 3.5 / 3.9 / 3.9 / 4.4; 1,036 poses: 4.8 / 5.1 / 6.5 /
+// 8.2 -> 4.1 / 4.4 / 4.9 / 5.7.
+constexpr int kPoseTeam = 4, kTeamPoses = 7;  // warps per pose, poses resident per SM
+template <int mode>
+__global__ void __launch_bounds__(32 * kPoseTeam, kTeamPoses) pose_team_kernel(PoseParams p) {
+    extern __shared__ float4 smem4[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, pose = blockIdx.x;
+    float* base = reinterpret_cast<float*>(smem4);
+    const LigView L = lig_view(p.lig, p.h);
+    const WarpMem m = carve(base, L.na, L.nn, L.np, L.nt);
+    const PairTeam tm = pair_team(base + p.warp_floats);
+    if (wid > 0) {
+        const auto view = [&](int, LigView& l, WarpMem& w) {
+            l = L;
+            w = m;
+        };
+        pair_team_helper<kPoseTeam>(view, p.smooth, p.ep.v_intra, p.ep.fix, wid, lane, tm, 1);
+        return;
+    }
+    const int nc = 7 + L.nt, n = 6 + L.nt;
+    if (lane == 0) *tm.work = 1;
+    const float* src = p.poses + size_t(pose) * nc;
+    for (int i = lane; i < nc; i += 32) m.x[i] = src[i];
+    __syncwarp();
+    const GridInter gi{&p.G, p.ep.v_inter, p.ep.slope};
+    const float thr = mode == 0 ? -INFINITY : INFINITY;  // energy only: no adjoint
+    const float e = eval_pose_team<kPoseTeam>(L, m, gi, p.ep.inv_fix, lane, tm, SkipAbove{thr});
+    if (lane == 0) {
+        p.e_out[pose] = e;
+        *tm.work = 0;
+    }
+    __syncwarp();
+    team_arrive<kPoseTeam>(1);
+    if (mode == 1)
+        for (int i = lane; i < n; i += 32) p.g_out[size_t(pose) * n + i] = m.g[i];
 }
 
 // ---------------------------------------------------------------- pose tiles
@@ -154,7 +194,7 @@ template <int mode, int PL>
 __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
     extern __shared__ float4 smem4[];
     const Tile<PL> T;
-    const LigView L = lig_view(p.pool, p.lig_off);
+    const LigView L = lig_view(p.lig, p.h);
     const int nc = 7 + L.nt, na = L.na;
     uint32_t* const W = reinterpret_cast<uint32_t*>(smem4);      // pairs: a | b << 8 | type pair << 16
     float* const C = reinterpret_cast<float*>(W + tile_words(mode, L.np));  // [3][na]
@@ -312,7 +352,7 @@ __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
             turn_to(-1);
         }
         if (mode == 1) __syncthreads();
-        // grid terms; an atom's total force takes the place of its pair force
+        // grid terms; an atom's total force takes the place of its pair force.
         const GridInter inter{&p.G, p.ep.v_inter, p.ep.slope};
         for (int i = T.slot; i < na; i += T.slots) {
             const float3 c = coords(i);
@@ -342,14 +382,20 @@ __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
                 const float* const F = reinterpret_cast<const float*>(Q) + T.p;
                 float fx = 0.f, fy = 0.f, fz = 0.f, tx = 0.f, ty = 0.f, tz = 0.f;
                 const int i1 = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 2).w), 0, na, kChkSubtree);
-                for (int i = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 1).w), 0, na, kChkSubtree); i < i1; ++i) {
-                    const float3 c = coords(i);
-                    const float x = F[i * PL], y = F[(na + i) * PL], z = F[(2 * na + i) * PL];
-                    const float dx = c.x - ox, dy = c.y - oy, dz = c.z - oz;
-                    fx += x; fy += y; fz += z;
-                    tx += dy * z - dz * y;
-                    ty += dz * x - dx * z;
-                    tz += dx * y - dy * x;
+                int i = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 1).w), 0, na, kChkSubtree);
+                while (i < i1) {  // sums of up to 8 atoms first: a long chain of additions loses digits
+                    float sx = 0.f, sy = 0.f, sz = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
+                    for (const int stop = min(i + 8, i1); i < stop; ++i) {
+                        const float3 c = coords(i);
+                        const float x = F[i * PL], y = F[(na + i) * PL], z = F[(2 * na + i) * PL];
+                        const float dx = c.x - ox, dy = c.y - oy, dz = c.z - oz;
+                        sx += x; sy += y; sz += z;
+                        ux += dy * z - dz * y;
+                        uy += dz * x - dx * z;
+                        uz += dx * y - dy * x;
+                    }
+                    fx += sx; fy += sy; fz += sz;
+                    tx += ux; ty += uy; tz += uz;
                 }
                 if (k == 0) {
                     b[0] = fx; b[PL] = fy; b[2 * PL] = fz; b[3 * PL] = tx; b[4 * PL] = ty; b[5 * PL] = tz;
@@ -381,9 +427,9 @@ __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
 constexpr int kTilePairs = 400;
 
 template <int mode>
-vd_status launch_tile(Ctx& c, const HostLigand& L, const PoseParams& p, int sms, cudaStream_t stream) {
+vd_status launch_tile(Ctx& c, const HostLigand& L, const PoseParams& p, cudaStream_t stream) {
     const int np = L.h.n_pairs;
-    const double per_sm = double(p.n_poses) / (2.0 * sms);  // poses per tile for two tiles per SM
+    const double per_sm = double(p.n_poses) / (2.0 * c.sms);  // poses per tile for two tiles per SM
     const int poses = per_sm >= 32 ? 32 : per_sm >= 16 ? 16 : per_sm >= 8 ? 8 : per_sm >= 1.5 ? 4 : 1;
     int warps = (poses == 32 && np >= kTilePairs) || (poses <= 4 && np >= 1500) ? 16 : 8;
     auto bytes = [&](int w) {
@@ -394,9 +440,8 @@ vd_status launch_tile(Ctx& c, const HostLigand& L, const PoseParams& p, int sms,
     VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the pose kernel");
     auto k = poses == 32 ? tile_kernel<mode, 32> : poses == 16 ? tile_kernel<mode, 16> : poses == 8 ? tile_kernel<mode, 8>
              : poses == 4 ? tile_kernel<mode, 4> : tile_kernel<mode, 1>;
-    VD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const int resident = std::max(1, std::min(int(227 * 1024 / (smem + 1024)), 32 / warps));  // 64 registers
-    VD_CUDA(prefer_l1(k, c.device, resident, smem));
+    VD_CUDA(set_launch(c, k, resident, smem));
     k<<<(p.n_poses + poses - 1) / poses, 32 * warps, smem, stream>>>(p);
     VD_CUDA(cudaGetLastError());
     return VD_OK;
@@ -410,7 +455,7 @@ __global__ void __launch_bounds__(32 * (team > 1 ? team : kPoseWarps), blocks) l
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float* base = reinterpret_cast<float*>(smem4) + (team > 1 ? size_t(0) : size_t(wid) * p.warp_floats);
-    const LigView L = lig_view(p.pool, p.lig_off);
+    const LigView L = lig_view(p.lig, p.h);
     SearchMem s;
     s.m = carve(base, L.na, L.nn, L.np, L.nt);
     const PairTeam tm = pair_team(base + p.warp_floats);
@@ -419,7 +464,7 @@ __global__ void __launch_bounds__(32 * (team > 1 ? team : kPoseWarps), blocks) l
             l = L;
             m = s.m;
         };
-        pair_team_helper<team>(view, p.smooth, p.ep.v_intra, p.ep.fix, wid, lane, tm);
+        pair_team_helper<team>(view, p.smooth, p.ep.v_intra, p.ep.fix, wid, lane, tm, 1);
         return;
     }
     s.xp = base + warp_floats(L.na, L.nn, L.np, L.nt);
@@ -464,9 +509,8 @@ __global__ void __launch_bounds__(32 * (team > 1 ? team : kPoseWarps), blocks) l
 // 431 (80 registers: 454), 2,000 593 -> 510 (531), 2,800 644 -> 480, 8,000 1,515
 // -> 1,150; 44 atoms, 1,000 poses 669 -> 415.
 vd_status launch_local_opt(Ctx& c, const HostLigand& L, const PoseParams& p, cudaStream_t stream) {
-    constexpr int kTeam = 4, kTeamPoses = 7, kWide = 4, kNarrow = 6;
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device);
+    constexpr int kTeam = kPoseTeam, kWide = 4, kNarrow = 6;
+    const int sms = c.sms;
     const size_t smem_team = (size_t(p.warp_floats) + pair_team_floats(L.h.sp_iters)) * sizeof(float);
     const bool team = p.n_poses <= sms * kTeamPoses && smem_team <= 227 * 1024 / kTeamPoses;
     const bool wide = p.n_poses <= sms * kWide * kPoseWarps;
@@ -474,8 +518,7 @@ vd_status launch_local_opt(Ctx& c, const HostLigand& L, const PoseParams& p, cud
     VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the pose kernel");
     auto k = team ? local_opt_kernel<kTeamPoses, kTeam> : wide ? local_opt_kernel<kWide, 1> : local_opt_kernel<kNarrow, 1>;
     const int threads = 32 * (team ? kTeam : kPoseWarps), poses = team ? 1 : kPoseWarps;  // per block
-    VD_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    VD_CUDA(prefer_l1(k, c.device, team ? kTeamPoses : wide ? kWide : kNarrow, smem));
+    VD_CUDA(set_launch(c, k, team ? kTeamPoses : wide ? kWide : kNarrow, smem));
     int per_sm = 0;
     VD_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem));
     const int blocks = std::min(sms * std::max(1, per_sm), (p.n_poses + poses - 1) / poses);
@@ -501,12 +544,20 @@ vd_status run_pose_kernel(Ctx& c, int lig, int n_poses, const float* d_poses, co
         if (st != VD_OK) return st;
     }
     const HostLigand& L = c.ligs[lig];
-    p.pool = c.d_pool;
-    p.lig_off = L.pool_offset;
+    p.lig = c.d_pool + L.pool_offset;
+    p.h = L.h;
     p.smooth = c.d_smooth;
     const vd_eval_params def = {10.0, 10.0, 1e6};
     const vd_eval_params* e = ep ? ep : &def;
-    p.ep = {float(e->v_intra), float(e->v_inter), float(e->slope), c.fix_scale, 1.f / c.fix_scale};
+    // One evaluation's forces may use the bits that the context's scale keeps
+    // for 128 partners of an atom where this ligand's atoms have fewer: a team or
+    // a tile rounds a pair's force more often than a warp, and this leaves the
+    // gradient's error below the warp's at the context's scale.  The optimisers
+    // keep that scale: their runs are the docking search's.
+    float fix = c.fix_scale;
+    if (mode == 0 || mode == 1)
+        for (int d = std::max(1, L.max_partners); 2 * d <= 128; d *= 2) fix *= 2.f;
+    p.ep = {float(e->v_intra), float(e->v_inter), float(e->slope), fix, 1.f / fix};
     p.poses = d_poses;
     p.n_poses = n_poses;
     p.e_out = d_e;
@@ -520,15 +571,21 @@ vd_status run_pose_kernel(Ctx& c, int lig, int n_poses, const float* d_poses, co
     if constexpr (mode == 3) {
         return launch_local_opt(c, L, p, stream);
     } else {
-        int dev_sms = 148;
-        cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, c.device);
-        if (L.h.n_pairs >= kTilePairs || n_poses >= 64 * dev_sms) return launch_tile<mode>(c, L, p, dev_sms, stream);
+        if (L.h.n_pairs >= kTilePairs || n_poses >= 64 * c.sms) return launch_tile<mode>(c, L, p, stream);
+        if constexpr (mode != 2) {
+            if (n_poses <= kTeamPoses * c.sms) {
+                const size_t smem = (size_t(p.warp_floats) + pair_team_floats(L.h.sp_iters)) * sizeof(float);
+                VD_CUDA(set_launch(c, pose_team_kernel<mode>, kTeamPoses, smem));
+                pose_team_kernel<mode><<<n_poses, 32 * kPoseTeam, smem, stream>>>(p);
+                VD_CUDA(cudaGetLastError());
+                return VD_OK;
+            }
+        }
         const size_t smem = size_t(p.warp_floats) * kPoseWarps * sizeof(float);
         VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the pose kernel");
         auto kern = pose_kernel<mode>;
-        VD_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        VD_CUDA(prefer_l1(kern, c.device, kPoseBlocks, smem));
-        const int blocks = std::min((n_poses + kPoseWarps - 1) / kPoseWarps, dev_sms * 16);
+        VD_CUDA(set_launch(c, kern, kPoseBlocks, smem));
+        const int blocks = std::min((n_poses + kPoseWarps - 1) / kPoseWarps, c.sms * 16);
         kern<<<blocks, 32 * kPoseWarps, smem, stream>>>(p);
         VD_CUDA(cudaGetLastError());
         return VD_OK;

@@ -1121,7 +1121,7 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     cp.warps = int(std::min<size_t>(kClusterThreads / 32, (227 * 1024 - 64 - smem_c1) / b_wf));
     cp.warps = std::max(1, cp.warps);
     const size_t smem_c = smem_c1 + cp.warps * b_wf;
-    VD_CUDA(cudaFuncSetAttribute(cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_c)));
+    VD_CUDA(set_launch(c, cluster_kernel, 0, smem_c, 64));
     // refine
     const bool refine = sp.refine != 0;
     RefineParams rp{};
@@ -1144,7 +1144,7 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
         rp.skip_invalid = 1;
         smem_r = size_t(max_rwf) * 4;
         VD_CHECK(smem_r <= 227 * 1024, VD_ERR_CAPACITY, "refine kernel shared memory exceeds 227 KB");
-        VD_CUDA(cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_r)));
+        VD_CUDA(set_launch(c, refine_kernel, 0, smem_r));
         blocks_r = n * VD_MAX_MODES;
     }
     // score
@@ -1164,7 +1164,7 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     sc.out = d_out;
     const size_t smem_s = size_t(VD_MAX_MODES) * pose_doubles(max_na, max_nn) * 8;
     VD_CHECK(smem_s <= 226 * 1024, VD_ERR_CAPACITY, "score kernel shared memory exceeds 226 KB");
-    VD_CUDA(cudaFuncSetAttribute(score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_s)));
+    VD_CUDA(set_launch(c, score_kernel, 0, smem_s, 1024));
     const int stride = db.stride;
     const float* conf = db.d_conf;
     const float* e = db.d_e;
@@ -1391,7 +1391,7 @@ vd_status vd_refine(vd_ctx* h, int32_t lig, int32_t n, float* poses, int32_t max
     rp.skip_invalid = 0;
     const size_t smem_r = size_t(refine_floats(L)) * 4;
     VD_CHECK(smem_r <= 227 * 1024, VD_ERR_CAPACITY, "refine kernel shared memory exceeds 227 KB");
-    VD_CUDA(cudaFuncSetAttribute(refine_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem_r)));
+    VD_CUDA(set_launch(c, refine_kernel, 0, smem_r));
     refine_kernel<<<n, 32 * kRefineWarps, smem_r, c.stream>>>(rp);
     VD_CUDA(cudaGetLastError());
     VD_CUDA(cudaMemcpyAsync(poses, d_p, size_t(n) * nc * 4, cudaMemcpyDeviceToHost, c.stream));
@@ -1422,8 +1422,7 @@ vd_status vd_score(vd_ctx* h, int32_t lig, int32_t n, const float* poses, float*
     VD_CUDA(cudaMemcpyAsync(d_p, poses, size_t(n) * nc * 4, cudaMemcpyHostToDevice, c.stream));
     const int64_t off = L.pool_offset;
     VD_CUDA(cudaMemcpyAsync(d_off, &off, 8, cudaMemcpyHostToDevice, c.stream));
-    VD_CUDA(cudaFuncSetAttribute(score_poses_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(pose_doubles(L.h.n_atoms, L.h.n_nodes)) * 8));
+    VD_CUDA(set_launch(c, score_poses_kernel, 0, size_t(pose_doubles(L.h.n_atoms, L.h.n_nodes)) * 8, 1024));
     score_poses_kernel<<<n, 32 * kScoreWarps, size_t(pose_doubles(L.h.n_atoms, L.h.n_nodes)) * 8, c.stream>>>(
         c.d_pool, d_off, d_p, nc, rec_view(c), c.d_fastd, d_o);
     VD_CUDA(cudaGetLastError());
@@ -1460,7 +1459,7 @@ vd_status vd_rmsd_bounds(vd_ctx* h, int32_t lig, int32_t n, const float* poses, 
     const int64_t off = L.pool_offset;
     VD_CUDA(cudaMemcpyAsync(d_off, &off, 8, cudaMemcpyHostToDevice, c.stream));
     const size_t smem = size_t(kRmsdWarps + 1) * pose_doubles(L.h.n_atoms, L.h.n_nodes) * 8;
-    VD_CUDA(cudaFuncSetAttribute(rmsd_poses_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    VD_CUDA(set_launch(c, rmsd_poses_kernel, 0, smem));
     rmsd_poses_kernel<<<(n + kRmsdWarps - 1) / kRmsdWarps, 32 * (kRmsdWarps + 1), smem, c.stream>>>(c.d_pool, d_off, d_p,
                                                                                                    n, nc, d_o);
     VD_CUDA(cudaGetLastError());

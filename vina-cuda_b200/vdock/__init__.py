@@ -303,12 +303,13 @@ class Context:
         return e, g
 
     def energy_grad_device(self, lig, n, poses_ptr, e_ptr, g_ptr, stream_ptr=0, ep=None):
-        _check(self.L.vd_energy_grad_device(self.h, lig, n, _vp(poses_ptr), C.byref(ep or eval_params()),
-                                            _vp(e_ptr), _vp(g_ptr), _vp(stream_ptr or None)))
+        # plain integers: the argument types convert them (None: the library's
+        # defaults, eval_params())
+        _check(self.L.vd_energy_grad_device(self.h, lig, n, poses_ptr, ep and C.byref(ep), e_ptr, g_ptr,
+                                            stream_ptr or None))
 
     def energy_device(self, lig, n, poses_ptr, e_ptr, stream_ptr=0, ep=None):
-        _check(self.L.vd_energy_device(self.h, lig, n, _vp(poses_ptr), C.byref(ep or eval_params()), _vp(e_ptr),
-                                       _vp(stream_ptr or None)))
+        _check(self.L.vd_energy_device(self.h, lig, n, poses_ptr, ep and C.byref(ep), e_ptr, stream_ptr or None))
 
     def pose_coords(self, lig, poses):
         p, pp = _f(poses)
