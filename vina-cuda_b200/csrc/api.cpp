@@ -163,9 +163,10 @@ vd_status vd_get_stats(vd_ctx* h, vd_stats* out) {
 }
 
 // After new tables: maps built with the old weights are stale.
-static void scoring_changed(Ctx& c, std::chrono::steady_clock::time_point t0) {
+static void scoring_changed(Ctx& c, double force_bound, bool on_device, std::chrono::steady_clock::time_point t0) {
     c.scoring = true;
-    c.fix_scale = pair_force_scale(c.sd);
+    c.fix_scale = pair_force_scale(force_bound);
+    c.tables_on_device = on_device;
     c.n_maps = 0;
     for (int i = 0; i < kTypes; ++i) c.map_slot[i] = -1;
     c.stats.scoring_ms = std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
@@ -200,7 +201,7 @@ vd_status vd_set_scoring(vd_ctx* h, const double weights[6]) {
     VD_CUDA(cudaMemcpy(c.d_fastd, fd.data(), fd.size() * sizeof(double), cudaMemcpyHostToDevice));
     VD_CUDA(cudaMemcpy(c.d_fast, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
     VD_CUDA(cudaMemcpy(c.d_smooth, s.data(), s.size() * sizeof(float4), cudaMemcpyHostToDevice));
-    scoring_changed(c, t0);
+    scoring_changed(c, pair_force_bound(c.sd), false, t0);
     return VD_OK;
 }
 
@@ -212,14 +213,19 @@ vd_status vd_set_scoring_device(vd_ctx* h, const double weights[6]) {
     const auto t0 = std::chrono::steady_clock::now();
     VD_CUDA(cudaSetDevice(c.device));
     std::memcpy(c.weights, weights, sizeof(c.weights));
-    vd_status st = build_tables_device(c, weights);
+    double bound = 0;
+    vd_status st = build_tables_device(c, bound);
     if (st != VD_OK) return st;
-    scoring_changed(c, t0);
+    scoring_changed(c, bound, true, t0);
     return VD_OK;
 }
 
 vd_status vd_get_tables(vd_ctx* h, double* fast, double* se, double* sd) {
     VD_CHECK(h, VD_ERR_ARG, "vd_get_tables: NULL context");
+    if (h->c.tables_on_device) {
+        VD_CUDA(cudaSetDevice(h->c.device));
+        return fetch_tables(h->c, fast, se, sd);
+    }
     const size_t n = size_t(kPairTypes) * kN * sizeof(double);
     if (fast) std::memcpy(fast, h->c.fast.data(), n);
     if (se) std::memcpy(se, h->c.se.data(), n);

@@ -137,7 +137,8 @@ struct Ctx {
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     bool scoring = false;
     double weights[6];
-    std::vector<double> fast, se, sd;     // [153][2051] double (host)
+    std::vector<double> fast, se, sd;     // [153][2051] double (host), of the last host build
+    bool tables_on_device = false;        // the current ones were built there: fast, se, sd are not they
     float* d_fast = nullptr;              // [153][2049] float (rescoring, eval_fast)
     float4* d_smooth = nullptr;           // [153][2049] {e_i, dor_i, e_i+1, dor_i+1}
     float fix_scale = 524288.f;           // fixed-point units per kcal/mol/A of the pair forces
@@ -260,13 +261,16 @@ vd_status sync_pool(Ctx* c);
 vd_status ensure_receptor_cells(Ctx* c);
 void build_tables(const double w[6], std::vector<double>& fast, std::vector<double>& se,
                   std::vector<double>& sd);
-// Largest power of two (at most 2^24) for which 128 times the largest pair
-// force of the derivative table stays below 2^30: the fixed-point scale of
-// the kernels' per-atom pair-force sums.
-float pair_force_scale(const std::vector<double>& sd);
-// Same tables built on the device into the context's device copies, with
-// the double tables copied back to c.fast / c.se / c.sd.
-vd_status build_tables_device(Ctx& c, const double w[6]);
+// Largest pair force of the derivative table, and the largest power of two (at
+// most 2^24) for which 128 times it stays below 2^30: the fixed-point scale of
+// the kernels' per-atom pair-force sums (an atom has at most 127 partners).
+double pair_force_bound(const std::vector<double>& sd);
+float pair_force_scale(double bound);
+// Same tables built on the device from c.weights into the context's device
+// copies, and their largest pair force; the double tables stay there until
+// fetch_tables (any of its arrays may be null).
+vd_status build_tables_device(Ctx& c, double& force_bound);
+vd_status fetch_tables(Ctx& c, double* fast, double* se, double* sd);
 
 }  // namespace vd
 

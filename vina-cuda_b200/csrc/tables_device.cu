@@ -5,8 +5,10 @@
 // evaluates the weighted XS energy at its own and its neighbouring sample
 // distances in FP64 and writes
 //   se[i], sd[i] = (e[i+1]-e[i-1]) / ((r[i+1]-r[i-1]) r[i]), fast[i] = (e[i]+e[i+1])/2
-// in double (copied back for the host-side consumers) plus the device copies
-// the kernels read: fast in FP32 and FP64, smooth as {e_i, dor_i, e_i+1, dor_i+1}.
+// in double plus the device copies the kernels read: fast in FP32 and FP64,
+// smooth as {e_i, dor_i, e_i+1, dor_i+1}.  The largest pair force, which sets the
+// fixed-point scale, is found here too; the double tables cross to the host
+// only for vd_get_tables (7.5 MB: 1.6 of the 2.1 ms a weight set took).
 // This file is compiled without FMA contraction so the arithmetic rounds like
 // the host build; only exp() may differ from the host's, by an ulp.
 #include <cfloat>
@@ -59,9 +61,24 @@ __global__ void __launch_bounds__(256) tables_kernel(TableParams p) {
     }
 }
 
+// Largest |derivative| x r over the reachable bins (pair_force_bound): the
+// doubles are not negative, so their bits order like them.
+__global__ void __launch_bounds__(256) force_bound_kernel(const double* sd, unsigned long long* bound) {
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x, tp = gid / kBins, i = gid - tp * kBins;
+    double v = 0;
+    if (tp < kPairTypes && i + 1 < kBins) {
+        const double* d = sd + size_t(tp) * kN + i;
+        v = fmax(0.0, fmax(fabs(d[0]), fabs(d[1])) * sqrt((i + 1) / 32.0));  // a NaN counts as 0, as on the host
+    }
+    for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(bound, static_cast<unsigned long long>(__double_as_longlong(v)));
+}
+
 }  // namespace
 
-vd_status build_tables_device(Ctx& c, const double w[6]) {
+// Tables of c.weights into the device copies, the doubles into the scratch
+// (fast, se, sd in turn).
+static vd_status run_tables(Ctx& c, double*& doubles) {
     const size_t n = size_t(kPairTypes) * kN, nb = size_t(kPairTypes) * kBins;
     vd_status st = VD_OK;
     if (!c.d_fast && (st = dev_alloc(c, &c.d_fast, nb * sizeof(float), "pair tables")) != VD_OK) return st;
@@ -70,8 +87,8 @@ vd_status build_tables_device(Ctx& c, const double w[6]) {
     st = ensure_scratch(&c, 3 * n * sizeof(double));
     if (st != VD_OK) return st;
     TableParams p{};
-    for (int k = 0; k < 6; ++k) p.w[k] = w[k];
-    p.fast = static_cast<double*>(c.d_scratch);
+    for (int k = 0; k < 6; ++k) p.w[k] = c.weights[k];
+    doubles = p.fast = static_cast<double*>(c.d_scratch);
     p.se = p.fast + n;
     p.sd = p.se + n;
     p.fast_f = c.d_fast;
@@ -79,12 +96,31 @@ vd_status build_tables_device(Ctx& c, const double w[6]) {
     p.smooth = c.d_smooth;
     tables_kernel<<<unsigned((n + 255) / 256), 256, 0, c.stream>>>(p);
     VD_CUDA(cudaGetLastError());
-    c.fast.resize(n);
-    c.se.resize(n);
-    c.sd.resize(n);
-    VD_CUDA(cudaMemcpyAsync(c.fast.data(), p.fast, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    VD_CUDA(cudaMemcpyAsync(c.se.data(), p.se, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
-    VD_CUDA(cudaMemcpyAsync(c.sd.data(), p.sd, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    return VD_OK;
+}
+
+vd_status build_tables_device(Ctx& c, double& force_bound) {
+    const size_t n = size_t(kPairTypes) * kN, nb = size_t(kPairTypes) * kBins;
+    double* d = nullptr;
+    const vd_status st = run_tables(c, d);
+    if (st != VD_OK) return st;
+    unsigned long long* const bound = reinterpret_cast<unsigned long long*>(c.d_counter + 16);
+    VD_CUDA(cudaMemsetAsync(bound, 0, sizeof(*bound), c.stream));
+    force_bound_kernel<<<unsigned((nb + 255) / 256), 256, 0, c.stream>>>(d + 2 * n, bound);
+    VD_CUDA(cudaGetLastError());
+    VD_CUDA(cudaMemcpyAsync(&force_bound, bound, sizeof(double), cudaMemcpyDeviceToHost, c.stream));
+    VD_CUDA(cudaStreamSynchronize(c.stream));
+    return VD_OK;
+}
+
+vd_status fetch_tables(Ctx& c, double* fast, double* se, double* sd) {
+    const size_t n = size_t(kPairTypes) * kN;
+    double* d = nullptr;
+    const vd_status st = run_tables(c, d);  // the same values again: the scratch has had other uses since
+    if (st != VD_OK) return st;
+    double* const out[3] = {fast, se, sd};
+    for (int k = 0; k < 3; ++k)
+        if (out[k]) VD_CUDA(cudaMemcpyAsync(out[k], d + k * n, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     VD_CUDA(cudaStreamSynchronize(c.stream));
     return VD_OK;
 }
