@@ -109,15 +109,16 @@ __device__ __forceinline__ Vec2 vload(const float* g, int n, int lane) {
 }
 
 // x = xp + alpha * d (conf.h:367-372); xp, x in shared memory.  Lanes 0-2
-// step the position components they hold; lane 3 rotates the orientation
-// by the rotation vector in lanes 3-5.
+// step the position components they hold; the orientation is rotated by the
+// vector in lanes 3-5 in all lanes alike, so that its long chain (square
+// root, division, sine) overlaps with the torsions' instead of standing in a
+// branch of its own.
 __device__ __forceinline__ void conf_step(const float* xp, float* x, Vec2 d, float alpha, int nt, int lane) {
-    const float d4 = __shfl_down_sync(0xffffffffu, d.a, 1), d5 = __shfl_down_sync(0xffffffffu, d.a, 2);
+    const float d3 = __shfl_sync(0xffffffffu, d.a, 3), d4 = __shfl_sync(0xffffffffu, d.a, 4),
+                d5 = __shfl_sync(0xffffffffu, d.a, 5);
+    const float4 q = quat_increment(make_float4(xp[3], xp[4], xp[5], xp[6]), alpha * d3, alpha * d4, alpha * d5);
     if (lane < 3) x[lane] = xp[lane] + alpha * d.a;
-    if (lane == 3) {
-        const float4 q = quat_increment(make_float4(xp[3], xp[4], xp[5], xp[6]), alpha * d.a, alpha * d4, alpha * d5);
-        x[3] = q.x; x[4] = q.y; x[5] = q.z; x[6] = q.w;
-    }
+    if (lane == 3) { x[3] = q.x; x[4] = q.y; x[5] = q.z; x[6] = q.w; }
     const int t0 = lane - 6, t1 = lane + 26;  // torsion held in slot a / b
     if (t0 >= 0 && t0 < nt) x[7 + t0] = norm_angle(xp[7 + t0] + norm_angle(alpha * d.a));
     if (t1 < nt) x[7 + t1] = norm_angle(xp[7 + t1] + norm_angle(alpha * d.b));
@@ -133,6 +134,13 @@ struct SearchMem {  // per-warp shared memory of the optimiser
     WarpMem m;      // m.x is the working pose
     float* xp;      // previous pose in the line search
     float* xo;      // pose at entry (restored if the run got worse)
+    // The working pose becomes the line search's start, the old start's array
+    // the next trial's (a step writes all of it).
+    __device__ __forceinline__ void keep_as_start() {
+        float* const x = xp;
+        xp = m.x;
+        m.x = x;
+    }
 };
 
 // quasi_newton.cuh:2172-2389 (RILC-BFGS) with the Lewis-Overton line search
@@ -152,7 +160,7 @@ struct SearchMem {  // per-warp shared memory of the optimiser
 // quasi_newton.cuh:1937-1939).
 // eval(skip): as in dense_bfgs below.
 template <class Eval>
-__device__ inline float rilc_bfgs(const LigView& L, const SearchMem& s, const Eval& eval, int max_steps, int lane,
+__device__ inline float rilc_bfgs(const LigView& L, SearchMem& s, const Eval& eval, int max_steps, int lane,
                                   int& evals, bool entry_only = false) {
     const int n = 6 + L.nt, nc = 7 + L.nt;
     if (max_steps <= 0) max_steps = 1000;  // the reference's 0 means unbounded
@@ -227,7 +235,7 @@ __device__ inline float rilc_bfgs(const LigView& L, const SearchMem& s, const Ev
             step = 1.f;
         }
         // start a line search from the current pose
-        copy_conf(s.m.x, s.xp, nc, lane);
+        s.keep_as_start();
         gp = g;
         fxp = fx;
         count = 0;
@@ -269,7 +277,7 @@ struct SkipArmijo {
 // --rilc_bfgs 0 (grid maps).  eval(skip): energy of the pose in s.m.x and,
 // unless skip(energy), its gradient in s.m.g.
 template <class Eval>
-__device__ float dense_bfgs(const LigView& L, const SearchMem& s, float* H, float* gc, float* pv, float* yv,
+__device__ float dense_bfgs(const LigView& L, SearchMem& s, float* H, float* gc, float* pv, float* yv,
                            float* mhy, const Eval& eval, int max_steps, int lane, int& evals) {
     const int n = 6 + L.nt, nc = 7 + L.nt;
     for (int i = lane; i < n * n; i += 32) H[i] = (i / n == i % n) ? 1.f : 0.f;
@@ -340,7 +348,7 @@ __device__ float dense_bfgs(const LigView& L, const SearchMem& s, float* H, floa
             pv[i] = -sum;
         }
         __syncwarp();
-        copy_conf(s.m.x, s.xp, nc, lane);
+        s.keep_as_start();
         p = vload(pv, n, lane);
         g = vload(gc, n, lane);
         pg = vdot(p, g);
