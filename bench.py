@@ -156,7 +156,7 @@ def fp32_roof(flops, ms, clk, device):
 # wavefront per SM per cycle.  Shapes not captured report neither.
 DOCK_DRAM_PER_ABYTE = {4: 0.07919}
 DOCK_L1_WAVEFRONTS_PER_ABYTE = {4: 0.10198}
-DOCK_SHAPES = 3  # launch shapes the docking autotuner explores (register budgets 64 / 80 / 128)
+DOCK_SHAPES = 3  # most launch shapes the docking autotuner explores for one workload (register budgets 64 / 80 / 128)
 # L1 data-pipe (LSU) wavefronts of one grid build of this workload (188^3
 # points x 8 maps, 8,000-atom receptor), from the ncu capture summarised in
 # profiles/grid_build_kernel_70A_8types.txt (l1tex__data_pipe_lsu_wavefronts.sum

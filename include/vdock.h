@@ -89,8 +89,10 @@ typedef struct {
     double   amplitude;       /* mutation amplitude 2 (monte_carlo.h:71)       */
     double   min_rmsd;        /* cluster radius 1.0                            */
     int32_t  refine;          /* 1 = refine + rescore on the GPU (main.cpp:434)*/
-    int32_t  launch_shape;    /* docking kernel shape: 0 = autotuned per
-                                 workload (among 1, 4, 5), 1/2/3/4/5 =
+    int32_t  launch_shape;    /* docking kernel shape: 0 = by the workload (4
+                                 when its chains fill the GPU several times
+                                 over, 5 when the longest decide, otherwise
+                                 autotuned), 1/2/3/4/5 =
                                  64/48/40/80/128 registers per thread
                                  (8/10/12/6/4 blocks of 4 chains per SM; with
                                  few chains shape 5 runs a team of 4 warps

@@ -17,7 +17,8 @@
 // block per four chains instead, a block's slots stayed empty until its
 // slowest chain ended: 6,500 chains of one ligand, 80 registers, B200, 24
 // atoms 5.37 -> 4.91 ms, 31 atoms 12.52 -> 11.92, 44 atoms 38.6 -> 37.6 (128
-// registers: 45.1 -> 36.4).
+// registers: 45.1 -> 36.4).  These three take 4.6, 10.9 and 34.6 with the evaluation
+// as it is now.
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -246,12 +247,12 @@ DockFn dense_dock_fn(int& shape) {
 // per chain takes the pairs off it (three warps compute them while the first
 // looks up the grid).  Chains of one ligand, 60 steps, 22 A box, ms on B200,
 // one warp per chain at 128 registers -> team:
-//   24 atoms / 5 torsions:  64 chains 9.96 -> 7.55, 592 11.39 -> 9.41, 1,024 11.87 -> 10.07,
-//                           1,500 12.99 -> 16.13
-//   40 atoms / 10 torsions: 256 chains 28.3 -> 16.7, 1,024 29.7 -> 20.9, 2,048 33.6 -> 36.7
+//   24 atoms / 5 torsions:  64 chains 9.41 -> 6.75, 592 10.68 -> 8.16, 1,024 11.30 -> 8.79
+//   40 atoms / 10 torsions: 256 chains 26.4 -> 15.8, 1,024 28.9 -> 18.8
+// (queued past 7 chains per SM: 1,500 chains 13.0 -> 16.1, 2,048 of the larger 33.6 -> 36.7)
 // so it is used while all chains are resident at once: 7 blocks per SM, the most
 // whose 72 registers per thread hold the kernel without spills.  (Teams of 2, 3, 6
-// and 8 warps: 10.94, 10.52, 16.1 and 16.4 at 1,024 chains of the first ligand.)
+// and 8 warps: 10.94, 10.52, 16.1 and 16.4 at 1,024 chains of the first ligand, when four took 10.07.)
 constexpr int kTeamWarps = 4;   // warps per chain
 constexpr int kTeamChains = 7;  // chains resident per SM
 constexpr int kWideShape = 4;   // the 128-register shape
@@ -268,28 +269,35 @@ int dense_floats(int ntors) {
 
 }  // namespace
 
-// The autotuner's candidates: 64, 80 and 128 registers.  The 48- and
-// 40-register shapes spill heavily and were slower on every measured
-// workload (wide-box screen, single ligand, uneven batch); they stay
-// available to callers that pin a shape.  Tried in this order: a new
-// context's first call runs the shape that is best or next to it on most
-// workloads (6,500 chains of a 31-atom ligand: 80 registers 11.9 ms, 128
-// 12.3, 64 12.5; 64 screened ligands: 793, 918, 839).
-constexpr int kTunedShapes[] = {3, 4, 0};
-constexpr int kNumTuned = int(sizeof(kTunedShapes) / sizeof(kTunedShapes[0]));
-
-int dock_shape_for(Ctx& c, const vd_search_params& sp, uint64_t key) {
-    if (sp.launch_shape >= 1 && sp.launch_shape <= kDockShapes) return sp.launch_shape - 1;
-    return kTunedShapes[c.dock_tune.pick(key, kNumTuned)];
-}
+// Which register budget a launch takes when the caller pins none.  The 48-
+// and 40-register shapes spill heavily and were slower on every measured
+// workload; they stay available to callers that pin a shape.  What decides
+// between 80 registers (24 chains per SM) and 128 (16, each faster) is how
+// much of the launch is its tail: `tail` is the longest chain's estimated
+// work over an even share of all chains' work, with 24 per SM resident.
+// Kernel ms at 80 registers and what 128 and 64 change, B200:
+//   tail 0.05  64 ligands x 6,500 chains       673   +11.6 %   +6.7 %
+//        0.2   31 atoms x 16,000 (24 / 44)     14.9 / 45.5   +15.8 / +5.1   +12.6 / +9.9
+//        0.4   31 atoms x 8,192 (24 / 44)      8.49 / 25.9   +12.7 / +4.8   +15.7 / +15.8
+//        1.0   3,600 chains (24 / 44 / 80)     4.39 / 14.1 / 48.0   +19.4 / +4.7 / -2.3   +28 to +37
+//        1.1   16 ligands x 400                21.6   -7.6   +33.9
+//        1.35  256 ligands x 32, 100 steps     156    -16.7  +25.3
+//        1.5   2,300 chains (24 / 44 / 80)     3.66 / 12.2 / 42.5   +1.5 / -4.9 / -4.6   +31 to +47
+//        2.4   1,500 chains (24 / 44)          3.36 / 11.7   -2.0 / -9.3   +29 / +39
+// Below kSaturated and above kTailBound the rule decides; between them the
+// autotuner runs both once and keeps the faster, since a wrong guess costs up
+// to 19 %.  Launches small enough for a team per chain (kTeamChains) take the
+// team for 128 registers and explore all three.
+constexpr int kNarrowShape = 3;  // the 80-register shape
+constexpr double kSaturated = 0.5, kTailBound = 1.25;
 
 void dock_tune_report(Ctx& c, const DockBuffers& b, double ms, const unsigned long long* lig_evals) {
     if (!b.tuned) return;
     double work = 0;
     for (size_t i = 0; i < b.eval_bytes.size(); ++i) work += double(lig_evals[i]) * b.eval_bytes[i];
     if (!(work > 0)) return;
-    for (int i = 0; i < kNumTuned; ++i)
-        if (kTunedShapes[i] == b.shape) c.dock_tune.report(b.tune_key, i, ms / work);
+    for (size_t i = 0; i < b.candidates.size(); ++i)
+        if (b.candidates[i] == b.shape) c.dock_tune.report(b.tune_key, int(i), ms / work);
 }
 
 // Heuristics of main.cpp:354-391 (atoms = all ligand atoms): search depth
@@ -331,6 +339,7 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     std::vector<int32_t> prefix(n + 1, 0), depth(n), steps(n);
     std::vector<uint32_t> uid(n);
     int max_wf = 0, max_nt = 0, max_sp = 0;
+    double work = 0, longest = 0;  // of all chains, of one chain: MC steps x BFGS steps x bytes per evaluation
     for (int i = 0; i < n; ++i) {
         st = check_ligand_maps(c, ligs[i]);
         if (st != VD_OK) return st;
@@ -340,6 +349,9 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
         search_defaults(L, sp, depth[i], steps[i]);
         prefix[i + 1] = prefix[i] + sp.n_chains;
         out.eval_bytes.push_back(32.0 * L.h.n_atoms + 16.0 * L.h.n_pairs);
+        const double chain = std::max(1.0, double(depth[i]) * steps[i]) * out.eval_bytes.back();
+        work += chain * sp.n_chains;
+        longest = std::max(longest, chain);
         max_wf = std::max(max_wf, lig_warp_floats(L) + 4 * pad4(7 + L.h.ntors) + kChainWords +
                                       (sp.dense_bfgs ? dense_floats(L.h.ntors) : 0));
         max_nt = std::max(max_nt, L.h.ntors);
@@ -401,7 +413,7 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     p.lig_evals = out.d_lig_evals;
     p.warp_floats = max_wf;
     p.visited = sp.visited_history;
-    // launch shape: register budget from the caller or the autotuner, keyed
+    // launch shape: register budget from the caller, the rule or the autotuner, keyed
     // by form, work items and shared memory per chain
     const int wpb = 4;
     const size_t smem_warps = size_t(max_wf) * wpb * sizeof(float);
@@ -409,19 +421,26 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     out.tune_key = (uint64_t(persistent) << 40) | (uint64_t(ceil_log2(uint64_t(items))) << 32) |
                    uint64_t(max_wf > 1024);  // above 4 KB per chain, shared memory caps the occupancy
     out.tune_key |= uint64_t(sp.dense_bfgs != 0) << 41;
-    out.tuned = sp.launch_shape == 0;
+    out.tuned = sp.launch_shape < 1 || sp.launch_shape > kDockShapes;
     // Few chains: a team of warps per chain (see kTeamChains) in the place of
     // the 128-register shape, whose aim is the same, for a caller or an
     // autotuner that picks that shape; the plain form, whose chains are alike,
-    // takes it without exploring.
+    // takes it without exploring.  More chains: see kTailBound.
     const int sms = c.sms;
     const size_t smem_team = (size_t(max_wf) + pair_team_floats(max_sp)) * sizeof(float);
     const bool few = items <= sms * kTeamChains && smem_team <= 227 * 1024 / kTeamChains;
-    if (out.tuned && few && !persistent) {
-        out.tuned = false;
+    const double tail = work > 0 ? longest * kShapeBlocks[kNarrowShape] * wpb * sms / work : 0;
+    out.tune_key |= uint64_t(few) << 42;
+    if (!out.tuned) {
+        out.shape = sp.launch_shape - 1;
+    } else if (few ? !persistent : tail > kTailBound) {
         out.shape = kWideShape;
+    } else if (!few && tail < kSaturated) {
+        out.shape = kNarrowShape;
     } else {
-        out.shape = dock_shape_for(c, sp, out.tune_key);
+        out.candidates = {kNarrowShape, kWideShape};
+        if (few) out.candidates = {kWideShape, kNarrowShape, 0};
+        out.shape = out.candidates[c.dock_tune.pick(out.tune_key, int(out.candidates.size()))];
     }
     const bool team = few && out.shape == kWideShape;
     const bool dense = sp.dense_bfgs != 0;

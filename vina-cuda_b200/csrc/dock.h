@@ -21,6 +21,7 @@ struct DockBuffers {
     std::vector<double> eval_bytes; // per ligand: algorithmic bytes of one evaluation (tuner cost unit)
     int shape = 0;                  // launch shape used (0-based)
     bool tuned = false;             // shape came from the autotuner
+    std::vector<int> candidates;    // shapes that the autotuner explores for this launch
     std::vector<unsigned char> h_params;  // packed parameter arrays (host)
     void* d_params = nullptr;             // their device copy
     std::function<cudaError_t(cudaStream_t)> launch;  // the kernel launch
