@@ -76,3 +76,23 @@ def test_refinement_sizes(rec_atoms, radius, na, nt):
             checked += 1
             same += abs(r - e1[i]) <= 2e-3 * max(1.0, abs(r))
     assert checked >= 10 and same >= 0.9 * checked, (same, checked)
+
+
+def test_non_finite_poses_stay_in_bounds():
+    """Positions and torsions that are infinite or not a number have no
+    receptor cell: they take an edge cell, and the poses beside them are
+    refined and scored to the same bits as without them."""
+    ctx, _, lig, lc, _, synth = _env(1200, 24.0, 33, 9)
+    starts = synth.random_poses(12, ctx.ntors[lc], -2.0, 2.0, seed=4)
+    e0, p0 = ctx.refine(lc, starts, 5)
+    s0 = ctx.score(lc, starts)
+    bad = starts.copy()
+    rows = {2: (0, np.nan), 5: (1, np.inf), 7: (2, -np.inf), 8: (7, np.nan), 10: (0, 3e38)}
+    for i, (k, v) in rows.items():
+        bad[i, k] = v
+    e1, p1 = ctx.refine(lc, bad, 5)
+    s1 = ctx.score(lc, bad)
+    keep = [i for i in range(len(starts)) if i not in rows]
+    assert np.array_equal(e0[keep], e1[keep]) and np.array_equal(p0[keep], p1[keep])
+    for a, b in zip(s0, s1):
+        assert np.array_equal(np.asarray(a)[keep], np.asarray(b)[keep])

@@ -1,6 +1,8 @@
 // Pose batches: forward energy kernel, adjoint kernel (energy + gradient,
 // recomputing atom coordinates from the torsion tree), coordinates, and
-// one RILC-BFGS local optimisation per pose.  One warp per pose.
+// one RILC-BFGS local optimisation per pose.  Batches run as tiles of poses
+// with one pose per lane (tile_kernel), a few poses as teams of warps
+// (pose_team_kernel), what is between on one warp per pose.
 #include <cstring>
 
 #include "launch.h"
@@ -505,9 +507,9 @@ __global__ void __launch_bounds__(32 * (team > 1 ? team : kPoseWarps), blocks) l
 // docking kernel), else one warp per pose, at 128 registers (4 blocks) while
 // all poses are resident, else at 80 (6 blocks).  31-atom ligand, at most 20
 // steps, us a call on B200, before (one warp a pose at 140 registers, 3 blocks
-// per SM, no queue) -> now: 50 poses 287 -> 215, 1,000 426 -> 340, 1,300 449 ->
-// 431 (80 registers: 454), 2,000 593 -> 510 (531), 2,800 644 -> 480, 8,000 1,515
-// -> 1,150; 44 atoms, 1,000 poses 669 -> 415.
+// per SM, no queue) -> now: 50 poses 287 -> 205, 1,000 426 -> 340, 1,300 449 ->
+// 426 (80 registers: 454), 2,000 593 -> 505 (531), 2,800 644 -> 480, 8,000 1,515
+// -> 1,150; 44 atoms, 1,000 poses 669 -> 400, 1,300 758 -> 636, 2,300 1,127 -> 930.
 vd_status launch_local_opt(Ctx& c, const HostLigand& L, const PoseParams& p, cudaStream_t stream) {
     constexpr int kTeam = kPoseTeam, kWide = 4, kNarrow = 6;
     const int sms = c.sms;

@@ -42,7 +42,8 @@ struct RecView {
 // szv_grid.cpp:92-107 (fl_to_sz) in FP32: a point within rounding of a cell
 // face may take the neighbour cell, whose list reaches a little further
 // than the cutoff (ensure_receptor_cells) and so holds the same atoms in
-// reach, in the same order.
+// reach, in the same order.  Optimisers do reach poses that are not finite:
+// the conversion saturates and takes a NaN to 0, so those get a cell too.
 __device__ __forceinline__ int cell_of(const RecView& R, float x, float y, float z) {
     const float c[3] = {x, y, z};
     int idx[3];
