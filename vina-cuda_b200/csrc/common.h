@@ -266,6 +266,7 @@ void build_tables(const double w[6], std::vector<double>& fast, std::vector<doub
 // the kernels' per-atom pair-force sums (an atom has at most 127 partners).
 double pair_force_bound(const std::vector<double>& sd);
 float pair_force_scale(double bound);
+float pair_force_scale(const std::vector<double>& sd);
 // Same tables built on the device from c.weights into the context's device
 // copies, and their largest pair force; the double tables stay there until
 // fetch_tables (any of its arrays may be null).

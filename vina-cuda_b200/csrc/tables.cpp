@@ -58,4 +58,6 @@ float pair_force_scale(double bound) {
     return float(std::ldexp(1.0, k));
 }
 
+float pair_force_scale(const std::vector<double>& sd) { return pair_force_scale(pair_force_bound(sd)); }
+
 }  // namespace vd
