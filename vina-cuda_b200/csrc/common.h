@@ -191,6 +191,10 @@ struct Ctx {
     // past it into VD_ERR_NOMEM
     std::unordered_map<void*, size_t> dev_bytes;
     size_t dev_used = 0, dev_cap = 0;
+    // Whether a *_device call has been made: work on a caller's stream, or
+    // replays of a graph that one was captured into, may read the context's
+    // memory at any time from then on.
+    bool device_calls = false;
     // launch-shape autotuner (tune.h); grid_shape_fixed > 0 pins the grid tile
     Tuner dock_tune;
     int grid_shape_fixed = 0;
@@ -259,6 +263,9 @@ void dev_release(Ctx& c, T*& p) {
 vd_status ensure_host_stage(Ctx* c, size_t bytes);
 vd_status sync_pool(Ctx* c);
 vd_status ensure_receptor_cells(Ctx* c);
+// Before memory that *_device calls read is written in place: waits for what
+// may be outstanding of them.
+vd_status settle_device_calls(Ctx& c);
 void build_tables(const double w[6], std::vector<double>& fast, std::vector<double>& se,
                   std::vector<double>& sd);
 // Largest pair force of the derivative table, and the largest power of two (at

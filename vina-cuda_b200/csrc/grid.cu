@@ -418,6 +418,7 @@ vd_status vd_build_grids(vd_ctx* h, const int32_t* types, int32_t n_types) {
     // all given back first.
     if (!dev_keeps(c, c.d_maps, bytes_maps)) dev_release(c, c.d_maps);
     if (!with_cells || !dev_keeps(c, c.d_cells, bytes_cells)) dev_release(c, c.d_cells);
+    const bool kept = c.d_maps || c.d_cells;
     vd_status st = VD_OK;
     if (!c.d_maps && (st = dev_alloc(c, &c.d_maps, bytes_maps, "vd_build_grids: maps")) != VD_OK) return st;
     st = ensure_scratch(&c, bytes_atoms + bytes_start + bytes_lut);
@@ -478,6 +479,8 @@ vd_status vd_build_grids(vd_ctx* h, const int32_t* types, int32_t n_types) {
     };
     if (nt > 4) VD_CUDA(carve(wide));
     if (nt % 8 >= 1 && nt % 8 <= 4) VD_CUDA(carve(narrow));
+    // calls on other streams may still read what was kept
+    if (kept && (st = settle_device_calls(c)) != VD_OK) return st;
     const dim3 grid((g.n[0] + kTileX - 1) / kTileX, (g.n[1] + kTileY - 1) / kTileY, (g.n[2] + tz - 1) / tz);
     VD_CUDA(cudaEventRecord(c.ev0, c.stream));
     for (int g0 = 0; g0 < nt; g0 += 8) {

@@ -607,7 +607,9 @@ vd_status vd_energy_grad_device(vd_ctx* h, int32_t lig, int32_t n, const float* 
     Ctx& c = h->c;
     VD_CUDA(cudaSetDevice(c.device));
     cudaStream_t s = static_cast<cudaStream_t>(stream);  // NULL: the CUDA default stream
-    return run_pose_kernel<1>(c, lig, n, poses, ep, e, g, nullptr, nullptr, 0, s);
+    const vd_status st = run_pose_kernel<1>(c, lig, n, poses, ep, e, g, nullptr, nullptr, 0, s);
+    c.device_calls |= st == VD_OK;
+    return st;
 }
 
 vd_status vd_energy_device(vd_ctx* h, int32_t lig, int32_t n, const float* poses, const vd_eval_params* ep,
@@ -616,7 +618,9 @@ vd_status vd_energy_device(vd_ctx* h, int32_t lig, int32_t n, const float* poses
     Ctx& c = h->c;
     VD_CUDA(cudaSetDevice(c.device));
     cudaStream_t s = static_cast<cudaStream_t>(stream);  // NULL: the CUDA default stream
-    return run_pose_kernel<0>(c, lig, n, poses, ep, e, nullptr, nullptr, nullptr, 0, s);
+    const vd_status st = run_pose_kernel<0>(c, lig, n, poses, ep, e, nullptr, nullptr, nullptr, 0, s);
+    c.device_calls |= st == VD_OK;
+    return st;
 }
 
 static vd_status pose_host(vd_ctx* h, int32_t lig, int32_t n, const float* poses, const vd_eval_params* ep,
