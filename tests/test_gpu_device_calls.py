@@ -66,3 +66,49 @@ def test_rebuild_of_the_same_box(env, n, captured):
         evaluate()
     torch.cuda.synchronize()
     assert not torch.equal(e, alone[0])  # the new receptor's
+
+
+@pytest.mark.parametrize("change", ["scoring", "scoring_device", "ligands"])
+def test_new_tables_and_ligands(env, change):
+    torch, vd, synth, ctx, lig, xyz, xs = env
+    p, e, g = _buffers(torch, synth, ctx, lig, 20000)
+    side = torch.cuda.Stream()
+
+    def evaluate():
+        ctx.energy_grad_device(lig, len(p), p.data_ptr(), e.data_ptr(), g.data_ptr(), side.cuda_stream)
+
+    torch.cuda.synchronize()
+    evaluate()
+    side.synchronize()
+    alone = e.clone(), g.clone()
+    torch.cuda.synchronize()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(HOLD)
+        evaluate()
+    if change == "ligands":
+        other = synth.ligand(30, 6, 9)
+        ctx.clear_ligands()
+        ctx.pose_coords(ctx.add_ligand(other), synth.random_poses(2, 6, -1.0, 1.0, seed=1))  # uploads it
+    else:
+        ctx.set_scoring(1.5 * np.array(vd.DEFAULT_WEIGHTS), device=change == "scoring_device")
+    torch.cuda.synchronize()
+    assert torch.equal(e, alone[0]) and torch.equal(g, alone[1])
+
+
+def test_ligand_uploaded_under_capture(env):
+    """A ligand in a cleared one's place, first used by a call that is being captured."""
+    torch, vd, synth, ctx, lig, xyz, xs = env
+    p, e, g = _buffers(torch, synth, ctx, lig, 64)
+    side = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    ctx.energy_grad_device(lig, 64, p.data_ptr(), e.data_ptr(), g.data_ptr(), side.cuda_stream)
+    side.synchronize()
+    ctx.clear_ligands()
+    lig = ctx.add_ligand(synth.ligand(30, 6, 9))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side, capture_error_mode="relaxed"):
+        ctx.energy_grad_device(lig, 64, p.data_ptr(), e.data_ptr(), g.data_ptr(), side.cuda_stream)
+    graph.replay()
+    torch.cuda.synchronize()
+    want_e, want_g = ctx.energy_grad(lig, p.cpu().numpy())
+    assert np.array_equal(e.cpu().numpy(), want_e) and np.array_equal(g.cpu().numpy(), want_g)

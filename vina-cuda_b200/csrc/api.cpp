@@ -220,6 +220,7 @@ vd_status vd_set_scoring(vd_ctx* h, const double weights[6]) {
         for (int i = 0; i < kBins; ++i) fd[size_t(p) * kBins + i] = c.fast[size_t(p) * kN + i];
     if (!c.d_fastd && (st = dev_alloc(c, &c.d_fastd, fd.size() * sizeof(double), "pair tables")) != VD_OK)
         return st;
+    if ((st = settle_device_calls(c)) != VD_OK) return st;
     VD_CUDA(cudaMemcpy(c.d_fastd, fd.data(), fd.size() * sizeof(double), cudaMemcpyHostToDevice));
     VD_CUDA(cudaMemcpy(c.d_fast, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
     VD_CUDA(cudaMemcpy(c.d_smooth, s.data(), s.size() * sizeof(float4), cudaMemcpyHostToDevice));

@@ -172,6 +172,7 @@ struct Ctx {
     std::vector<HostLigand> ligs;
     float4* d_pool = nullptr;
     int64_t pool_words = 0, pool_cap = 0;   // words of all added ligands / device capacity
+    int64_t pool_high = 0;                  // words of the device pool written so far
     size_t pool_synced = 0;                 // ligands already on the device
     bool pool_dirty = false;
     // scratch

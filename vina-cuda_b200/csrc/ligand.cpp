@@ -35,6 +35,7 @@ vd_status sync_pool(Ctx* c) {
         dev_release(*c, c->d_pool);
         c->d_pool = fresh;
         c->pool_cap = cap;
+        c->pool_high = 0;
     }
     const size_t first = c->pool_synced;
     if (first < c->ligs.size()) {
@@ -44,10 +45,14 @@ vd_status sync_pool(Ctx* c) {
             const HostLigand& L = c->ligs[i];
             std::memcpy(&host[size_t(L.pool_offset - begin)], L.blob.data(), L.blob.size() * sizeof(float4));
         }
+        // where cleared ligands lay, calls on other streams may still read them
+        const vd_status st = begin < c->pool_high ? settle_device_calls(*c) : VD_OK;
+        if (st != VD_OK) return st;
         VD_CUDA(cudaMemcpyAsync(c->d_pool + begin, host.data(), host.size() * sizeof(float4), cudaMemcpyHostToDevice,
                                 c->stream));
         VD_CUDA(cudaStreamSynchronize(c->stream));
     }
+    c->pool_high = std::max(c->pool_high, words);
     c->pool_synced = c->ligs.size();
     c->pool_dirty = false;
     return VD_OK;

@@ -102,7 +102,8 @@ static vd_status run_tables(Ctx& c, double*& doubles) {
 vd_status build_tables_device(Ctx& c, double& force_bound) {
     const size_t n = size_t(kPairTypes) * kN, nb = size_t(kPairTypes) * kBins;
     double* d = nullptr;
-    const vd_status st = run_tables(c, d);
+    vd_status st = settle_device_calls(c);
+    if (st == VD_OK) st = run_tables(c, d);
     if (st != VD_OK) return st;
     unsigned long long* const bound = reinterpret_cast<unsigned long long*>(c.d_counter + 16);
     VD_CUDA(cudaMemsetAsync(bound, 0, sizeof(*bound), c.stream));
