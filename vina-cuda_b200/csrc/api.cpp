@@ -87,15 +87,40 @@ vd_status ensure_scratch(Ctx* c, size_t bytes) {
     return VD_OK;
 }
 
+// Replaces the pinned stage by one of `bytes`; keep: not before it is there.
+// A failure leaves no pending CUDA error behind.
+static cudaError_t grow_host_stage(Ctx& c, size_t bytes, bool keep) {
+    auto drop = [&] {
+        if (c.h_stage) cudaFreeHost(c.h_stage);
+        c.h_stage = nullptr;
+        c.h_stage_bytes = 0;
+    };
+    if (!keep) drop();
+    void* p = nullptr;
+    const cudaError_t e = cudaMallocHost(&p, bytes);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return e;
+    }
+    drop();
+    c.h_stage = p;
+    c.h_stage_bytes = bytes;
+    return cudaSuccess;
+}
+
 vd_status ensure_host_stage(Ctx* c, size_t bytes) {
     if (c->h_stage_bytes >= bytes) return VD_OK;
-    if (c->h_stage) VD_CUDA(cudaFreeHost(c->h_stage));
-    c->h_stage = nullptr;
-    c->h_stage_bytes = 0;
-    const size_t want = bytes + bytes / 4;
-    VD_CUDA(cudaMallocHost(&c->h_stage, want));
-    c->h_stage_bytes = want;
+    VD_CUDA(grow_host_stage(*c, bytes + bytes / 4, false));
     return VD_OK;
+}
+
+char* map_slab(Ctx& c, size_t bytes) {
+    constexpr int kPinAfter = 40;
+    if (c.h_stage_bytes < bytes && c.slab_reads <= kPinAfter && ++c.slab_reads > kPinAfter)
+        grow_host_stage(c, std::max(bytes, kMapSlab), true);  // asked for once
+    if (c.h_stage_bytes >= bytes) return static_cast<char*>(c.h_stage);
+    if (c.h_slab.size() < bytes) c.h_slab.resize(bytes);
+    return c.h_slab.data();
 }
 
 }  // namespace vd

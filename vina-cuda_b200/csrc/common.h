@@ -184,7 +184,7 @@ struct Ctx {
     void* h_stage = nullptr;
     size_t h_stage_bytes = 0;
     std::vector<char> h_slab;             // vd_get_grid: rows on their way out (about 1 MB at most)
-    int slab_reads = 0;                   // maps read through it
+    int slab_reads = 0;                   // maps read without a pinned stage, up to the one that asked for it
     cudaGraphExec_t pipe_exec = nullptr;
     vd_stats stats{};
     // device memory owned by the context (dev_alloc / dev_free): bytes in use
@@ -262,6 +262,10 @@ void dev_release(Ctx& c, T*& p) {
     p = nullptr;
 }
 vd_status ensure_host_stage(Ctx* c, size_t bytes);
+// Host memory of `bytes` through which a map is read, about kMapSlab at a time:
+// the pinned stage where it is large enough, else pageable memory.
+constexpr size_t kMapSlab = size_t(1) << 20;
+char* map_slab(Ctx& c, size_t bytes);
 vd_status sync_pool(Ctx* c);
 vd_status ensure_receptor_cells(Ctx* c);
 // Before memory that *_device calls read is written in place: waits for what

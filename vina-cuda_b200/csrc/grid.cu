@@ -537,18 +537,10 @@ vd_status vd_get_grid(vd_ctx* h, int32_t t, float* out) {
     // for a 61 x 50 x 71 map, 120 us through pinned memory; a row-wise 2D copy
     // took ~800 us, one piece straight into memory that the caller has not
     // touched yet 240 us.  Pinned memory takes 4 ms to allocate, what it saves
-    // on 40 such calls: a context allocates it once it has made that many.
-    constexpr size_t kSlab = size_t(1) << 20;
-    constexpr int kPinAfter = 40;
+    // on 40 such calls: a context asks for it once, when it has made that many.
     const size_t row = size_t(g.n[0]) * sizeof(float), pitch = size_t(g.pitch) * sizeof(float);
-    const size_t rows = size_t(g.n[1]) * g.n[2], per = std::max<size_t>(1, std::min(rows, kSlab / pitch));
-    char* slab = nullptr;
-    if (c.h_stage_bytes >= per * pitch || (++c.slab_reads > kPinAfter && ensure_host_stage(&c, per * pitch) == VD_OK)) {
-        slab = static_cast<char*>(c.h_stage);
-    } else {
-        if (c.h_slab.size() < per * pitch) c.h_slab.resize(per * pitch);
-        slab = c.h_slab.data();
-    }
+    const size_t rows = size_t(g.n[1]) * g.n[2], per = std::max<size_t>(1, std::min(rows, kMapSlab / pitch));
+    char* const slab = map_slab(c, per * pitch);
     for (size_t r0 = 0; r0 < rows; r0 += per) {
         const size_t n = std::min(per, rows - r0);
         VD_CUDA(cudaMemcpyAsync(slab, src + r0 * g.pitch, n * pitch, cudaMemcpyDeviceToHost, c.stream));
