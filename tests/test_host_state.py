@@ -26,3 +26,8 @@ def _host_check(tmp_path, name, *sources):
 def test_host_stage_check(tmp_path):
     """The pinned stage when pinned memory is refused (a compiled host check)."""
     _host_check(tmp_path, "host_stage_check", "api.cpp", "tables.cpp")
+
+
+def test_launch_settings_check(tmp_path):
+    """The kernels' launch settings when several contexts set them (a compiled host check)."""
+    _host_check(tmp_path, "launch_settings_check", "api.cpp", "tables.cpp")

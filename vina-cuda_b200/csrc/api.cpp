@@ -5,6 +5,7 @@
 #include <cstring>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 
 #include "common.h"
 
@@ -72,6 +73,36 @@ vd_status settle_device_calls(Ctx& c) {
     VD_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
     VD_CUDA(e);
     return VD_OK;
+}
+
+namespace {
+struct LaunchSettings {
+    int max_dynamic = -1, carveout = -1;  // as they are before anyone sets them: the driver's
+};
+std::mutex g_launch_mu;
+std::unordered_map<int, std::unordered_map<const void*, LaunchSettings>> g_launch;  // by device and kernel
+}  // namespace
+
+cudaError_t apply_launch_settings(int device, const void* kernel, int max_dynamic, int carveout) {
+    std::lock_guard<std::mutex> lock(g_launch_mu);
+    LaunchSettings& now = g_launch[device][kernel];
+    if (now.max_dynamic != max_dynamic) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, max_dynamic);
+        if (e != cudaSuccess) return e;
+        now.max_dynamic = max_dynamic;
+    }
+    if (now.carveout != carveout) {
+        const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
+        if (e != cudaSuccess) return e;
+        now.carveout = carveout;
+    }
+    return cudaSuccess;
+}
+
+// The kernels of a device that was reset start from the driver's settings again.
+void forget_launch_settings(int device) {
+    std::lock_guard<std::mutex> lock(g_launch_mu);
+    g_launch.erase(device);
 }
 
 vd_status ensure_scratch(Ctx* c, size_t bytes) {
@@ -148,6 +179,7 @@ vd_status vd_create(vd_ctx** out, int device) {
                   std::to_string(prop.major) + std::to_string(prop.minor));
         return VD_ERR_CUDA;
     }
+    forget_launch_settings(device);
     vd_ctx* h = new vd_ctx();
     Ctx& c = h->c;
     c.device = device;

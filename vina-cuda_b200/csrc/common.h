@@ -130,9 +130,6 @@ struct GridGeom {
 struct Ctx {
     int device = 0;
     int sms = 148, smem_sm = 0, smem_reserved = 0;  // device attributes: SMs, shared memory per SM, per block for the driver
-    // Launch settings this context has given its kernels (set_launch): the
-    // driver is asked again only when they change.
-    std::unordered_map<const void*, int> carveout;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr;
     bool scoring = false;
@@ -222,22 +219,22 @@ inline cudaError_t record_event(cudaEvent_t e, cudaStream_t s) {
 // blocks (plus the driver's per-block reservation); the percentage is rounded
 // up and the driver rounds it up again to a capacity it supports.  The rest
 // is L1, which caches the kernels' table and grid gathers.  It is a hint: two
-// contexts that want different ones only lose some L1.  Each of the two
-// driver calls costs about 0.6 us, of 6 for a small pose batch.
+// contexts on two threads that want different ones only lose some L1.
+//
+// Each of the two driver calls costs about 0.6 us, of 6 for a small pose
+// batch, so they are made when a kernel's settings on the device change.
+// These belong to the process, and so does the record of them
+// (apply_launch_settings): contexts that take turns each get their own.
+cudaError_t apply_launch_settings(int device, const void* kernel, int max_dynamic, int carveout);
+void forget_launch_settings(int device);
 template <class K>
-inline cudaError_t set_launch(Ctx& c, K kernel, int blocks, size_t smem, size_t static_smem = 0) {
-    int pct = -1;
+inline cudaError_t set_launch(const Ctx& c, K kernel, int blocks, size_t smem, size_t static_smem = 0) {
+    int pct = -1;  // the driver's choice
     if (blocks > 0 && c.smem_sm > 0) {
         const size_t need = size_t(blocks) * (smem + static_smem + size_t(c.smem_reserved));
         pct = int(std::min<size_t>(100, (need * 100 + size_t(c.smem_sm) - 1) / size_t(c.smem_sm)));
     }
-    const void* const key = reinterpret_cast<const void*>(kernel);
-    const auto it = c.carveout.find(key);
-    if (it != c.carveout.end() && it->second == pct) return cudaSuccess;
-    cudaError_t r = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(227 * 1024 - static_smem));
-    if (r == cudaSuccess && pct >= 0) r = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
-    if (r == cudaSuccess) c.carveout[key] = pct;
-    return r;
+    return apply_launch_settings(c.device, reinterpret_cast<const void*>(kernel), int(227 * 1024 - static_smem), pct);
 }
 
 vd_status ensure_scratch(Ctx* c, size_t bytes);

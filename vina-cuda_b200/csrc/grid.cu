@@ -472,7 +472,6 @@ vd_status vd_build_grids(vd_ctx* h, const int32_t* types, int32_t n_types) {
     const GridFn wide = tz == 8 ? grid_build_kernel<8, 8> : grid_build_kernel<8, 4>;
     const GridFn narrow = tz == 8 ? grid_build_kernel<4, 8> : grid_build_kernel<4, 4>;
     auto carve = [&](GridFn kern) -> cudaError_t {
-        if (c.carveout.count(reinterpret_cast<const void*>(kern))) return cudaSuccess;
         cudaFuncAttributes fa{};
         const cudaError_t r = cudaFuncGetAttributes(&fa, kern);
         return r != cudaSuccess ? r : set_launch(c, kern, 16 / tz, 0, fa.sharedSizeBytes);
