@@ -468,7 +468,7 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
 vd_status enqueue_dock(Ctx& c, const DockBuffers& b, const void* params_src, cudaStream_t stream) {
     VD_CUDA(cudaMemcpyAsync(b.d_params, params_src, b.h_params.size(), cudaMemcpyHostToDevice, stream));
     VD_CUDA(cudaMemsetAsync(b.d_lig_evals, 0, (b.prefix.size() - 1) * sizeof(unsigned long long), stream));
-    VD_CUDA(cudaMemsetAsync(c.d_counter, 0, 16, stream));
+    VD_CUDA(cudaMemsetAsync(c.d_counter, 0, 24, stream));  // queue, search and refinement evaluations
     VD_CUDA(record_event(c.ev0, stream));
     VD_CUDA(b.launch(stream));
     VD_CUDA(record_event(c.ev1, stream));

@@ -1369,11 +1369,10 @@ vd_status vd_refine(vd_ctx* h, int32_t lig, int32_t n, float* poses, int32_t max
     float* d_p = reinterpret_cast<float*>(s); s += al256(size_t(n) * nc * 4);
     float* d_e = reinterpret_cast<float*>(s); s += al256(n * 4);
     int64_t* d_off = reinterpret_cast<int64_t*>(s);
-    int32_t* d_plig = reinterpret_cast<int32_t*>(s + 16);
     VD_CUDA(cudaMemcpyAsync(d_p, poses, size_t(n) * nc * 4, cudaMemcpyHostToDevice, c.stream));
     const int64_t off = L.pool_offset;
     VD_CUDA(cudaMemcpyAsync(d_off, &off, 8, cudaMemcpyHostToDevice, c.stream));
-    VD_CUDA(cudaMemsetAsync(d_plig, 0, n * 4 > 0 ? 4 : 4, c.stream));
+    VD_CUDA(cudaMemsetAsync(c.d_counter + 4, 0, 8, c.stream));
     RefineParams rp{};
     rp.pool = c.d_pool;
     rp.lig_off = d_off;
@@ -1397,8 +1396,11 @@ vd_status vd_refine(vd_ctx* h, int32_t lig, int32_t n, float* poses, int32_t max
     VD_CUDA(cudaGetLastError());
     VD_CUDA(cudaMemcpyAsync(poses, d_p, size_t(n) * nc * 4, cudaMemcpyDeviceToHost, c.stream));
     VD_CUDA(cudaMemcpyAsync(e_out, d_e, n * 4, cudaMemcpyDeviceToHost, c.stream));
+    unsigned long long ev = 0;
+    VD_CUDA(cudaMemcpyAsync(&ev, c.d_counter + 4, 8, cudaMemcpyDeviceToHost, c.stream));
     VD_CUDA(cudaStreamSynchronize(c.stream));
     { const vd_status cs = take_device_checks("refinement kernel"); if (cs != VD_OK) return cs; }
+    c.stats.bfgs_evals += int64_t(ev);
     return VD_OK;
 }
 
