@@ -1,4 +1,5 @@
-"""vd_stats: what a call adds does not depend on what the context did before."""
+"""vd_stats: what a call adds does not depend on what the context did before, and
+the corner cells' time is the kernel's."""
 import pytest
 
 from conftest import has_gpu
@@ -45,3 +46,21 @@ def test_evaluation_counts(vd):
         n, (_, _, ev) = counted(lambda: ctx.local_opt(lig, poses, 5))
         assert n == ev
         assert counted(lambda: ctx.energy_grad(lig, poses))[0] == len(poses)
+
+
+def test_cell_time_is_the_kernels(vd):
+    """A build that allocates the cells against one that keeps them: the same kernel on the same sizes (1.1 GB written,
+    about 0.2 ms); the bound leaves half of that for clocks."""
+    from vdock import synth
+    ctx = vd.Context()
+    ctx.set_receptor(*synth.receptor(1000, 30.0, 1))
+    ctx.set_box([0.0, 0.0, 0.0], [12.0] * 3)
+    ctx.build_grids(synth.TYPES8)  # loads the kernels
+    ctx.set_box([0.0, 0.0, 0.0], [60.0] * 3)
+    ctx.build_grids(synth.TYPES8)
+    first = ctx.stats()["cells_ms"]
+    again = []
+    for _ in range(3):
+        ctx.build_grids(synth.TYPES8)
+        again.append(ctx.stats()["cells_ms"])
+    assert 0 < first <= 1.5 * max(again), (first, again)

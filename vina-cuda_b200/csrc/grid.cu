@@ -423,6 +423,9 @@ vd_status vd_build_grids(vd_ctx* h, const int32_t* types, int32_t n_types) {
     if (!c.d_maps && (st = dev_alloc(c, &c.d_maps, bytes_maps, "vd_build_grids: maps")) != VD_OK) return st;
     st = ensure_scratch(&c, bytes_atoms + bytes_start + bytes_lut);
     if (st != VD_OK) return st;
+    // allocated before the events below, which time the kernels
+    if (with_cells && !c.d_cells && (st = dev_alloc(c, &c.d_cells, bytes_cells, "vd_build_grids: corner cells")) != VD_OK)
+        return st;
     // atoms and cell starts in one upload
     char* s = static_cast<char*>(c.d_scratch);
     StagedAtom* d_atoms = reinterpret_cast<StagedAtom*>(s);
@@ -492,10 +495,6 @@ vd_status vd_build_grids(vd_ctx* h, const int32_t* types, int32_t n_types) {
     VD_CUDA(cudaEventRecord(c.ev1, c.stream));
     // corner cells of the new maps (cells_ms)
     if (with_cells) {
-        if (!c.d_cells && (st = dev_alloc(c, &c.d_cells, bytes_cells, "vd_build_grids: corner cells")) != VD_OK) {
-            VD_CUDA(cudaStreamSynchronize(c.stream));
-            return st;
-        }
         c.cell_stride = n_cells_map * 8;
         const dim3 cells((size_t(g.n[0] - 1) * (g.n[1] - 1) + 255) / 256, std::min((g.n[2] - 1 + kCellZ - 1) / kCellZ, 65535), nt);
         corner_cells_kernel<<<cells, 256, 0, c.stream>>>(c.d_maps, map_stride, c.d_cells, c.cell_stride, g.n[0], g.n[1],
