@@ -278,7 +278,8 @@ vd_status vd_rmsd_bounds(vd_ctx* ctx, int32_t lig_id, int32_t n_poses, const flo
                          float* lb_out, float* ub_out);
 
 /* ---- host helpers (no GPU work) --------------------------------------------- */
-/* Pair tables built by vd_set_scoring: fast[153][2051], smooth e / dor. */
+/* The current pair tables: fast[153][2051], smooth e / dor.  Tables of
+ * vd_set_scoring_device are built again on the GPU by this call. */
 vd_status vd_get_tables(vd_ctx* ctx, double* fast, double* smooth_e, double* smooth_dor);
 /* PDBQT ingestion (lib/parse_pdbqt.cpp, lib/model.cpp typing).  Returned
  * arrays are owned by the handle and live until vd_pdbqt_free. */

@@ -242,7 +242,9 @@ vd_status vd_get_stats(vd_ctx* h, vd_stats* out) {
 }
 
 // After new tables: maps built with the old weights are stale.
-static void scoring_changed(Ctx& c, double force_bound, bool on_device, std::chrono::steady_clock::time_point t0) {
+static void scoring_changed(Ctx& c, const double* weights, double force_bound, bool on_device,
+                            std::chrono::steady_clock::time_point t0) {
+    std::copy(weights, weights + 6, c.weights);
     c.scoring = true;
     c.fix_scale = pair_force_scale(force_bound);
     c.tables_on_device = on_device;
@@ -257,7 +259,6 @@ vd_status vd_set_scoring(vd_ctx* h, const double weights[6]) {
     Ctx& c = h->c;
     const auto t0 = std::chrono::steady_clock::now();
     VD_CUDA(cudaSetDevice(c.device));
-    std::memcpy(c.weights, weights, sizeof(c.weights));
     build_tables(weights, c.fast, c.se, c.sd);
     std::vector<float> f(size_t(kPairTypes) * kBins);
     std::vector<float4> s(size_t(kPairTypes) * kBins);
@@ -281,7 +282,7 @@ vd_status vd_set_scoring(vd_ctx* h, const double weights[6]) {
     VD_CUDA(cudaMemcpy(c.d_fastd, fd.data(), fd.size() * sizeof(double), cudaMemcpyHostToDevice));
     VD_CUDA(cudaMemcpy(c.d_fast, f.data(), f.size() * sizeof(float), cudaMemcpyHostToDevice));
     VD_CUDA(cudaMemcpy(c.d_smooth, s.data(), s.size() * sizeof(float4), cudaMemcpyHostToDevice));
-    scoring_changed(c, pair_force_bound(c.sd), false, t0);
+    scoring_changed(c, weights, pair_force_bound(c.sd), false, t0);
     return VD_OK;
 }
 
@@ -292,11 +293,10 @@ vd_status vd_set_scoring_device(vd_ctx* h, const double weights[6]) {
     Ctx& c = h->c;
     const auto t0 = std::chrono::steady_clock::now();
     VD_CUDA(cudaSetDevice(c.device));
-    std::memcpy(c.weights, weights, sizeof(c.weights));
     double bound = 0;
-    vd_status st = build_tables_device(c, bound);
+    vd_status st = build_tables_device(c, weights, bound);
     if (st != VD_OK) return st;
-    scoring_changed(c, bound, true, t0);
+    scoring_changed(c, weights, bound, true, t0);
     return VD_OK;
 }
 

@@ -276,10 +276,10 @@ void build_tables(const double w[6], std::vector<double>& fast, std::vector<doub
 double pair_force_bound(const std::vector<double>& sd);
 float pair_force_scale(double bound);
 float pair_force_scale(const std::vector<double>& sd);
-// Same tables built on the device from c.weights into the context's device
-// copies, and their largest pair force; the double tables stay there until
-// fetch_tables (any of its arrays may be null).
-vd_status build_tables_device(Ctx& c, double& force_bound);
+// Same tables built on the device into the context's device copies, and their
+// largest pair force; fetch_tables gives the double tables of c.weights as the
+// device builds them (any of its arrays may be null).
+vd_status build_tables_device(Ctx& c, const double w[6], double& force_bound);
 vd_status fetch_tables(Ctx& c, double* fast, double* se, double* sd);
 
 }  // namespace vd

@@ -11,8 +11,8 @@
 // only for vd_get_tables (7.5 MB: 1.6 of the 2.1 ms a weight set took).
 // This file is compiled without FMA contraction so the arithmetic rounds like
 // the host build; only exp() may differ from the host's, by an ulp.
+#include <algorithm>
 #include <cfloat>
-#include <chrono>
 
 #include "common.h"
 #include "xs_terms.h"
@@ -25,7 +25,7 @@ struct TableParams {
     double* fast;     // [kPairTypes][kN]
     double* se;
     double* sd;
-    float* fast_f;    // [kPairTypes][kBins]
+    float* fast_f;    // [kPairTypes][kBins]; null: the doubles above only
     double* fast_d;   // [kPairTypes][kBins]
     float4* smooth;   // [kPairTypes][kBins]
 };
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(256) tables_kernel(TableParams p) {
     p.se[o] = e_i;
     p.sd[o] = sd_i;
     p.fast[o] = fast_i;
-    if (i < kBins) {  // i + 2 <= kN - 1: the next entry's derivative is defined
+    if (p.fast_f && i < kBins) {  // i + 2 <= kN - 1: the next entry's derivative is defined
         const double sd_p = dor(i + 1, e_i, energy(i + 2));
         const size_t ob = size_t(tp) * kBins + i;
         p.fast_f[ob] = float(fast_i);
@@ -76,22 +76,15 @@ __global__ void __launch_bounds__(256) force_bound_kernel(const double* sd, unsi
 
 }  // namespace
 
-// Tables of c.weights into the device copies, the doubles into the scratch
-// (fast, se, sd in turn).
-static vd_status run_tables(Ctx& c, double*& doubles) {
-    const size_t n = size_t(kPairTypes) * kN, nb = size_t(kPairTypes) * kBins;
-    vd_status st = VD_OK;
-    if (!c.d_fast && (st = dev_alloc(c, &c.d_fast, nb * sizeof(float), "pair tables")) != VD_OK) return st;
-    if (!c.d_smooth && (st = dev_alloc(c, &c.d_smooth, nb * sizeof(float4), "pair tables")) != VD_OK) return st;
-    if (!c.d_fastd && (st = dev_alloc(c, &c.d_fastd, nb * sizeof(double), "pair tables")) != VD_OK) return st;
-    st = ensure_scratch(&c, 3 * n * sizeof(double));
-    if (st != VD_OK) return st;
+// Tables of w: the doubles (fast, se, sd in turn) to `doubles`; the kernels' copies too, where device is true.
+static vd_status run_tables(Ctx& c, const double* w, double* doubles, bool device) {
+    const size_t n = size_t(kPairTypes) * kN;
     TableParams p{};
-    for (int k = 0; k < 6; ++k) p.w[k] = c.weights[k];
-    doubles = p.fast = static_cast<double*>(c.d_scratch);
+    for (int k = 0; k < 6; ++k) p.w[k] = w[k];
+    p.fast = doubles;
     p.se = p.fast + n;
     p.sd = p.se + n;
-    p.fast_f = c.d_fast;
+    p.fast_f = device ? c.d_fast : nullptr;
     p.fast_d = c.d_fastd;
     p.smooth = c.d_smooth;
     tables_kernel<<<unsigned((n + 255) / 256), 256, 0, c.stream>>>(p);
@@ -99,12 +92,16 @@ static vd_status run_tables(Ctx& c, double*& doubles) {
     return VD_OK;
 }
 
-vd_status build_tables_device(Ctx& c, double& force_bound) {
+vd_status build_tables_device(Ctx& c, const double w[6], double& force_bound) {
     const size_t n = size_t(kPairTypes) * kN, nb = size_t(kPairTypes) * kBins;
-    double* d = nullptr;
-    vd_status st = settle_device_calls(c);
-    if (st == VD_OK) st = run_tables(c, d);
-    if (st != VD_OK) return st;
+    vd_status st = VD_OK;
+    if (!c.d_fast && (st = dev_alloc(c, &c.d_fast, nb * sizeof(float), "pair tables")) != VD_OK) return st;
+    if (!c.d_smooth && (st = dev_alloc(c, &c.d_smooth, nb * sizeof(float4), "pair tables")) != VD_OK) return st;
+    if (!c.d_fastd && (st = dev_alloc(c, &c.d_fastd, nb * sizeof(double), "pair tables")) != VD_OK) return st;
+    if ((st = ensure_scratch(&c, 3 * n * sizeof(double))) != VD_OK) return st;
+    if ((st = settle_device_calls(c)) != VD_OK) return st;
+    double* const d = static_cast<double*>(c.d_scratch);
+    if ((st = run_tables(c, w, d, true)) != VD_OK) return st;
     unsigned long long* const bound = reinterpret_cast<unsigned long long*>(c.d_counter + 16);
     VD_CUDA(cudaMemsetAsync(bound, 0, sizeof(*bound), c.stream));
     force_bound_kernel<<<unsigned((nb + 255) / 256), 256, 0, c.stream>>>(d + 2 * n, bound);
@@ -114,12 +111,28 @@ vd_status build_tables_device(Ctx& c, double& force_bound) {
     return VD_OK;
 }
 
+// Builds the doubles again (the scratch has had other uses since) and leaves
+// the kernels' copies alone.  Without room for 7.5 MB of scratch under the
+// context's cap they go straight to host memory.
 vd_status fetch_tables(Ctx& c, double* fast, double* se, double* sd) {
     const size_t n = size_t(kPairTypes) * kN;
-    double* d = nullptr;
-    const vd_status st = run_tables(c, d);  // the same values again: the scratch has had other uses since
-    if (st != VD_OK) return st;
     double* const out[3] = {fast, se, sd};
+    vd_status st = ensure_scratch(&c, 3 * n * sizeof(double));
+    if (st == VD_ERR_NOMEM) {
+        void* host = nullptr;
+        VD_CUDA(cudaHostAlloc(&host, 3 * n * sizeof(double), cudaHostAllocMapped));
+        double* const h = static_cast<double*>(host);
+        st = run_tables(c, c.weights, h, false);
+        const cudaError_t e = cudaStreamSynchronize(c.stream);
+        for (int k = 0; k < 3 && st == VD_OK && e == cudaSuccess; ++k)
+            if (out[k]) std::copy(h + k * n, h + (k + 1) * n, out[k]);
+        cudaFreeHost(host);
+        VD_CUDA(e);
+        return st;
+    }
+    if (st != VD_OK) return st;
+    double* const d = static_cast<double*>(c.d_scratch);
+    if ((st = run_tables(c, c.weights, d, false)) != VD_OK) return st;
     for (int k = 0; k < 3; ++k)
         if (out[k]) VD_CUDA(cudaMemcpyAsync(out[k], d + k * n, n * sizeof(double), cudaMemcpyDeviceToHost, c.stream));
     VD_CUDA(cudaStreamSynchronize(c.stream));
