@@ -91,8 +91,9 @@ typedef struct {
     int32_t  refine;          /* 1 = refine + rescore on the GPU (main.cpp:434)*/
     int32_t  launch_shape;    /* docking kernel shape: 0 = by the workload (4
                                  when its chains fill the GPU several times
-                                 over, 5 when the longest decide, otherwise
-                                 autotuned), 1/2/3/4/5 =
+                                 over, 5 when the longest decide or each takes
+                                 much shared memory, otherwise autotuned),
+                                 1/2/3/4/5 =
                                  64/48/40/80/128 registers per thread
                                  (8/10/12/6/4 blocks of 4 chains per SM; with
                                  few chains shape 5 runs a team of 4 warps

@@ -286,10 +286,25 @@ int dense_floats(int ntors) {
 //        2.4   1,500 chains (24 / 44)          3.36 / 11.7   -2.0 / -9.3   +29 / +39
 // Below kSaturated and above kTailBound the rule decides; between them the
 // autotuner runs both once and keeps the faster, since a wrong guess costs up
-// to 19 %.  Launches small enough for a team per chain (kTeamChains) take the
+// to 19 %.  The dense search: 24 / 44 atoms +7 to +9 % and +4 to +8 % below
+// kSaturated, -4 and -6 % at tail 1.7.
+// Chains of large ligands, those of the dense search above all, leave little
+// of the SM's memory for L1 at 24 per SM, or do not get 24.  By what 80
+// registers' resident blocks take of its 228 KB, change at 128 registers for
+// tails of 0.2 / 0.4 / 0.9 / 1.7:
+//   107 KB  60 atoms / 15 torsions           +2.2   +2.6   +2.9   -5.6 %
+//   126     72 / 18                          -0.1   +0.4    0.0   -5.0
+//   151     88 / 22                          -0.2   +1.1   -1.2   +3.8
+//   158     60 / 15 dense                    +2.7   +0.1   +1.6   -5.3
+//   170     66 / 16 dense                    -2.2   -0.9   -4.0   -5.8
+//   194     88 / 40                          -6.9   -6.7   -7.9   -7.9
+//   198     70 / 48                          -4.6   -5.7   -6.9   -4.5
+//   212     80 / 20 dense                    -7.3   -5.6   -7.1   -5.5
+//   205     88 / 40 dense (12 chains either way)  -0.3   -0.5   -2.4   -3.5
+// so above kCrowded of it they take 128 whatever the tail.  Launches small enough for a team per chain (kTeamChains) take the
 // team for 128 registers and explore all three.
 constexpr int kNarrowShape = 3;  // the 80-register shape
-constexpr double kSaturated = 0.5, kTailBound = 1.25;
+constexpr double kSaturated = 0.5, kTailBound = 1.25, kCrowded = 0.7;
 
 void dock_tune_report(Ctx& c, const DockBuffers& b, double ms, const unsigned long long* lig_evals) {
     if (!b.tuned) return;
@@ -430,10 +445,14 @@ vd_status prepare_dock(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     const size_t smem_team = (size_t(max_wf) + pair_team_floats(max_sp)) * sizeof(float);
     const bool few = items <= sms * kTeamChains && smem_team <= 227 * 1024 / kTeamChains;
     const double tail = work > 0 ? longest * kShapeBlocks[kNarrowShape] * wpb * sms / work : 0;
+    const size_t per_block = smem_warps + size_t(c.smem_reserved);
+    const size_t narrow_blocks = std::min<size_t>(kShapeBlocks[kNarrowShape], size_t(c.smem_sm) / per_block);
+    const bool crowded = double(narrow_blocks * per_block) > kCrowded * c.smem_sm ||
+                         narrow_blocks <= size_t(kShapeBlocks[kWideShape]);
     out.tune_key |= uint64_t(few) << 42;
     if (!out.tuned) {
         out.shape = sp.launch_shape - 1;
-    } else if (few ? !persistent : tail > kTailBound) {
+    } else if (few ? !persistent : (tail > kTailBound || crowded)) {
         out.shape = kWideShape;
     } else if (!few && tail < kSaturated) {
         out.shape = kNarrowShape;
