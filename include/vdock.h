@@ -142,8 +142,11 @@ typedef struct {
     int64_t device_bytes;        /* device memory the context holds for maps, tables,
                                     ligands, receptor cells and scratch           */
     double  pair_force_scale;    /* fixed-point units per kcal/mol/A in which the
-                                    kernels sum intra-pair forces (a power of two
-                                    set from the current tables; 2^19 by default) */
+                                    search, local optimisation and refinement sum
+                                    intra-pair forces (a power of two set from the
+                                    current tables; 2^19 by default).  vd_energy*
+                                    take 128 / (most partners of an atom, rounded
+                                    up to a power of two) times as many          */
     double  cells_ms;            /* last vd_build_grids: time to lay the maps out as
                                     32-byte trilinear corner cells for the
                                     evaluation kernels (0 when the box is too
@@ -204,6 +207,10 @@ vd_status vd_ligand_info(vd_ctx* ctx, int32_t lig_id, int32_t* n_heavy, int32_t*
 vd_status vd_clear_ligands(vd_ctx* ctx);
 
 /* ---- pose batches: forward energy and adjoint (model.cpp:1324-1333) ------- */
+/* The number of poses of a call picks its kernel, and these add a pose's terms
+ * in different orders: energies and gradients repeat bit for bit for the same
+ * call, and a pose's may differ by the rounding of its FP32 sums between calls
+ * with other numbers of poses.  Coordinates (vd_pose_coords) do not. */
 vd_status vd_energy(vd_ctx* ctx, int32_t lig_id, int32_t n_poses, const float* poses,
                     const vd_eval_params* p, float* e_out);
 vd_status vd_energy_grad(vd_ctx* ctx, int32_t lig_id, int32_t n_poses, const float* poses,

@@ -7,12 +7,13 @@
 //      (rotation about a body-fixed axis; equals tree.h:282-292)
 //   3. lanes = atoms: coordinates, trilinear grid term (grid.cpp:50-160)
 //   4. intra pair term (model.cpp:1241-1256), two pairs per lane per
-//      iteration.  The search (pair_atomics) walks the ligand's search
-//      schedule: rounds of one pair per lane in which few lanes share an
-//      atom, both atoms' forces added with shared-memory atomics.  The pose
-//      kernels walk per-lane segments of the pair list sorted by second atom,
-//      the second atom's force summed in registers while it repeats, the
-//      first atom's added with an atomic.  Pair forces are summed in 32-bit
+//      iteration.  The search (pair_atomics), local optimisation and teams
+//      walk the ligand's search schedule: rounds of one pair per lane in which
+//      few lanes share an atom, both atoms' forces added with shared-memory
+//      atomics.  A pose batch on one warp per pose walks per-lane segments of
+//      the pair list sorted by second atom, the second atom's force summed in
+//      registers while it repeats, the first atom's added with an atomic
+//      (pose tiles likewise, with a kernel of their own).  Pair forces are summed in 32-bit
 //      fixed point (EvalParams::fix units per kcal/mol/A, set from the tables
 //      so that no atom's sum can overflow): integer sums are exact, so the
 //      result does not depend on the order in which the atomics land, and
@@ -28,7 +29,9 @@
 //        tree.h:169-178, 341-348, 373-422)
 //   8. warp butterfly sum of the energy (deterministic).
 // The per-body and subtree sums run in a fixed order, so every result is
-// reproducible run to run and across launch shapes.
+// reproducible run to run, and the docking search's across launch shapes, with
+// and without teams.  The kernels for pose batches add in other orders, which
+// depend on the number of poses (pose.cu).
 #pragma once
 
 #include "checks.cuh"
