@@ -1363,16 +1363,18 @@ vd_status vd_refine(vd_ctx* h, int32_t lig, int32_t n, float* poses, int32_t max
     if (st != VD_OK) return st;
     const HostLigand& L = c.ligs[lig];
     const int nc = 7 + L.h.ntors;
-    st = ensure_scratch(&c, al256(size_t(n) * nc * 4) + al256(n * 4) + al256(n * 4) + 256);
+    // poses, then the blob's offset and a count of evaluations that starts at
+    // zero (one upload), then the energies (one download with the count)
+    struct { int64_t off; unsigned long long evals; } head = {L.pool_offset, 0};
+    st = ensure_scratch(&c, al256(size_t(n) * nc * 4) + sizeof(head) + size_t(n) * 4);
     if (st != VD_OK) return st;
-    char* s = static_cast<char*>(c.d_scratch);
-    float* d_p = reinterpret_cast<float*>(s); s += al256(size_t(n) * nc * 4);
-    float* d_e = reinterpret_cast<float*>(s); s += al256(n * 4);
-    int64_t* d_off = reinterpret_cast<int64_t*>(s);
+    float* d_p = static_cast<float*>(c.d_scratch);
+    char* d_head = static_cast<char*>(c.d_scratch) + al256(size_t(n) * nc * 4);
+    int64_t* d_off = reinterpret_cast<int64_t*>(d_head);
+    unsigned long long* d_evals = reinterpret_cast<unsigned long long*>(d_head + sizeof(int64_t));
+    float* d_e = reinterpret_cast<float*>(d_head + sizeof(head));
     VD_CUDA(cudaMemcpyAsync(d_p, poses, size_t(n) * nc * 4, cudaMemcpyHostToDevice, c.stream));
-    const int64_t off = L.pool_offset;
-    VD_CUDA(cudaMemcpyAsync(d_off, &off, 8, cudaMemcpyHostToDevice, c.stream));
-    VD_CUDA(cudaMemsetAsync(c.d_counter + 4, 0, 8, c.stream));
+    VD_CUDA(cudaMemcpyAsync(d_head, &head, sizeof(head), cudaMemcpyHostToDevice, c.stream));
     RefineParams rp{};
     rp.pool = c.d_pool;
     rp.lig_off = d_off;
@@ -1387,7 +1389,7 @@ vd_status vd_refine(vd_ctx* h, int32_t lig, int32_t n, float* poses, int32_t max
     rp.smooth = c.d_smooth;
     rp.fix = c.fix_scale;
     rp.inv_fix = 1.f / c.fix_scale;
-    rp.evals = reinterpret_cast<unsigned long long*>(c.d_counter + 4);
+    rp.evals = d_evals;
     rp.skip_invalid = 0;
     const size_t smem_r = size_t(refine_floats(L)) * 4;
     VD_CHECK(smem_r <= 227 * 1024, VD_ERR_CAPACITY, "refine kernel shared memory exceeds 227 KB");
@@ -1395,12 +1397,13 @@ vd_status vd_refine(vd_ctx* h, int32_t lig, int32_t n, float* poses, int32_t max
     refine_kernel<<<n, 32 * kRefineWarps, smem_r, c.stream>>>(rp);
     VD_CUDA(cudaGetLastError());
     VD_CUDA(cudaMemcpyAsync(poses, d_p, size_t(n) * nc * 4, cudaMemcpyDeviceToHost, c.stream));
-    VD_CUDA(cudaMemcpyAsync(e_out, d_e, n * 4, cudaMemcpyDeviceToHost, c.stream));
-    unsigned long long ev = 0;
-    VD_CUDA(cudaMemcpyAsync(&ev, c.d_counter + 4, 8, cudaMemcpyDeviceToHost, c.stream));
+    std::vector<char> tail(sizeof(head.evals) + size_t(n) * 4);
+    VD_CUDA(cudaMemcpyAsync(tail.data(), d_evals, tail.size(), cudaMemcpyDeviceToHost, c.stream));
     VD_CUDA(cudaStreamSynchronize(c.stream));
     { const vd_status cs = take_device_checks("refinement kernel"); if (cs != VD_OK) return cs; }
-    c.stats.bfgs_evals += int64_t(ev);
+    std::memcpy(&head.evals, tail.data(), sizeof(head.evals));
+    std::memcpy(e_out, tail.data() + sizeof(head.evals), size_t(n) * 4);
+    c.stats.bfgs_evals += int64_t(head.evals);
     return VD_OK;
 }
 
