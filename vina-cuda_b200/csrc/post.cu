@@ -33,19 +33,20 @@ struct RecView {
     const double4* recd;        // same in double
     const int32_t* cell_start;  // [cells+1]
     const int32_t* cell_list;   // atom indices per cell
-    float init[3], per[3];      // szv_grid cell geometry: origin, cells per A
+    double init[3], per[3];     // szv_grid cell geometry: origin, cells per A
     int32_t dim[3];
     double gb[3], ge[3];        // box (non_cache gd)
     float gbf[3], gef[3];       // the same in FP32
 };
 
-// szv_grid.cpp:92-107 (fl_to_sz) in FP32: a point within rounding of a cell
-// face may take the neighbour cell, whose list reaches a little further
-// than the cutoff (ensure_receptor_cells) and so holds the same atoms in
-// reach, in the same order.  Optimisers do reach poses that are not finite:
-// the conversion saturates and takes a NaN to 0, so those get a cell too.
-__device__ __forceinline__ int cell_of(const RecView& R, float x, float y, float z) {
-    const float c[3] = {x, y, z};
+// szv_grid.cpp:92-107 (fl_to_sz), with the cells per A in place of a division:
+// a point within rounding of a cell face may take the neighbour cell, whose
+// list reaches a little further than the cutoff (ensure_receptor_cells) and so
+// holds the same atoms in reach, in the same order.  Optimisers do reach poses
+// that are not finite: the conversion saturates and takes a NaN to the lowest
+// integer, so clamping gives those a cell too.
+__device__ __forceinline__ int cell_of(const RecView& R, double x, double y, double z) {
+    const double c[3] = {x, y, z};
     int idx[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) idx[d] = max(0, min(int((c[d] - R.init[d]) * R.per[d]), R.dim[d] - 1));
@@ -687,7 +688,7 @@ __device__ __forceinline__ double inter_fast(const LigView& L, const RecView& R,
                 if (a[j][d] < R.gb[d]) { oob[j] += fabs(a[j][d] - R.gb[d]); a[j][d] = R.gb[d]; }
                 else if (a[j][d] > R.ge[d]) { oob[j] += fabs(a[j][d] - R.ge[d]); a[j][d] = R.ge[d]; }
             }
-            const int ce = cell_of(R, float(a[j][0]), float(a[j][1]), float(a[j][2]));
+            const int ce = cell_of(R, a[j][0], a[j][1], a[j][2]);
             q0[j] = __ldg(&R.cell_start[ce]);
             q1[j] = __ldg(&R.cell_start[ce + 1]);
             longest = max(longest, q1[j] - q0[j]);
@@ -949,11 +950,11 @@ vd_status ensure_receptor_cells(Ctx* c) {
     for (int i = 0; i < n_rec; ++i)
         if (c->rec_xs[i] >= 0 && brick(init, end, &c->rec_xyz[3 * size_t(i)]) < kCutoff2) rel.push_back(i);
     // A cell's list reaches a little further than the cutoff, so that a point
-    // that FP32 rounding puts into the cell next to its own (cell_of) still
-    // finds every atom within 8 A there.
+    // that rounding puts into the cell next to its own (cell_of) still finds
+    // every atom within 8 A there.
     double far = 0;
     for (int d = 0; d < 3; ++d) far = std::max({far, std::fabs(init[d]), std::fabs(end[d])});
-    const double margin = 1e-3 + 1e-6 * far, reach2 = (8.0 + margin) * (8.0 + margin);
+    const double margin = 1e-6 + 1e-12 * far, reach2 = (8.0 + margin) * (8.0 + margin);
     const int ncell = dim[0] * dim[1] * dim[2];
     std::vector<std::vector<int>> cells(ncell);
     auto coord = [&](int d, int i) { return init[d] + range[d] * i / dim[d]; };
@@ -1024,8 +1025,8 @@ RecView rec_view(const Ctx& c) {
     R.cell_start = c.d_cell_start;
     R.cell_list = c.d_cell_list;
     for (int d = 0; d < 3; ++d) {
-        R.init[d] = float(c.cell_init[d]);
-        R.per[d] = float(c.cell_dim[d] / c.cell_range[d]);
+        R.init[d] = c.cell_init[d];
+        R.per[d] = c.cell_dim[d] / c.cell_range[d];
         R.dim[d] = c.cell_dim[d];
         R.gbf[d] = float(c.geom.begin[d]);
         R.gef[d] = float(c.geom.end[d]);
