@@ -172,13 +172,74 @@ __device__ __forceinline__ void store_frame(float4 q, float3 o, float* nd) {
     r[2] = make_float4(2.f * (-ac + bd), 2.f * (ab + cd), aa - bb - cc + dd, o.z);
 }
 
+// The same with the fused multiply-adds written out, for the pose batches: each
+// of their kernels places an atom at the same coordinates to the bit.  The
+// trilinear gradient jumps at cell faces and the penalty's at the box, so a
+// coordinate an ulp off would now and then give another gradient.  (The search
+// leaves the choice to the compiler, which makes the same one today: written
+// out there, it spills 4 bytes at 80 registers and a 64-ligand screen takes
+// 777 ms in place of 722.)
+__device__ __forceinline__ float dot2(float a, float b, float c, float d) {  // a b + c d
+    return __fmaf_rn(a, b, __fmul_rn(c, d));
+}
+// a_j P of the walk up the ancestors
+__device__ __forceinline__ float4 walk_qmul(float4 a, float4 b) {
+    return make_float4(__fmaf_rn(-a.w, b.w, __fmaf_rn(-a.z, b.z, dot2(a.x, b.x, -a.y, b.y))),
+                       __fmaf_rn(-a.w, b.z, __fmaf_rn(a.z, b.w, dot2(a.x, b.y, a.y, b.x))),
+                       __fmaf_rn(a.w, b.y, __fmaf_rn(a.z, b.x, dot2(a.x, b.z, -a.y, b.w))),
+                       __fmaf_rn(a.w, b.x, __fmaf_rn(-a.z, b.y, dot2(a.x, b.w, a.y, b.z))));
+}
+// q_root P
+__device__ __forceinline__ float4 root_qmul(float4 a, float4 b) {
+    return make_float4(__fmaf_rn(-a.w, b.w, __fmaf_rn(-a.z, b.z, dot2(a.x, b.x, -a.y, b.y))),
+                       __fmaf_rn(-a.w, b.z, __fmaf_rn(a.z, b.w, dot2(a.y, b.x, a.x, b.y))),
+                       __fmaf_rn(a.w, b.y, __fmaf_rn(a.z, b.x, dot2(a.x, b.z, -a.y, b.w))),
+                       __fmaf_rn(a.w, b.x, __fmaf_rn(-a.z, b.y, dot2(a.y, b.z, a.x, b.w))));
+}
+__device__ __forceinline__ float3 body_qrot(float4 q, float3 v) {
+    const float tx = __fmaf_rn(q.x, v.x, dot2(q.z, v.z, -q.w, v.y));
+    const float ty = __fmaf_rn(q.x, v.y, dot2(q.w, v.x, -q.y, v.z));
+    const float tz = __fmaf_rn(q.x, v.z, dot2(q.y, v.y, -q.z, v.x));
+    return make_float3(__fmaf_rn(2.f, dot2(q.z, tz, -q.w, ty), v.x), __fmaf_rn(2.f, dot2(q.w, tx, -q.y, tz), v.y),
+                       __fmaf_rn(2.f, dot2(q.y, ty, -q.z, tx), v.z));
+}
+// Frame of a body: rotation matrix of its quaternion, normalised here, and origin.
+struct BodyFrame {
+    float r[3][3], o[3];
+    __device__ __forceinline__ BodyFrame(float4 q, float3 origin) : o{origin.x, origin.y, origin.z} {
+        const float inv = rsqrtf(__fmaf_rn(q.w, q.w, __fmaf_rn(q.z, q.z, dot2(q.x, q.x, q.y, q.y))));
+        const float a = __fmul_rn(q.x, inv), b = __fmul_rn(q.y, inv), c = __fmul_rn(q.z, inv), d = __fmul_rn(q.w, inv);
+        r[0][0] = __fmaf_rn(-d, d, __fmaf_rn(-c, c, dot2(a, a, b, b)));
+        r[0][1] = 2.f * dot2(b, c, -a, d);
+        r[0][2] = 2.f * dot2(a, c, b, d);
+        r[1][0] = 2.f * dot2(b, c, a, d);
+        r[1][1] = __fmaf_rn(-d, d, __fmaf_rn(c, c, dot2(a, a, -b, b)));
+        r[1][2] = 2.f * dot2(c, d, -a, b);
+        r[2][0] = 2.f * dot2(-a, c, b, d);
+        r[2][1] = 2.f * dot2(c, d, a, b);
+        r[2][2] = __fmaf_rn(d, d, __fmaf_rn(-c, c, dot2(a, a, -b, b)));
+    }
+    __device__ __forceinline__ float direction(int i, float x, float y, float z) const {
+        return __fmaf_rn(r[i][2], z, dot2(r[i][0], x, r[i][1], y));
+    }
+    __device__ __forceinline__ float point(int i, float4 a) const { return __fadd_rn(o[i], direction(i, a.x, a.y, a.z)); }
+    // three 128-bit rows [R(i,0) R(i,1) R(i,2) o_i]
+    __device__ __forceinline__ void store(float* nd) const {
+        float4* const row = reinterpret_cast<float4*>(nd);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) row[i] = make_float4(r[i][0], r[i][1], r[i][2], o[i]);
+    }
+};
+
 // Node words as 128-bit loads (NodeRec: {origin, parent}, {axis, first
 // atom}, {atom end, subtree end, depth, subtree atom end}).
 __device__ __forceinline__ float4 node_word(const NodeRec* nodes, int k, int w) {
     return __ldg(reinterpret_cast<const float4*>(nodes + k) + w);
 }
 
-// Phases 1-2: rigid-body frames from the pose in m.x.
+// Phases 1-2: rigid-body frames from the pose in m.x.  pinned: with the fused
+// multiply-adds written out (above), here and below.
+template <bool pinned = false>
 __device__ __forceinline__ void frames(const LigView& L, const WarpMem& m, int lane) {
     // 1: local rotation of each body about its axis (angle_to_quaternion)
     for (int k = lane; k < L.nn; k += 32) {
@@ -209,11 +270,23 @@ __device__ __forceinline__ void frames(const LigView& L, const WarpMem& m, int l
             while (j > 0) {
                 const float4 aj = *reinterpret_cast<const float4*>(m.nd + kNodeF * j + kNdAA);
                 const float4 oj = node_word(L.nodes, j, 0);
-                const float3 r = qrot(aj, w);
-                w = make_float3(oj.x + r.x, oj.y + r.y, oj.z + r.z);
-                P = qmul(aj, P);
+                if constexpr (pinned) {
+                    const float3 r = body_qrot(aj, w);
+                    w = make_float3(__fadd_rn(oj.x, r.x), __fadd_rn(oj.y, r.y), __fadd_rn(oj.z, r.z));
+                    P = walk_qmul(aj, P);
+                } else {
+                    const float3 r = qrot(aj, w);
+                    w = make_float3(oj.x + r.x, oj.y + r.y, oj.z + r.z);
+                    P = qmul(aj, P);
+                }
                 j = VD_DCLAMP(__float_as_int(oj.w), 0, j - 1, kChkParent);
             }
+        }
+        if constexpr (pinned) {
+            const float3 ro = body_qrot(qr, w);
+            const float3 o = make_float3(__fadd_rn(orr.x, ro.x), __fadd_rn(orr.y, ro.y), __fadd_rn(orr.z, ro.z));
+            BodyFrame(root_qmul(qr, P), o).store(m.nd + kNodeF * k);
+            continue;
         }
         float4 q = qmul(qr, P);
         const float inv = rsqrtf(q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
@@ -225,18 +298,24 @@ __device__ __forceinline__ void frames(const LigView& L, const WarpMem& m, int l
 }
 
 // Phase 3a for one heavy atom: its coordinates from its body's frame.
+template <bool pinned = false>
 __device__ __forceinline__ float4 atom_position(const LigView& L, const WarpMem& m, float4 a) {
     const int k = VD_DCLAMP((__float_as_int(a.w) >> 8) & 0xff, 0, L.nn - 1, kChkAtomBody);
     const float4* nd = reinterpret_cast<const float4*>(m.nd + kNodeF * k);
     const float4 r0 = nd[0], r1 = nd[1], r2 = nd[2];
+    if constexpr (pinned) {
+        const auto point = [&](float4 r) { return __fadd_rn(r.w, __fmaf_rn(r.z, a.z, dot2(r.x, a.x, r.y, a.y))); };
+        return make_float4(point(r0), point(r1), point(r2), 0.f);
+    }
     return make_float4(r0.w + (r0.x * a.x + r0.y * a.y + r0.z * a.z), r1.w + (r1.x * a.x + r1.y * a.y + r1.z * a.z),
                        r2.w + (r2.x * a.x + r2.y * a.y + r2.z * a.z), 0.f);
 }
 
 // Phases 1-3a: rigid-body frames and heavy-atom coordinates from the pose in m.x.
+template <bool pinned = false>
 __device__ __forceinline__ void kinematics(const LigView& L, const WarpMem& m, int lane) {
-    frames(L, m, lane);
-    for (int i = lane; i < L.na; i += 32) m.c[i] = atom_position(L, m, __ldg(&L.atoms[i]));
+    frames<pinned>(L, m, lane);
+    for (int i = lane; i < L.na; i += 32) m.c[i] = atom_position<pinned>(L, m, __ldg(&L.atoms[i]));
     __syncwarp();
 }
 
@@ -577,16 +656,16 @@ __device__ __forceinline__ float pair_rounds(const LigView& L, const WarpMem& m,
 // skipped and m.g is left as it was.  The line searches pass a test that
 // holds exactly when the trial's gradient will not be read (a failed Armijo
 // test that is not the search's last trial).
-template <bool want_grad, bool pair_atomics = false, class Inter, class Skip = NoSkip>
+template <bool want_grad, bool pair_atomics = false, bool pinned = false, class Inter, class Skip = NoSkip>
 __device__ inline float eval_pose_t(const LigView& L, const WarpMem& m, const Inter& inter, const float4* smooth,
                              float v_intra, float fix, float inv_fix, int lane, const Skip& skip = Skip()) {
-    frames(L, m, lane);
+    frames<pinned>(L, m, lane);
     float e = 0.f;
     // 3: per atom its coordinates (kept for the pair phase) and the grid
     // term, whose gradient seeds the atom's force
     for (int i = lane; i < L.na; i += 32) {
         const float4 a = __ldg(&L.atoms[i]);
-        const float4 ci = atom_position(L, m, a);
+        const float4 ci = atom_position<pinned>(L, m, a);
         m.c[i] = ci;
         const int t = __float_as_int(a.w) & 0xff;
         float gx, gy, gz;
@@ -710,14 +789,6 @@ __device__ inline float eval_pose_t(const LigView& L, const WarpMem& m, const In
     return e;
 }
 
-template <bool want_grad, bool pair_atomics = false, class Skip = NoSkip>
-__device__ __forceinline__ float eval_pose(const LigView& L, const WarpMem& m, const MapView& G,
-                                           const float4* smooth, const EvalParams ep, int lane,
-                                           const Skip& skip = Skip()) {
-    const GridInter gi{&G, ep.v_inter, ep.slope};
-    return eval_pose_t<want_grad, pair_atomics>(L, m, gi, smooth, ep.v_intra, ep.fix, ep.inv_fix, lane, skip);
-}
-
 // ---------------------------------------------------------------- teams
 // A team of `warps` warps evaluates one pose: the first places the atoms,
 // looks up the grid and runs everything else; the others compute the intra
@@ -748,14 +819,14 @@ __device__ __forceinline__ PairTeam pair_team(float* p) {
 }
 
 // Evaluation by the team's first warp (the search's form: gradient wanted).
-template <int warps, class Inter, class Skip>
+template <int warps, bool pinned = false, class Inter, class Skip>
 __device__ inline float eval_pose_team(const LigView& L, const WarpMem& m, const Inter& inter, float inv_fix, int lane,
                                        const PairTeam& tm, const Skip& skip) {
-    frames(L, m, lane);
+    frames<pinned>(L, m, lane);
     int* const q = reinterpret_cast<int*>(m.ns);
     const int a4 = pad4(L.na);
     for (int i = lane; i < L.na; i += 32) {
-        m.c[i] = atom_position(L, m, __ldg(&L.atoms[i]));
+        m.c[i] = atom_position<pinned>(L, m, __ldg(&L.atoms[i]));
         q[i] = 0; q[a4 + i] = 0; q[2 * a4 + i] = 0;
     }
     __syncwarp();

@@ -47,15 +47,14 @@ __global__ void __launch_bounds__(32 * kPoseWarps, kPoseBlocks) pose_kernel(Pose
         const float* src = p.poses + size_t(pose) * nc;
         for (int i = lane; i < nc; i += 32) m.x[i] = src[i];
         __syncwarp();
-        if (mode == 0) {
-            const float e = eval_pose<false>(L, m, p.G, p.smooth, p.ep, lane);
+        if (mode != 2) {
+            const GridInter gi{&p.G, p.ep.v_inter, p.ep.slope};
+            const float e = eval_pose_t<mode == 1, false, true>(L, m, gi, p.smooth, p.ep.v_intra, p.ep.fix, p.ep.inv_fix, lane);
             if (lane == 0) p.e_out[pose] = e;
-        } else if (mode == 1) {
-            const float e = eval_pose<true>(L, m, p.G, p.smooth, p.ep, lane);
-            if (lane == 0) p.e_out[pose] = e;
-            for (int i = lane; i < n; i += 32) p.g_out[size_t(pose) * n + i] = m.g[i];
+            if (mode == 1)
+                for (int i = lane; i < n; i += 32) p.g_out[size_t(pose) * n + i] = m.g[i];
         } else {
-            kinematics(L, m, lane);
+            kinematics<true>(L, m, lane);
             float* dst = p.xyz_out + size_t(pose) * 3 * L.na;
             for (int i = lane; i < L.na; i += 32) {
                 dst[3 * i] = m.c[i].x;
@@ -96,7 +95,7 @@ __global__ void __launch_bounds__(32 * kPoseTeam, kTeamPoses) pose_team_kernel(P
     __syncwarp();
     const GridInter gi{&p.G, p.ep.v_inter, p.ep.slope};
     const float thr = mode == 0 ? -INFINITY : INFINITY;  // energy only: no adjoint
-    const float e = eval_pose_team<kPoseTeam>(L, m, gi, p.ep.inv_fix, lane, tm, SkipAbove{thr});
+    const float e = eval_pose_team<kPoseTeam, true>(L, m, gi, p.ep.inv_fix, lane, tm, SkipAbove{thr});
     if (lane == 0) {
         p.e_out[pose] = e;
         *tm.work = 0;
@@ -139,58 +138,6 @@ __host__ __device__ inline int tile_rows(int mode, int na, int nn, int nt, int w
 }
 // Before them: the pairs as 32-bit words, an even number.
 __host__ __device__ inline int tile_words(int mode, int np) { return mode == 2 ? 0 : pad4(np); }
-
-// Kinematics of the tile kernel.  Its coordinates equal frames() and
-// atom_position() bit for bit: the trilinear gradient jumps at cell faces and
-// the penalty's at the box, so a coordinate an ulp off would now and then give
-// another gradient than the other kernels do.  Where a sum of two products
-// leaves the compiler the choice of which one to fuse, the choice it makes
-// there is spelled out here (dot2: the first one).
-__device__ __forceinline__ float dot2(float a, float b, float c, float d) {  // a b + c d
-    return __fmaf_rn(a, b, __fmul_rn(c, d));
-}
-// a_j P of the walk up the ancestors
-__device__ __forceinline__ float4 walk_qmul(float4 a, float4 b) {
-    return make_float4(__fmaf_rn(-a.w, b.w, __fmaf_rn(-a.z, b.z, dot2(a.x, b.x, -a.y, b.y))),
-                       __fmaf_rn(-a.w, b.z, __fmaf_rn(a.z, b.w, dot2(a.x, b.y, a.y, b.x))),
-                       __fmaf_rn(a.w, b.y, __fmaf_rn(a.z, b.x, dot2(a.x, b.z, -a.y, b.w))),
-                       __fmaf_rn(a.w, b.x, __fmaf_rn(-a.z, b.y, dot2(a.x, b.w, a.y, b.z))));
-}
-// q_root P
-__device__ __forceinline__ float4 root_qmul(float4 a, float4 b) {
-    return make_float4(__fmaf_rn(-a.w, b.w, __fmaf_rn(-a.z, b.z, dot2(a.x, b.x, -a.y, b.y))),
-                       __fmaf_rn(-a.w, b.z, __fmaf_rn(a.z, b.w, dot2(a.y, b.x, a.x, b.y))),
-                       __fmaf_rn(a.w, b.y, __fmaf_rn(a.z, b.x, dot2(a.x, b.z, -a.y, b.w))),
-                       __fmaf_rn(a.w, b.x, __fmaf_rn(-a.z, b.y, dot2(a.y, b.z, a.x, b.w))));
-}
-__device__ __forceinline__ float3 tile_qrot(float4 q, float3 v) {
-    const float tx = __fmaf_rn(q.x, v.x, dot2(q.z, v.z, -q.w, v.y));
-    const float ty = __fmaf_rn(q.x, v.y, dot2(q.w, v.x, -q.y, v.z));
-    const float tz = __fmaf_rn(q.x, v.z, dot2(q.y, v.y, -q.z, v.x));
-    return make_float3(__fmaf_rn(2.f, dot2(q.z, tz, -q.w, ty), v.x), __fmaf_rn(2.f, dot2(q.w, tx, -q.y, tz), v.y),
-                       __fmaf_rn(2.f, dot2(q.y, ty, -q.z, tx), v.z));
-}
-// Rotation matrix rows and origin of a unit quaternion's frame
-struct TileFrame {
-    float r[3][3], o[3];
-    __device__ __forceinline__ TileFrame(float4 q, float3 origin) : o{origin.x, origin.y, origin.z} {
-        const float inv = rsqrtf(__fmaf_rn(q.w, q.w, __fmaf_rn(q.z, q.z, dot2(q.x, q.x, q.y, q.y))));
-        const float a = __fmul_rn(q.x, inv), b = __fmul_rn(q.y, inv), c = __fmul_rn(q.z, inv), d = __fmul_rn(q.w, inv);
-        r[0][0] = __fmaf_rn(-d, d, __fmaf_rn(-c, c, dot2(a, a, b, b)));
-        r[0][1] = 2.f * dot2(b, c, -a, d);
-        r[0][2] = 2.f * dot2(a, c, b, d);
-        r[1][0] = 2.f * dot2(b, c, a, d);
-        r[1][1] = __fmaf_rn(-d, d, __fmaf_rn(c, c, dot2(a, a, -b, b)));
-        r[1][2] = 2.f * dot2(c, d, -a, b);
-        r[2][0] = 2.f * dot2(-a, c, b, d);
-        r[2][1] = 2.f * dot2(c, d, a, b);
-        r[2][2] = __fmaf_rn(d, d, __fmaf_rn(-c, c, dot2(a, a, -b, b)));
-    }
-    __device__ __forceinline__ float direction(int i, float x, float y, float z) const {
-        return __fmaf_rn(r[i][2], z, dot2(r[i][0], x, r[i][1], y));
-    }
-    __device__ __forceinline__ float point(int i, float4 a) const { return __fadd_rn(o[i], direction(i, a.x, a.y, a.z)); }
-};
 
 template <int mode, int PL>
 __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
@@ -247,15 +194,15 @@ __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
             while (j > 0) {
                 const float4 aj = rotation(j);
                 const float4 oj = node_word(L.nodes, j, 0);
-                const float3 r = tile_qrot(aj, w);
+                const float3 r = body_qrot(aj, w);
                 w = make_float3(__fadd_rn(oj.x, r.x), __fadd_rn(oj.y, r.y), __fadd_rn(oj.z, r.z));
                 P = walk_qmul(aj, P);
                 j = VD_DCLAMP(__float_as_int(oj.w), 0, j - 1, kChkParent);
             }
         }
         const float4 qr = make_float4(X[3 * PL + T.p], X[4 * PL + T.p], X[5 * PL + T.p], X[6 * PL + T.p]);
-        const float3 ro = tile_qrot(qr, w);
-        const TileFrame f(root_qmul(qr, P), make_float3(__fadd_rn(X[T.p], ro.x), __fadd_rn(X[PL + T.p], ro.y),
+        const float3 ro = body_qrot(qr, w);
+        const BodyFrame f(root_qmul(qr, P), make_float3(__fadd_rn(X[T.p], ro.x), __fadd_rn(X[PL + T.p], ro.y),
                                                         __fadd_rn(X[2 * PL + T.p], ro.z)));
         const float4 w1 = node_word(L.nodes, k, 1);
         const int i1 = __float_as_int(node_word(L.nodes, k, 2).x);
