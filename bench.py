@@ -50,7 +50,7 @@ def args_():
     a.add_argument("--no-cpu-baseline", action="store_true")
     a.add_argument("--cpu-ligands", type=int, default=3, help="whole ligands per CPU sample step")
     a.add_argument("--no-configs", action="store_true", help="skip the plain / adjoint / uneven-batch lines")
-    a.add_argument("--launch-shape", type=int, default=0, help="docking kernel shape (0 = autotuned, 1-3 pinned)")
+    a.add_argument("--launch-shape", type=int, default=0, help="docking kernel shape (0 = by the workload, 1-5 pinned)")
     a.add_argument("--configs", default="plain,adjoint,uneven", help="secondary lines to run (comma list)")
     a.add_argument("--only-configs", action="store_true", help="skip the headline; print the secondary lines")
     return a.parse_args()

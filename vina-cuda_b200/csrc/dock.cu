@@ -68,10 +68,9 @@ __device__ __forceinline__ int find_ligand(const int32_t* prefix, int n, int ite
 }
 
 // MINB: 4-warp blocks per SM the register budget targets (8/10/12/6/4 ->
-// 64/48/40/80/128 registers per thread); the autotuner picks one per
-// workload.  The small budgets keep more chains resident for large batches;
-// the large ones drop the register spills (ptxas: 84 bytes of spill stores
-// at 64, none at 128), which pays when a launch has few chains per SM.
+// 64/48/40/80/128 registers per thread); kTailBound below says which a launch
+// takes.  The small budgets keep more chains resident; the large ones drop the
+// register spills (ptxas: 94 bytes of spill stores at 64, none at 80 and 128).
 // Per-warp shared memory: the evaluation's arrays, then the poses xp, xo,
 // xt, xb (pad4(7 + ntors) floats each), then kChainWords chain scalars,
 // then (dense BFGS) the inverse Hessian and four pose-space vectors

@@ -90,7 +90,7 @@ __device__ __forceinline__ LigView lig_view(const float4* pool, int64_t off) {
 constexpr int kNodeF = 20;
 constexpr int kNdAA = 16;
 
-__host__ __device__ inline int pad4(int n) { return (n + 3) & ~3; }
+__host__ __device__ constexpr int pad4(int n) { return (n + 3) & ~3; }
 // Shared-memory floats one warp needs for a ligand of the given size.
 __host__ __device__ inline int warp_floats(int na, int nn, int np, int nt) {
     return pad4(7 + nt) + kNodeF * nn + 4 * na + 3 * pad4(na) + 3 * pad4(na) + pad4(6 + nt);

@@ -131,13 +131,15 @@ struct Tile {
 // Rows of a tile: coordinates [3][na]; pair forces [3][na] after the poses'
 // components [7 + nt] and the bodies' local rotations [nn][4]; per body its
 // axis and origin [6], then its part of the gradient; a partial energy per warp.
-__host__ __device__ inline int tile_rows(int mode, int na, int nn, int nt, int warps) {
+__host__ __device__ constexpr int tile_rows(int mode, int na, int nn, int nt, int warps) {
     const int early = 7 + nt + 4 * nn;
     const int forces = mode == 1 && 3 * na > early ? 3 * na : early;
     return 3 * na + forces + (mode == 1 ? 6 * nn : 0) + (mode == 2 ? 0 : warps);
 }
 // Before them: the pairs as 32-bit words, an even number.
-__host__ __device__ inline int tile_words(int mode, int np) { return mode == 2 ? 0 : pad4(np); }
+__host__ __device__ constexpr int tile_words(int mode, int np) { return mode == 2 ? 0 : pad4(np); }
+static_assert((tile_words(1, VD_MAX_PAIRS) + tile_rows(1, VD_MAX_ATOMS, VD_MAX_TORS + 1, VD_MAX_TORS, 16) * 32) * 4 <= 227 * 1024,
+              "the largest ligand fits the widest tile");
 
 template <int mode, int PL>
 __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
@@ -390,7 +392,6 @@ vd_status launch_tile(Ctx& c, const HostLigand& L, const PoseParams& p, cudaStre
                sizeof(float);
     };
     const size_t smem = bytes(warps);
-    VD_CHECK(smem <= 227 * 1024, VD_ERR_CAPACITY, "ligand too large for the pose kernel");
     auto k = poses == 32 ? tile_kernel<mode, 32> : poses == 16 ? tile_kernel<mode, 16> : poses == 8 ? tile_kernel<mode, 8>
              : poses == 4 ? tile_kernel<mode, 4> : tile_kernel<mode, 1>;
     const int resident = std::max(1, std::min(int(227 * 1024 / (smem + 1024)), 32 / warps));  // 64 registers
