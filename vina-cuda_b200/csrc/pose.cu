@@ -1,8 +1,8 @@
 // Pose batches: forward energy kernel, adjoint kernel (energy + gradient,
 // recomputing atom coordinates from the torsion tree), coordinates, and
-// one RILC-BFGS local optimisation per pose.  Batches run as tiles of poses
-// with one pose per lane (tile_kernel), a few poses as teams of warps
-// (pose_team_kernel), what is between on one warp per pose.
+// one RILC-BFGS local optimisation per pose.  Energies and gradients run as tiles
+// of poses with one pose per lane (tile_kernel), those of a few poses as teams of
+// warps (pose_team_kernel), what is between and coordinates on one warp per pose.
 #include <cstring>
 
 #include "launch.h"
@@ -134,11 +134,11 @@ struct Tile {
 __host__ __device__ constexpr int tile_rows(int mode, int na, int nn, int nt, int warps) {
     const int early = 7 + nt + 4 * nn;
     const int forces = mode == 1 && 3 * na > early ? 3 * na : early;
-    return 3 * na + forces + (mode == 1 ? 6 * nn : 0) + (mode == 2 ? 0 : warps);
+    return 3 * na + forces + (mode == 1 ? 6 * nn : 0) + warps;
 }
 // Before them: the pairs as 32-bit words, an even number.
-__host__ __device__ constexpr int tile_words(int mode, int np) { return mode == 2 ? 0 : pad4(np); }
-static_assert((tile_words(1, VD_MAX_PAIRS) + tile_rows(1, VD_MAX_ATOMS, VD_MAX_TORS + 1, VD_MAX_TORS, 16) * 32) * 4 <= 227 * 1024,
+__host__ __device__ constexpr int tile_words(int np) { return pad4(np); }
+static_assert((tile_words(VD_MAX_PAIRS) + tile_rows(1, VD_MAX_ATOMS, VD_MAX_TORS + 1, VD_MAX_TORS, 16) * 32) * 4 <= 227 * 1024,
               "the largest ligand fits the widest tile");
 
 template <int mode, int PL>
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
     const LigView L = lig_view(p.lig, p.h);
     const int nc = 7 + L.nt, na = L.na;
     uint32_t* const W = reinterpret_cast<uint32_t*>(smem4);      // pairs: a | b << 8 | type pair << 16
-    float* const C = reinterpret_cast<float*>(W + tile_words(mode, L.np));  // [3][na]
+    float* const C = reinterpret_cast<float*>(W + tile_words(L.np));  // [3][na]
     float* const X = C + 3 * na * PL;                            // [nc], then
     float* const A = X + nc * PL;                                // [nn][4]
     int* const Q = reinterpret_cast<int*>(X);                    // [3][na], later
@@ -161,11 +161,10 @@ __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
         const int q = i / nc, c = i - q * nc;
         X[c * PL + q] = p.poses[size_t(first + min(q, here - 1)) * nc + c];
     }
-    if (mode != 2)
-        for (int i = threadIdx.x; i < L.np; i += blockDim.x) {
-            const int2 q = __ldg(&L.pairs[i]);
-            W[i] = uint32_t(q.x & 0xff) | uint32_t(q.x >> 16) << 8 | uint32_t(q.y) << 16;
-        }
+    for (int i = threadIdx.x; i < L.np; i += blockDim.x) {
+        const int2 q = __ldg(&L.pairs[i]);
+        W[i] = uint32_t(q.x & 0xff) | uint32_t(q.x >> 16) << 8 | uint32_t(q.y) << 16;
+    }
     __syncthreads();
     // local rotations, frames and coordinates: the arithmetic of frames() and
     // atom_position(), a slot per body
@@ -223,152 +222,145 @@ __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
         }
     }
     __syncthreads();
-    if constexpr (mode == 2) {
-        for (int i = threadIdx.x; i < here * 3 * na; i += blockDim.x) {
-            const int q = i / (3 * na), c = i - q * 3 * na, a = c / 3;
-            p.xyz_out[size_t(first) * 3 * na + i] = C[((c - 3 * a) * na + a) * PL + q];
-        }
-    } else {
-        if (mode == 1) {
-            for (int i = threadIdx.x; i < 3 * na * PL; i += blockDim.x) Q[i] = 0;
-            __syncthreads();
-        }
-        auto coords = [&](int i) {
-            return make_float3(C[i * PL + T.p], C[(na + i) * PL + T.p], C[(2 * na + i) * PL + T.p]);
-        };
-        // intra pairs: a slot takes a stretch of the pair list (sorted by second
-        // atom), the second atom's position and force in registers while it repeats
-        float e = 0.f;
-        {
-            const int twos = (L.np + 1) >> 1;  // two pairs at a time
-            const int q1 = min(L.np, 2 * int(uint32_t(T.slot + 1) * uint32_t(twos) / uint32_t(T.slots)));
-            int cur = -1;
-            float3 cb = make_float3(0.f, 0.f, 0.f);
-            float bx = 0.f, by = 0.f, bz = 0.f;  // in fixed-point units: fix is a power of two
-            auto add_to = [&](int i, float x, float y, float z) {
-                int* const d = Q + i * PL + T.p;
-                atomicAdd(d, __float2int_rn(x));
-                atomicAdd(d + na * PL, __float2int_rn(y));
-                atomicAdd(d + 2 * na * PL, __float2int_rn(z));
-            };
-            auto turn_to = [&](int b) {
-                if (mode == 1 && cur >= 0) add_to(cur, bx, by, bz);
-                cur = b;
-                bx = by = bz = 0.f;
-            };
-            for (int q = 2 * int(uint32_t(T.slot) * uint32_t(twos) / uint32_t(T.slots)); q < q1; q += 2) {
-                const bool two = q + 1 < q1;
-                const uint2 w = *reinterpret_cast<const uint2*>(W + q);
-                const uint32_t w1 = two ? w.y : w.x;
-                const int a0 = VD_DCLAMP(int(w.x & 0xff), 0, na - 1, kChkPairAtom), b0 = VD_DCLAMP(int(w.x >> 8 & 0xff), 0, na - 1, kChkPairAtom);
-                const int a1 = VD_DCLAMP(int(w1 & 0xff), 0, na - 1, kChkPairAtom), b1 = VD_DCLAMP(int(w1 >> 8 & 0xff), 0, na - 1, kChkPairAtom);
-                if (b0 != cur) {
-                    turn_to(b0);
-                    cb = coords(b0);
-                }
-                float3 cb1 = cb;
-                if (b1 != b0) cb1 = coords(b1);
-                const float3 ca0 = coords(a0), ca1 = coords(a1);
-                const float r0x = cb.x - ca0.x, r0y = cb.y - ca0.y, r0z = cb.z - ca0.z;
-                const float r1x = cb1.x - ca1.x, r1y = cb1.y - ca1.y, r1z = cb1.z - ca1.z;
-                const float d0 = r0x * r0x + r0y * r0y + r0z * r0z, d1 = r1x * r1x + r1y * r1y + r1z * r1z;
-                const float rf0 = fminf(32.f * d0, 2047.5f), rf1 = fminf(32.f * d1, 2047.5f);
-                const Trunc bin0 = trunc_pos(rf0), bin1 = trunc_pos(rf1);
-                const bool in0 = d0 < 64.f, in1 = two && d1 < 64.f;
-                float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
-                if (in0) t0 = __ldg(table_row(p.smooth, VD_DCLAMP(int(w.x >> 16), 0, kPairTypes - 1, kChkPairType), VD_DCLAMP(bin0.i, 0, kBins - 2, kChkTableBin)));
-                if (in1) t1 = __ldg(table_row(p.smooth, VD_DCLAMP(int(w1 >> 16), 0, kPairTypes - 1, kChkPairType), VD_DCLAMP(bin1.i, 0, kBins - 2, kChkTableBin)));
-                const float m0 = rf0 - bin0.f, m1 = rf1 - bin1.f, v = p.ep.v_intra;
-                const float e0 = t0.x + m0 * (t0.z - t0.x), g0 = t0.y + m0 * (t0.w - t0.y);
-                const float e1 = t1.x + m1 * (t1.z - t1.x), g1 = t1.y + m1 * (t1.w - t1.y);
-                const float c0 = (e0 > 0.f) ? __fdividef(v, v + e0) : 1.f, c1 = (e1 > 0.f) ? __fdividef(v, v + e1) : 1.f;
-                e += e0 * c0 + e1 * c1;  // zero past the cutoff
-                if (mode == 1) {
-                    if (in0) {
-                        const float h = g0 * c0 * c0 * p.ep.fix, Fx = h * r0x, Fy = h * r0y, Fz = h * r0z;
-                        add_to(a0, -Fx, -Fy, -Fz);
-                        bx += Fx; by += Fy; bz += Fz;
-                    }
-                    if (b1 != b0) turn_to(b1);
-                    if (in1) {
-                        const float h = g1 * c1 * c1 * p.ep.fix, Fx = h * r1x, Fy = h * r1y, Fz = h * r1z;
-                        add_to(a1, -Fx, -Fy, -Fz);
-                        bx += Fx; by += Fy; bz += Fz;
-                    }
-                } else {
-                    cur = b1;
-                }
-                cb = cb1;
-            }
-            turn_to(-1);
-        }
-        if (mode == 1) __syncthreads();
-        // grid terms; an atom's total force takes the place of its pair force.
-        // Energies from here on are added in FP64, rounded once per warp and once at
-        // the end: an FP32 chain lost small terms behind an out-of-box penalty
-        // and was 1 to 2 % further from FP64 than a warp per pose.
-        const GridInter inter{&p.G, p.ep.v_inter, p.ep.slope};
-        double sum = double(e);
-        for (int i = T.slot; i < na; i += T.slots) {
-            const float3 c = coords(i);
-            float g[3];
-            sum += inter(__float_as_int(__ldg(&L.atoms[i].w)) & 0xff, c.x, c.y, c.z, g[0], g[1], g[2]);
-            if (mode == 1)
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    int* const f = Q + (d * na + i) * PL + T.p;
-                    *reinterpret_cast<float*>(f) = g[d] + from_fixed(*f, p.ep.inv_fix);
-                }
-        }
-#pragma unroll
-        for (int o = 16; o >= PL; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);  // the warp's slots
-        if ((threadIdx.x & 31) < PL) E[(threadIdx.x >> 5) * PL + T.p] = float(sum);
+    if (mode == 1) {
+        for (int i = threadIdx.x; i < 3 * na * PL; i += blockDim.x) Q[i] = 0;
         __syncthreads();
-        if (threadIdx.x < here) {
-            double total = 0;
-            for (int s = 0; s < blockDim.x >> 5; ++s) total += E[s * PL + threadIdx.x];
-            p.e_out[first + threadIdx.x] = float(total);
+    }
+    auto coords = [&](int i) {
+        return make_float3(C[i * PL + T.p], C[(na + i) * PL + T.p], C[(2 * na + i) * PL + T.p]);
+    };
+    // intra pairs: a slot takes a stretch of the pair list (sorted by second
+    // atom), the second atom's position and force in registers while it repeats
+    float e = 0.f;
+    {
+        const int twos = (L.np + 1) >> 1;  // two pairs at a time
+        const int q1 = min(L.np, 2 * int(uint32_t(T.slot + 1) * uint32_t(twos) / uint32_t(T.slots)));
+        int cur = -1;
+        float3 cb = make_float3(0.f, 0.f, 0.f);
+        float bx = 0.f, by = 0.f, bz = 0.f;  // in fixed-point units: fix is a power of two
+        auto add_to = [&](int i, float x, float y, float z) {
+            int* const d = Q + i * PL + T.p;
+            atomicAdd(d, __float2int_rn(x));
+            atomicAdd(d + na * PL, __float2int_rn(y));
+            atomicAdd(d + 2 * na * PL, __float2int_rn(z));
+        };
+        auto turn_to = [&](int b) {
+            if (mode == 1 && cur >= 0) add_to(cur, bx, by, bz);
+            cur = b;
+            bx = by = bz = 0.f;
+        };
+        for (int q = 2 * int(uint32_t(T.slot) * uint32_t(twos) / uint32_t(T.slots)); q < q1; q += 2) {
+            const bool two = q + 1 < q1;
+            const uint2 w = *reinterpret_cast<const uint2*>(W + q);
+            const uint32_t w1 = two ? w.y : w.x;
+            const int a0 = VD_DCLAMP(int(w.x & 0xff), 0, na - 1, kChkPairAtom), b0 = VD_DCLAMP(int(w.x >> 8 & 0xff), 0, na - 1, kChkPairAtom);
+            const int a1 = VD_DCLAMP(int(w1 & 0xff), 0, na - 1, kChkPairAtom), b1 = VD_DCLAMP(int(w1 >> 8 & 0xff), 0, na - 1, kChkPairAtom);
+            if (b0 != cur) {
+                turn_to(b0);
+                cb = coords(b0);
+            }
+            float3 cb1 = cb;
+            if (b1 != b0) cb1 = coords(b1);
+            const float3 ca0 = coords(a0), ca1 = coords(a1);
+            const float r0x = cb.x - ca0.x, r0y = cb.y - ca0.y, r0z = cb.z - ca0.z;
+            const float r1x = cb1.x - ca1.x, r1y = cb1.y - ca1.y, r1z = cb1.z - ca1.z;
+            const float d0 = r0x * r0x + r0y * r0y + r0z * r0z, d1 = r1x * r1x + r1y * r1y + r1z * r1z;
+            const float rf0 = fminf(32.f * d0, 2047.5f), rf1 = fminf(32.f * d1, 2047.5f);
+            const Trunc bin0 = trunc_pos(rf0), bin1 = trunc_pos(rf1);
+            const bool in0 = d0 < 64.f, in1 = two && d1 < 64.f;
+            float4 t0 = make_float4(0.f, 0.f, 0.f, 0.f), t1 = t0;
+            if (in0) t0 = __ldg(table_row(p.smooth, VD_DCLAMP(int(w.x >> 16), 0, kPairTypes - 1, kChkPairType), VD_DCLAMP(bin0.i, 0, kBins - 2, kChkTableBin)));
+            if (in1) t1 = __ldg(table_row(p.smooth, VD_DCLAMP(int(w1 >> 16), 0, kPairTypes - 1, kChkPairType), VD_DCLAMP(bin1.i, 0, kBins - 2, kChkTableBin)));
+            const float m0 = rf0 - bin0.f, m1 = rf1 - bin1.f, v = p.ep.v_intra;
+            const float e0 = t0.x + m0 * (t0.z - t0.x), g0 = t0.y + m0 * (t0.w - t0.y);
+            const float e1 = t1.x + m1 * (t1.z - t1.x), g1 = t1.y + m1 * (t1.w - t1.y);
+            const float c0 = (e0 > 0.f) ? __fdividef(v, v + e0) : 1.f, c1 = (e1 > 0.f) ? __fdividef(v, v + e1) : 1.f;
+            e += e0 * c0 + e1 * c1;  // zero past the cutoff
+            if (mode == 1) {
+                if (in0) {
+                    const float h = g0 * c0 * c0 * p.ep.fix, Fx = h * r0x, Fy = h * r0y, Fz = h * r0z;
+                    add_to(a0, -Fx, -Fy, -Fz);
+                    bx += Fx; by += Fy; bz += Fz;
+                }
+                if (b1 != b0) turn_to(b1);
+                if (in1) {
+                    const float h = g1 * c1 * c1 * p.ep.fix, Fx = h * r1x, Fy = h * r1y, Fz = h * r1z;
+                    add_to(a1, -Fx, -Fy, -Fz);
+                    bx += Fx; by += Fy; bz += Fz;
+                }
+            } else {
+                cur = b1;
+            }
+            cb = cb1;
         }
-        if constexpr (mode == 1) {
-            // a body's force and torque about its origin: the atoms of its subtree
-            for (int k = T.slot; k < L.nn; k += T.slots) {
-                float* const b = B + 6 * k * PL + T.p;
-                const float ox = b[3 * PL], oy = b[4 * PL], oz = b[5 * PL];
-                const float* const F = reinterpret_cast<const float*>(Q) + T.p;
-                float fx = 0.f, fy = 0.f, fz = 0.f, tx = 0.f, ty = 0.f, tz = 0.f;
-                const int i1 = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 2).w), 0, na, kChkSubtree);
-                int i = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 1).w), 0, na, kChkSubtree);
-                while (i < i1) {  // sums of up to 8 atoms first: a long chain of additions loses digits
-                    float sx = 0.f, sy = 0.f, sz = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
-                    for (const int stop = min(i + 8, i1); i < stop; ++i) {
-                        const float3 c = coords(i);
-                        const float x = F[i * PL], y = F[(na + i) * PL], z = F[(2 * na + i) * PL];
-                        const float dx = c.x - ox, dy = c.y - oy, dz = c.z - oz;
-                        sx += x; sy += y; sz += z;
-                        ux += dy * z - dz * y;
-                        uy += dz * x - dx * z;
-                        uz += dx * y - dy * x;
-                    }
-                    fx += sx; fy += sy; fz += sz;
-                    tx += ux; ty += uy; tz += uz;
-                }
-                if (k == 0) {
-                    b[0] = fx; b[PL] = fy; b[2 * PL] = fz; b[3 * PL] = tx; b[4 * PL] = ty; b[5 * PL] = tz;
-                } else {
-                    b[0] = tx * b[0] + ty * b[PL] + tz * b[2 * PL];
-                }
+        turn_to(-1);
+    }
+    if (mode == 1) __syncthreads();
+    // grid terms; an atom's total force takes the place of its pair force.
+    // Energies from here on are added in FP64, rounded once per warp and once at
+    // the end: an FP32 chain lost small terms behind an out-of-box penalty
+    // and was 1 to 2 % further from FP64 than a warp per pose.
+    const GridInter inter{&p.G, p.ep.v_inter, p.ep.slope};
+    double sum = double(e);
+    for (int i = T.slot; i < na; i += T.slots) {
+        const float3 c = coords(i);
+        float g[3];
+        sum += inter(__float_as_int(__ldg(&L.atoms[i].w)) & 0xff, c.x, c.y, c.z, g[0], g[1], g[2]);
+        if (mode == 1)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                int* const f = Q + (d * na + i) * PL + T.p;
+                *reinterpret_cast<float*>(f) = g[d] + from_fixed(*f, p.ep.inv_fix);
             }
-            __syncthreads();
-            const int n = 6 + L.nt;
-            for (int i = threadIdx.x; i < here * n; i += blockDim.x) {
-                const int q = i / n, c = i - q * n;
-                p.g_out[size_t(first) * n + i] = B[(c < 6 ? c : 6 * (c - 5)) * PL + q];
+    }
+#pragma unroll
+    for (int o = 16; o >= PL; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);  // the warp's slots
+    if ((threadIdx.x & 31) < PL) E[(threadIdx.x >> 5) * PL + T.p] = float(sum);
+    __syncthreads();
+    if (threadIdx.x < here) {
+        double total = 0;
+        for (int s = 0; s < blockDim.x >> 5; ++s) total += E[s * PL + threadIdx.x];
+        p.e_out[first + threadIdx.x] = float(total);
+    }
+    if constexpr (mode == 1) {
+        // a body's force and torque about its origin: the atoms of its subtree
+        for (int k = T.slot; k < L.nn; k += T.slots) {
+            float* const b = B + 6 * k * PL + T.p;
+            const float ox = b[3 * PL], oy = b[4 * PL], oz = b[5 * PL];
+            const float* const F = reinterpret_cast<const float*>(Q) + T.p;
+            float fx = 0.f, fy = 0.f, fz = 0.f, tx = 0.f, ty = 0.f, tz = 0.f;
+            const int i1 = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 2).w), 0, na, kChkSubtree);
+            int i = VD_DCLAMP(__float_as_int(node_word(L.nodes, k, 1).w), 0, na, kChkSubtree);
+            while (i < i1) {  // sums of up to 8 atoms first: a long chain of additions loses digits
+                float sx = 0.f, sy = 0.f, sz = 0.f, ux = 0.f, uy = 0.f, uz = 0.f;
+                for (const int stop = min(i + 8, i1); i < stop; ++i) {
+                    const float3 c = coords(i);
+                    const float x = F[i * PL], y = F[(na + i) * PL], z = F[(2 * na + i) * PL];
+                    const float dx = c.x - ox, dy = c.y - oy, dz = c.z - oz;
+                    sx += x; sy += y; sz += z;
+                    ux += dy * z - dz * y;
+                    uy += dz * x - dx * z;
+                    uz += dx * y - dy * x;
+                }
+                fx += sx; fy += sy; fz += sz;
+                tx += ux; ty += uy; tz += uz;
             }
+            if (k == 0) {
+                b[0] = fx; b[PL] = fy; b[2 * PL] = fz; b[3 * PL] = tx; b[4 * PL] = ty; b[5 * PL] = tz;
+            } else {
+                b[0] = tx * b[0] + ty * b[PL] + tz * b[2 * PL];
+            }
+        }
+        __syncthreads();
+        const int n = 6 + L.nt;
+        for (int i = threadIdx.x; i < here * n; i += blockDim.x) {
+            const int q = i / n, c = i - q * n;
+            p.g_out[size_t(first) * n + i] = B[(c < 6 ? c : 6 * (c - 5)) * PL + q];
         }
     }
 }
 
-// Which kernel, and tile, by measurement (us on B200, energy + gradient | energy,
+// Which kernel, by measurement (us on B200, energy + gradient | energy,
 // warp per pose -> tile):
 //   24 atoms / 5 torsions (~200 pairs): 64 poses 8.8 -> 9.7, 1,000 8.5 -> 10.5,
 //     3,000 10.6 -> 12.4, 10,000 22.8 -> 17.7 | 16.7 -> 14.6, 65,536 105 -> 60 | 66 -> 50
@@ -378,25 +370,73 @@ __global__ void __launch_bounds__(512, 2) tile_kernel(PoseParams p) {
 //   90 / 32 (~3,500 pairs): 64 poses 47.6 -> 16.7, 500 49.5 -> 22.8, 3,001 78 -> 62 | 74 -> 55
 // A small ligand's evaluation in one warp is as short as a tile's phases, so
 // below kTilePairs pairs it takes 64 poses per SM (two tiles of 32) for the
-// tiles to pay.  Poses per tile: as many as leave two tiles per SM.
+// tiles to pay.
 constexpr int kTilePairs = 400;
+
+// The size of a tile: PL poses (as many as leave two tiles per SM) and 8 or 16
+// warps, by where the SMs run out of tiles or of L1; us with 8 | 16 warps:
+//   up to 4 poses, 1,500 pairs and more: 16 warps while two tiles per SM hold all
+//     poses, 80 atoms / 6 torsions 1,036 poses 23 | 22, 1,600 27 | 39
+//   8 poses become 16 on 16 warps from 24 poses per SM (four tiles of 8 per SM):
+//     4,096 poses of 60 / 15 39 -> 35, of 90 / 32 86 -> 74, of 128 / 3 68 -> 62
+//   16 poses: 16 warps where the tiles of 8 that fit would need a second wave,
+//     90 / 32 6,000 poses 111 | 114, 7,500 177 | 140; 128 / 3 144 | 116
+//   32 poses become 16 on 16 warps where an SM holds one tile (20,000 poses of 128 /
+//     3 327 -> 248), or where two take more than 160 KB and leave little L1 for the
+//     records of many bodies: of 80 / 6 (154 KB) 178 and 180, 100 / 12 (202 KB) 266 ->
+//     247, 90 / 32 (222 KB) 414 -> 306; with few bodies 100 / 4 (176 KB) 9 % slower
+// A warp per pose took 282 for those of 128 / 3 and 111 for 7,500 of them.
+inline bool few_bodies(const HostLigand& L) { return L.h.n_atoms > 8 * L.h.n_nodes; }
+struct TileShape {
+    int poses, warps;
+    size_t smem;
+    int resident;  // tiles per SM
+};
+template <int mode>
+TileShape tile_shape(const Ctx& c, const HostLigand& L, int n_poses) {
+    const int np = L.h.n_pairs;
+    auto shape = [&](int poses, int warps) {
+        TileShape t{poses, warps, 0, 0};
+        t.smem = (size_t(tile_words(np)) + size_t(tile_rows(mode, L.h.n_atoms, L.h.n_nodes, L.h.ntors, warps)) * poses) * sizeof(float);
+        t.resident = std::max(1, std::min(int(227 * 1024 / (t.smem + 1024)), 32 / warps));  // 64 registers
+        return t;
+    };
+    const double per_sm = double(n_poses) / (2.0 * c.sms);  // poses per tile for two tiles per SM
+    auto tiles = [&](int poses) { return (n_poses + poses - 1) / poses; };
+    if (per_sm >= 32) {
+        const TileShape t = shape(32, np >= kTilePairs ? 16 : 8);
+        return t.resident < 2 || (2 * (t.smem + 1024) > 160 * 1024 && !few_bodies(L)) ? shape(16, 16) : t;
+    }
+    if (per_sm >= 16) {
+        const TileShape t = shape(16, 8);
+        return tiles(16) > t.resident * c.sms ? shape(16, 16) : t;
+    }
+    if (per_sm >= 12) return shape(16, 16);
+    if (per_sm >= 8) return shape(8, 8);
+    const int poses = per_sm >= 1.5 ? 4 : 1;
+    return shape(poses, np >= 1500 && tiles(poses) <= 2 * c.sms ? 16 : 8);
+}
+
+// Ligands of many pairs in middle-sized batches that a warp per pose evaluates
+// faster than tiles: with more than 8 atoms per body a tile's slots idle while
+// bodies are placed and summed.  us, warp per pose and tile:
+//   50 atoms / 5 torsions: 1,036 poses 12.3 and 12.7, 1,600 12.9 and 14.4, 2,500
+//     15.4 and 17.8, 4,096 21.6 and 22.0, 4,900 31.1 and 26.2
+//   60 / 3: 2,500 17.1 and 20.3, 3,300 20.4 and 21.7; 80 / 2: 1,600 24.5 and 22.6,
+//     2,500 27.0 and 30.8, 3,300 33.7 and 32.6; 128 / 3: 2,500 49.8 and 54.3, 3,300 56.4 and 56.4
+inline bool warps_win(const Ctx& c, const HostLigand& L, int n_poses) {
+    const double per_sm = double(n_poses) / c.sms;
+    const int np = L.h.n_pairs;
+    return few_bodies(L) && (per_sm >= 16 ? per_sm < (np < 1500 ? 28 : 18) : np < 1000 && per_sm >= 10);
+}
 
 template <int mode>
 vd_status launch_tile(Ctx& c, const HostLigand& L, const PoseParams& p, cudaStream_t stream) {
-    const int np = L.h.n_pairs;
-    const double per_sm = double(p.n_poses) / (2.0 * c.sms);  // poses per tile for two tiles per SM
-    const int poses = per_sm >= 32 ? 32 : per_sm >= 16 ? 16 : per_sm >= 8 ? 8 : per_sm >= 1.5 ? 4 : 1;
-    int warps = (poses == 32 && np >= kTilePairs) || (poses <= 4 && np >= 1500) ? 16 : 8;
-    auto bytes = [&](int w) {
-        return (size_t(tile_words(mode, np)) + size_t(tile_rows(mode, L.h.n_atoms, L.h.n_nodes, L.h.ntors, w)) * poses) *
-               sizeof(float);
-    };
-    const size_t smem = bytes(warps);
-    auto k = poses == 32 ? tile_kernel<mode, 32> : poses == 16 ? tile_kernel<mode, 16> : poses == 8 ? tile_kernel<mode, 8>
-             : poses == 4 ? tile_kernel<mode, 4> : tile_kernel<mode, 1>;
-    const int resident = std::max(1, std::min(int(227 * 1024 / (smem + 1024)), 32 / warps));  // 64 registers
-    VD_CUDA(set_launch(c, k, resident, smem));
-    k<<<(p.n_poses + poses - 1) / poses, 32 * warps, smem, stream>>>(p);
+    const TileShape t = tile_shape<mode>(c, L, p.n_poses);
+    auto k = t.poses == 32 ? tile_kernel<mode, 32> : t.poses == 16 ? tile_kernel<mode, 16> : t.poses == 8 ? tile_kernel<mode, 8>
+             : t.poses == 4 ? tile_kernel<mode, 4> : tile_kernel<mode, 1>;
+    VD_CUDA(set_launch(c, k, t.resident, t.smem));
+    k<<<(p.n_poses + t.poses - 1) / t.poses, 32 * t.warps, t.smem, stream>>>(p);
     VD_CUDA(cudaGetLastError());
     return VD_OK;
 }
@@ -525,8 +565,9 @@ vd_status run_pose_kernel(Ctx& c, int lig, int n_poses, const float* d_poses, co
     if constexpr (mode == 3) {
         return launch_local_opt(c, L, p, stream);
     } else {
-        if (L.h.n_pairs >= kTilePairs || n_poses >= 64 * c.sms) return launch_tile<mode>(c, L, p, stream);
         if constexpr (mode != 2) {
+            if ((L.h.n_pairs >= kTilePairs && !warps_win(c, L, n_poses)) || n_poses >= 64 * c.sms)
+                return launch_tile<mode>(c, L, p, stream);
             if (n_poses <= kTeamPoses * c.sms) {
                 const size_t smem = (size_t(p.warp_floats) + pair_team_floats(L.h.sp_iters)) * sizeof(float);
                 VD_CUDA(set_launch(c, pose_team_kernel<mode>, kTeamPoses, smem));
