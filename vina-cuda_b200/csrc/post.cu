@@ -178,11 +178,12 @@ struct RefineParams {
     int32_t skip_invalid;       // leave poses whose e_out is FLT_MAX untouched
 };
 
-// One block refines one pose.  A dense-BFGS run is a serial chain of
-// evaluations, and an evaluation on the direct-sum score is mostly receptor
-// neighbours (tens to hundreds per atom, three dependent loads each) and
-// intra pairs: with one warp a pose, one lane walked an atom's neighbours
-// one after the other and a 20-pose call kept 5 SMs busy.  Warp 0 runs the
+// One block refines one pose, on 16 warps or fewer (refine_launch).  A
+// dense-BFGS run is a serial chain of evaluations, and an evaluation on the
+// direct-sum score is mostly receptor neighbours (tens to hundreds per atom,
+// three dependent loads each) and intra pairs: with one warp a pose, one lane
+// walked an atom's neighbours one after the other and a 20-pose call kept 5 SMs
+// busy.  Warp 0 runs the
 // optimiser; for each evaluation it places the atoms, then all warps compute
 // the neighbour and pair terms in parallel into shared memory, and their sums
 // are taken from there in the order a single lane would take them (a
@@ -193,7 +194,6 @@ struct RefineParams {
 // 20 modes, 31 atoms / 8 torsions: 1.95 -> 0.57 ms).  What is left is latency:
 // ~1,900 cycles of body frames, ~5,000 of receptor terms (two thirds of them
 // gathers from L2), ~1,200 of pairs, ~2,300 of optimiser per evaluation.
-constexpr int kRefineWarps = 16;
 constexpr int kNb = 32;    // neighbours of an atom per tile (one per lane)
 constexpr int kSlots = 4;  // atoms a warp takes at a time
 
@@ -215,21 +215,22 @@ struct TeamMem {
     int* runs;
 };
 
-__host__ __device__ inline int team_floats(int na, int np) {
-    return kRefineWarps * kTileFloats + pad4(na) + 4 * np + pad4((np + 2) / 2) + 4;
+__host__ __device__ inline int team_floats(int warps, int na, int np) {
+    return warps * kTileFloats + pad4(na) + 4 * np + pad4((np + 2) / 2) + 4;
 }
 
 // non_cache::eval_deriv terms (FP32, smooth table, curl v) of the atom
-// groups `wid`, `wid` + kRefineWarps, ..: gradients to m.fx/fy/fz, energies
+// groups `wid`, `wid` + warps, ..: gradients to m.fx/fy/fz, energies
 // to eatom.  Lanes are neighbours, a tile of kNb per atom at a time; then
 // lane 4 s + c adds up component c (x, y, z, energy) of atom s in list order.
+template <int warps>
 __device__ __forceinline__ void direct_terms(const LigView& L, const WarpMem& m, const RecView& R, const float4* smooth,
                                              float v, float slope, const TeamMem& tm, int wid, int lane) {
     float* const td = tm.tile + kSlots * 4 * kRow;
     float4* const at = reinterpret_cast<float4*>(td + kSlots * kRow);
     int2* const range = reinterpret_cast<int2*>(at + kSlots);
     const int groups = (L.na + kSlots - 1) / kSlots;
-    for (int g = wid; g < groups; g += kRefineWarps) {
+    for (int g = wid; g < groups; g += warps) {
         float a[3] = {0.f, 0.f, 0.f}, od[3] = {0.f, 0.f, 0.f}, oob = 0.f;
         int n = 0;
         if (lane < kSlots) {
@@ -335,9 +336,10 @@ __device__ __forceinline__ void direct_terms(const LigView& L, const WarpMem& m,
 // energy and force to tm.pair, the force on the first atom into its
 // fixed-point accumulator (integer sums: exact in any order).  Two pairs'
 // loads are in flight per thread.
+template <int warps>
 __device__ __forceinline__ void pair_terms(const LigView& L, const WarpMem& m, const float4* smooth, float v, float fix,
                                            const TeamMem& tm, int tid) {
-    constexpr int kStep = 32 * kRefineWarps;
+    constexpr int kStep = 32 * warps;
     int* const qx = reinterpret_cast<int*>(m.ns);
     int* const qy = qx + pad4(L.na);
     int* const qz = qy + pad4(L.na);
@@ -457,7 +459,8 @@ __device__ __forceinline__ bool m_out(float v, double b, double e) {
 // forces are added.  Warp 0 arrives at 1 and waits at 2, the others the other
 // way round; every thread takes part in each once per evaluation, and in 1
 // once more at the end.
-__global__ void __launch_bounds__(32 * kRefineWarps, 1) refine_kernel(RefineParams p) {
+template <int warps, int blocks>
+__global__ void __launch_bounds__(32 * warps, blocks) refine_kernel(RefineParams p) {
     extern __shared__ float4 smem4[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, pose = blockIdx.x;
     const int li = p.pose_lig ? p.pose_lig[pose] : 0;
@@ -477,28 +480,28 @@ __global__ void __launch_bounds__(32 * kRefineWarps, 1) refine_kernel(RefinePara
     TeamMem tm;
     float* team = mhy + pad4(n);
     tm.tile = team + wid * kTileFloats;
-    tm.eatom = team + kRefineWarps * kTileFloats;
+    tm.eatom = team + warps * kTileFloats;
     tm.pair = tm.eatom + pad4(L.na);
     tm.run = reinterpret_cast<uint16_t*>(tm.pair + 4 * L.np);
     tm.cmd = reinterpret_cast<int*>(tm.eatom + pad4(L.na) + 4 * L.np + pad4((L.np + 2) / 2));
     tm.slope = reinterpret_cast<float*>(tm.cmd + 1);
     tm.runs = tm.cmd + 2;
     auto terms = [&](float slope) {
-        direct_terms(L, s.m, p.R, p.smooth, 1000.f, slope, tm, wid, lane);
-        pair_terms(L, s.m, p.smooth, 1000.f, p.fix, tm, threadIdx.x);
+        direct_terms<warps>(L, s.m, p.R, p.smooth, 1000.f, slope, tm, wid, lane);
+        pair_terms<warps>(L, s.m, p.smooth, 1000.f, p.fix, tm, threadIdx.x);
         __syncwarp();
-        team_sync<kRefineWarps>(3);
+        if (warps > 1) team_sync<warps>(3);
     };
     if (wid == 0) find_runs(L, tm, lane);
     __syncthreads();
     if (wid > 0) {
         for (;;) {
-            team_sync<kRefineWarps>(1);
+            team_sync<warps>(1);
             if (*tm.cmd == 0) break;
             terms(*tm.slope);
-            run_terms(L, s.m, p.fix, tm, threadIdx.x - 32, 32 * (kRefineWarps - 1));
+            run_terms(L, s.m, p.fix, tm, threadIdx.x - 32, 32 * (warps - 1));
             __syncwarp();
-            team_arrive<kRefineWarps>(2);
+            team_arrive<warps>(2);
         }
         return;
     }
@@ -524,11 +527,12 @@ __global__ void __launch_bounds__(32 * kRefineWarps, 1) refine_kernel(RefinePara
                 *tm.slope = slope;
             }
             __syncwarp();
-            team_arrive<kRefineWarps>(1);
+            if (warps > 1) team_arrive<warps>(1);
             terms(slope);
             const float sum = sum_energy(L, tm, lane);
+            if (warps == 1) run_terms(L, s.m, p.fix, tm, lane, 32);
             __syncwarp();
-            team_sync<kRefineWarps>(2);
+            if (warps > 1) team_sync<warps>(2);
             if (skip(sum)) return sum;
             adjoint_phases(L, s.m, p.inv_fix, lane);
             return sum;
@@ -552,7 +556,7 @@ __global__ void __launch_bounds__(32 * kRefineWarps, 1) refine_kernel(RefinePara
         *tm.cmd = 0;
     }
     __syncwarp();
-    team_arrive<kRefineWarps>(1);
+    if (warps > 1) team_arrive<warps>(1);
 }
 
 // ------------------------------------------------------------ score (double)
@@ -1036,10 +1040,40 @@ RecView rec_view(const Ctx& c) {
     return R;
 }
 
-// Shared-memory floats of one pose's refinement block.
+// Shared-memory floats of one pose's refinement block, without its tiles.
 int refine_floats(const HostLigand& L) {
     const int n = 6 + L.h.ntors, nc = 7 + L.h.ntors;
-    return lig_warp_floats(L) + 2 * pad4(nc) + pad4(n * n) + 4 * pad4(n) + team_floats(L.h.n_atoms, L.h.n_pairs);
+    return lig_warp_floats(L) + 2 * pad4(nc) + pad4(n * n) + 4 * pad4(n) + team_floats(0, L.h.n_atoms, L.h.n_pairs);
+}
+
+// Refinement of `poses` poses of `atoms` heavy atoms (on average): kernel,
+// threads and shared memory.  Few poses take 16 warps each, for their latency;
+// more share the SMs on 8 (3 blocks per SM), or 4 where an evaluation is short,
+// and thousands of small ones run a warp each.  The poses do not depend on it.
+// ms with 16 / 8 / 4 / 1 warps, in a 4,000-atom receptor, and as it was with a
+// warp per pose and four poses per block:
+//   10 atoms / 1 torsion: 148 poses 0.26 / 0.28 / 0.26 / 0.43 (0.65), 1,500 1.01 / 0.89 /
+//     0.78 / 1.14 (1.43), 10,000 4.81 / 3.05 / 2.24 / 1.94 (2.47)
+//   24 / 5: 600 0.97 / 0.99 / 1.27 / 2.76 (2.59), 1,500 1.52 / 1.19 / 1.34 / 2.57 (2.26),
+//     5,000 3.97 / 2.63 / 2.72 / 3.41 (3.26), 10,000 7.19 / 4.34 / 4.20 / 3.78 (3.87)
+//   45 / 12: 1,000 2.14 / 2.24 / 2.54 / 7.04 (6.23), 1,500 2.72 / 2.70 / 3.10 / 8.49 (7.63),
+//     10,000 12.4 / 9.2 / 9.2 / 15.5 (14.1)
+struct RefineLaunch {
+    void (*kernel)(RefineParams) = nullptr;
+    int threads = 0;
+    size_t smem = 0;
+};
+vd_status refine_launch(Ctx& c, int poses, double atoms, int floats, RefineLaunch& r) {
+    const double per_sm = double(poses) / c.sms;
+    const int warps = atoms <= 16   ? (per_sm > 30 ? 1 : per_sm > 2 ? 4 : 16)
+                      : atoms <= 28 ? (per_sm > 60 ? 1 : per_sm > 40 ? 4 : per_sm > 6 ? 8 : 16)
+                                    : (per_sm > 10 ? 8 : 16);
+    r.kernel = warps == 16 ? refine_kernel<16, 1> : warps == 8 ? refine_kernel<8, 3> : warps == 4 ? refine_kernel<4, 5> : refine_kernel<1, 16>;
+    r.threads = 32 * warps;
+    r.smem = size_t(floats + warps * kTileFloats) * 4;
+    VD_CHECK(r.smem <= 227 * 1024, VD_ERR_CAPACITY, "refine kernel shared memory exceeds 227 KB");
+    VD_CUDA(set_launch(c, r.kernel, 0, r.smem));
+    return VD_OK;
 }
 
 inline size_t al256(size_t b) { return (b + 255) & ~size_t(255); }
@@ -1077,7 +1111,8 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     int sort_n = 2;  // >= 2: the warp's arrays after the 8-byte keys start 16-byte aligned
     while (sort_n < max_chains) sort_n <<= 1;
     VD_CHECK(sort_n <= 16384, VD_ERR_CAPACITY, "more than 16384 chains per ligand");
-    std::vector<int32_t> plig(size_t(n) * VD_MAX_MODES), nin(n, VD_MAX_MODES);
+    const int max_kept = std::min(VD_MAX_MODES, max_chains);
+    std::vector<int32_t> plig(size_t(n) * VD_MAX_MODES), nin(n, max_kept);
     for (int i = 0; i < n * VD_MAX_MODES; ++i) plig[i] = i / VD_MAX_MODES;
     // parameter arrays (host), mirrored at the start of the extra scratch
     size_t o = 0;
@@ -1117,18 +1152,18 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     cp.kept = d_kept;
     cp.sort_n = sort_n;
     cp.warp_floats = max_wf;
-    // as many candidates at a time as the shared memory left holds
+    // as many candidates at a time as there are chains and the shared memory left holds
     const size_t smem_c1 = size_t(sort_n) * 8 + size_t(VD_MAX_MODES) * 3 * max_na * 4, b_wf = size_t(max_wf) * 4;
     VD_CHECK(smem_c1 + b_wf <= 227 * 1024, VD_ERR_CAPACITY, "cluster kernel shared memory exceeds 227 KB");
     cp.warps = int(std::min<size_t>(kClusterThreads / 32, (227 * 1024 - 64 - smem_c1) / b_wf));
-    cp.warps = std::max(1, cp.warps);
+    cp.warps = std::max(1, std::min(cp.warps, max_chains));
     const size_t smem_c = smem_c1 + cp.warps * b_wf;
+    const int threads_c = std::max(32 * cp.warps, std::min(kClusterThreads, sort_n / 2));
     VD_CUDA(set_launch(c, cluster_kernel, 0, smem_c, 64));
     // refine
     const bool refine = sp.refine != 0;
     RefineParams rp{};
-    size_t smem_r = 0;
-    int blocks_r = 0;
+    RefineLaunch rl;
     if (refine) {
         rp.pool = c.d_pool;
         rp.lig_off = d_off;
@@ -1144,10 +1179,14 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
         rp.inv_fix = 1.f / c.fix_scale;
         rp.evals = reinterpret_cast<unsigned long long*>(c.d_counter + 4);
         rp.skip_invalid = 1;
-        smem_r = size_t(max_rwf) * 4;
-        VD_CHECK(smem_r <= 227 * 1024, VD_ERR_CAPACITY, "refine kernel shared memory exceeds 227 KB");
-        VD_CUDA(set_launch(c, refine_kernel, 0, smem_r));
-        blocks_r = n * VD_MAX_MODES;
+        int poses = 0;
+        double atoms = 0;
+        for (int i = 0; i < n; ++i) {
+            const int kept = std::min(VD_MAX_MODES, db.prefix[i + 1] - db.prefix[i]);
+            poses += kept;
+            atoms += double(kept) * c.ligs[ligs[i]].h.n_atoms;
+        }
+        if ((st = refine_launch(c, poses, atoms / poses, max_rwf, rl)) != VD_OK) return st;
     }
     // score
     ScoreParams sc{};
@@ -1164,18 +1203,18 @@ vd_status prepare_post(Ctx& c, const std::vector<int>& ligs, const vd_search_par
     sc.energy_range = sp.energy_range > 0 ? sp.energy_range : 3.0;
     sc.min_rmsd = 1.0;
     sc.out = d_out;
-    const size_t smem_s = size_t(VD_MAX_MODES) * pose_doubles(max_na, max_nn) * 8;
+    const size_t smem_s = size_t(max_kept) * pose_doubles(max_na, max_nn) * 8;
     VD_CHECK(smem_s <= 226 * 1024, VD_ERR_CAPACITY, "score kernel shared memory exceeds 226 KB");
     VD_CUDA(set_launch(c, score_kernel, 0, smem_s, 1024));
     const int stride = db.stride;
     const float* conf = db.d_conf;
     const float* e = db.d_e;
     pp.launch = [=](cudaStream_t stream) {
-        cluster_kernel<<<n, kClusterThreads, smem_c, stream>>>(cp);
+        cluster_kernel<<<n, threads_c, smem_c, stream>>>(cp);
         // gather kept poses (missing slots get e = FLT_MAX)
         gather_kernel<<<n * VD_MAX_MODES, 64, 0, stream>>>(d_kept, conf, e, stride, n * VD_MAX_MODES, d_rp, d_re);
-        if (refine) refine_kernel<<<blocks_r, 32 * kRefineWarps, smem_r, stream>>>(rp);
-        score_kernel<<<n, 32 * VD_MAX_MODES, smem_s, stream>>>(sc);
+        if (refine) rl.kernel<<<n * VD_MAX_MODES, rl.threads, rl.smem, stream>>>(rp);
+        score_kernel<<<n, 32 * max_kept, smem_s, stream>>>(sc);
         return cudaGetLastError();
     };
     return VD_OK;
@@ -1392,10 +1431,9 @@ vd_status vd_refine(vd_ctx* h, int32_t lig, int32_t n, float* poses, int32_t max
     rp.inv_fix = 1.f / c.fix_scale;
     rp.evals = d_evals;
     rp.skip_invalid = 0;
-    const size_t smem_r = size_t(refine_floats(L)) * 4;
-    VD_CHECK(smem_r <= 227 * 1024, VD_ERR_CAPACITY, "refine kernel shared memory exceeds 227 KB");
-    VD_CUDA(set_launch(c, refine_kernel, 0, smem_r));
-    refine_kernel<<<n, 32 * kRefineWarps, smem_r, c.stream>>>(rp);
+    RefineLaunch rl;
+    if ((st = refine_launch(c, n, L.h.n_atoms, refine_floats(L), rl)) != VD_OK) return st;
+    rl.kernel<<<n, rl.threads, rl.smem, c.stream>>>(rp);
     VD_CUDA(cudaGetLastError());
     VD_CUDA(cudaMemcpyAsync(poses, d_p, size_t(n) * nc * 4, cudaMemcpyDeviceToHost, c.stream));
     std::vector<char> tail(sizeof(head.evals) + size_t(n) * 4);
