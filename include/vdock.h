@@ -219,7 +219,9 @@ vd_status vd_energy_grad(vd_ctx* ctx, int32_t lig_id, int32_t n_poses, const flo
  * cudaStream_t; NULL is the CUDA default stream, as for a kernel launch), so
  * a caller orders it with its own work by passing its stream (e.g. torch's
  * current stream).  Ligand and map uploads made by earlier calls have
- * completed before these return. */
+ * completed before these return, and later calls that would overwrite what
+ * they read (vd_build_grids, vd_set_scoring and _device, the first call with
+ * ligands added after vd_clear_ligands) wait for them. */
 vd_status vd_energy_grad_device(vd_ctx* ctx, int32_t lig_id, int32_t n_poses,
                                 const float* poses_device, const vd_eval_params* p,
                                 float* e_device, float* g_device, void* stream);
