@@ -114,10 +114,10 @@ __global__ void __launch_bounds__(32 * kPoseTeam, kTeamPoses) pose_team_kernel(P
 // random places of shared memory and the lanes past a ligand's bodies and
 // atoms idle: 1,198 L1 wavefronts and 3,241 warp instructions per evaluation
 // of 40 atoms / 595 pairs at 65,536 poses, 90 % of the L1 data pipe.  With
-// lanes as poses the loads are conflict-free and the pair list is uniform:
-// 605 and 2,218; what is left is the table gathers, about one wavefront per
-// lane, and L1 hit rate decides (33 % at 4 tiles per SM), so large ligands
-// take 16 warps per tile and two tiles per SM.
+// lanes as poses the loads are conflict-free and the pair list is uniform: 605
+// and 2,218 with 8 warps a tile, 621 and 2,206 with 16; what is left is the
+// table gathers, about one wavefront per lane, and L1 (27 to 33 % hits) decides:
+// tile_shape below.
 template <int PL>
 struct Tile {
     int p, slot, slots;
